@@ -81,3 +81,35 @@ def test_codec_matches_the_reference_store(cuda_device, location):
     np.testing.assert_array_equal(store._data[0].float().cpu().numpy(), g["stored"])
     np.testing.assert_array_equal(store.get(0).cpu().numpy(), g["decoded"])
     assert float(g["scale"][1, 2].item()) == 1.0 and float(g["scale"][2, 5].item()) == 1.0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("groups,cells", [(1, (1, 1, 1)), (3, (2, 5, 25)), (8, (8, 8, 4)), (16, (1, 1, 257)),
+                                          (33, (3, 5, 17)), (40, (1, 16, 33))])
+@pytest.mark.parametrize("cell_major", [True, False])
+def test_codec_over_tile_edges(cuda_device, groups, cells, cell_major):
+    """Cells around the 256 of a tile and groups around its 32, in cell-major and in contiguous storage, with a plane
+    that holds an infinity, one of negative zeros and one with a single NaN: the float32 tensor arithmetic, bit for
+    bit."""
+    shape = (groups, 4, 4, *cells)
+    gen = torch.Generator().manual_seed(groups)
+    phi = 1e-6 * torch.randn(shape, generator=gen)
+    phi[0, 1, 0, 0, 0, 0] = float("nan")
+    phi[-1, 2, 0, -1, -1, -1] = -float("inf")
+    phi[0, 3, 0] = -0.0
+    if cell_major:
+        phi = phi.permute(1, 3, 4, 5, 0, 2).contiguous().permute(4, 0, 5, 1, 2, 3)
+        phi = phi.to(cuda_device)
+    else:
+        phi = phi.to(cuda_device)
+    store = StateStore(1, shape, cuda_device, location="gpu")
+    store.put(0, phi)
+    mean = phi[:, :, :1]
+    maximum = mean.abs().amax(dim=(2, 3, 4, 5), keepdim=True)
+    scale = torch.where(maximum > 0, maximum / 2.0 ** 14, torch.ones_like(maximum))
+    stored = (mean / scale).to(torch.float16)
+    assert torch.equal(store._scale[0].view(torch.int32), scale.view(torch.int32))
+    np.testing.assert_array_equal(store._data[0].float().cpu().numpy(), stored.float().cpu().numpy())
+    out = store.get(0)
+    np.testing.assert_array_equal(out[:, :, :1].cpu().numpy(), (stored.float() * scale).cpu().numpy())
+    assert not bool(out[:, :, 1:].any())
