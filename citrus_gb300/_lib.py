@@ -48,6 +48,8 @@ SIGNATURES = {
     "citrus_group_transmission": [P, I64, I64, P, P, P, I64, I64, P, P, P, P, P],
     "citrus_source_weight": [P, P, P, P, P, P, I64, I32, P, P],
     "citrus_source_field": [P, P, P, P, I64, F64, P, P, I64, P, P, P, P, P, I64, I32, P, P, P],
+    "citrus_primary_image": [P, I64, I64, I64, I64, P, P, P, I64, I64, P, P, P, P, P, I64, P, P, P, I64, F64, P, P, P, P,
+                             P, P],
     "citrus_first_collision_source": [P, I64, P, I64, P, P, P, P, I64, F64, F64, P, I64, P, P],
     "citrus_first_collision_moments": [P, I64, P, I64, P, P, I64, P, P, I64, F64, F64, P, I64, P, P, P, P, P, I64,
                                        P],

@@ -236,6 +236,14 @@ class ConeGeometry:
                 + (2.0 * radius * np.sin(0.5 * gamma) ** 2)[..., None] * n_hat
                 + (v * np.cos(gamma))[..., None] * v_hat)
 
+    def pixel_columns_np(self, angle: float) -> tuple:
+        """float64 [channels, 3] positions of the pixel columns at v = 0 and [channels, 3] directions of v there: pixel
+        (r, c) lies at position[c] + v[r] direction[c], the values of ``pixel_centers_np``."""
+        u, _ = self.pixel_uv()
+        _, v_hat, _ = self.panel_axes(angle)
+        rise = np.cos(u / float(self.source_detector_dist)) if self.use_curved_detector else np.ones_like(u)
+        return self.panel_points_np(u, np.zeros_like(u), angle), rise[:, None] * np.asarray(v_hat)
+
     def pixel_centers_np(self, angle: float) -> np.ndarray:
         """float64 [rows, channels, 3] pixel-centre positions."""
         u, v = self.pixel_uv()

@@ -27,7 +27,7 @@ from .quadrature import Quadrature, hemisphere_quadrature, real_spherical_harmon
 from .ray_tracing import HostArgs
 from .responses import (DetectorResponse, GridResponse, SourceModel, detector_angle, grid_angles,
                         septa_dependence)
-from .uncollided import _FCArgs, group_transmission, present_materials
+from .uncollided import _FCArgs, fine_tables, group_transmission, present_materials
 
 IMAGE_CHUNK_MAX_DIRECTIONS = 32
 IMAGE_CHUNK_BUDGET_BYTES = 256 * 2 ** 20
@@ -476,6 +476,55 @@ def primary_path_lengths(projectors, rho: Tensor, grid: Grid, geometry: ConeGeom
     return projectors.primary_project(rho, grid, fine, angle)
 
 
+def _primary_on_device(geometry, source, detector, grid_response, library: MultigroupLibrary) -> bool:
+    """Whether ``citrus_primary_image`` evaluates this primary: the package's own panel, source and detector models
+    (another class may place its pixels or weigh its rays as it likes), a grid without angles (its table per pixel
+    needs the host's grid angles), and fine energies in group order (a group's sum is then one run)."""
+    group = np.asarray(library.fine_group)
+    return (type(geometry) is ConeGeometry and type(source) is SourceModel and type(detector) is DetectorResponse
+            and geometry.source_detector_dist > 0 and geometry.delta_det_row > 0 and geometry.delta_det_channel > 0
+            and not grid_response.depends_on_angles and group.size > 0 and int(group[0]) >= 0
+            and int(group[-1]) < library.num_groups and bool(np.all(group[1:] >= group[:-1])))
+
+
+def _device_primary(library: MultigroupLibrary, path: Tensor, materials, geometry: ConeGeometry, angle: float,
+                    source: SourceModel, detector: DetectorResponse, grid_response: GridResponse, n: int) -> dict:
+    """:func:`primary_from_path_lengths` in one launch: the geometry goes to the device as its pixel columns and rows,
+    the responses as their table at the group energies (one node where it does not depend on the incidence)."""
+    device = path.device
+    Rd, Cd = geometry.image_shape
+    G = library.num_groups
+    mu, w, g = fine_tables(library, materials, device)
+    if mu.shape[0] != int(path.shape[0]):
+        raise ValueError(f"path has {int(path.shape[0])} materials, the library {mu.shape[0]}")
+    position, direction = geometry.pixel_columns_np(angle)
+    columns = np.concatenate([position - np.asarray(geometry.source_position(angle)), direction,
+                              geometry.local_normals_np(position, angle)], axis=1)
+    u, v = geometry.pixel_uv()
+    theta = np.asarray(detector.theta_rad, dtype=np.float64).reshape(-1)
+    response = detector.at(library.group_energy, theta) * grid_response.at_energy(library.group_energy)[:, None]
+    if np.array_equal(response, np.broadcast_to(response[:, :1], response.shape)):
+        theta, response = theta[:1], response[:, :1]
+    host = np.concatenate([np.ravel(a) for a in (columns, u, v, theta, response)])
+    tables = _lib.upload(host, device, torch.float64)
+    starts = np.cumsum([0, columns.size, u.size, v.size, theta.size]) * 8 + tables.data_ptr()
+    extras = source.device_tables(geometry, angle, device)
+    thickness = extras["thickness"]
+    filter_mu = None if thickness is None else _lib.upload(source.filter_attenuation(library), device, torch.float32)
+    path = path.to(torch.float32).contiguous()
+    fluence, planar, per_group = (torch.empty(G, Rd, Cd, device=device) for _ in range(3))
+    signal = torch.empty(Rd, Cd, device=device)
+    args = HostArgs()
+    panel = args.doubles([geometry.delta_det_row, geometry.delta_det_channel, geometry.det_row_offset,
+                          geometry.det_channel_offset])
+    _lib.call("citrus_primary_image", path.data_ptr(), int(path.shape[0]), Rd, Cd, n, mu.data_ptr(), w.data_ptr(),
+              g.data_ptr(), int(w.numel()), G, *(int(a) for a in starts), theta.size, panel,
+              _lib.ptr(extras["profile"]), _lib.ptr(thickness), 0 if thickness is None else int(thickness.shape[0]),
+              source.filter_density, _lib.ptr(filter_mu), fluence.data_ptr(), planar.data_ptr(),
+              per_group.data_ptr(), signal.data_ptr(), _lib.stream_handle(device))
+    return {"fluence": fluence, "planar_fluence": planar, "signal_per_group": per_group, "signal": signal}
+
+
 def primary_from_path_lengths(library: MultigroupLibrary, path: Tensor, materials, geometry: ConeGeometry,
                               angle: float, source: SourceModel, detector: DetectorResponse,
                               grid_response: GridResponse) -> dict:
@@ -488,6 +537,8 @@ def primary_from_path_lengths(library: MultigroupLibrary, path: Tensor, material
     n = int(path.shape[1]) // Rd if path.dim() == 3 else 0
     if n < 1 or tuple(path.shape[1:]) != (Rd * n, Cd * n):
         raise ValueError(f"path must be [M', {Rd} n, {Cd} n] (n >= 1 sub-pixels per axis), got {tuple(path.shape)}")
+    if _primary_on_device(geometry, source, detector, grid_response, library):
+        return _device_primary(library, path, materials, geometry, angle, source, detector, grid_response, n)
     r0 = np.asarray(geometry.source_position(angle))
     filter_path = None
     if source.has_filter:

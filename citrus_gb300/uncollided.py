@@ -105,6 +105,19 @@ def source_weight(source: SourceModel, geometry: ConeGeometry, angle: float, poi
     return source_field(source, geometry, angle, points, device, divide_by_distance_squared)[0]
 
 
+def fine_tables(library: MultigroupLibrary, materials: Optional[Sequence[int]], device) -> tuple:
+    """Device copies of the fine attenuation [M', E], weights [E] and groups [E] int32, kept with the library."""
+    key = ("fine", None if materials is None else tuple(int(m) for m in materials), str(device))
+    cached = library._device_cache.get(key)
+    if cached is None:
+        fine_mu = library.fine_mu_t if materials is None else library.fine_mu_t[list(materials)]
+        cached = (torch.as_tensor(np.ascontiguousarray(fine_mu), dtype=torch.float32).to(device),
+                  library.tensor("fine_weight", device),
+                  torch.as_tensor(library.fine_group.astype(np.int32)).to(device))
+        library._device_cache[key] = cached
+    return cached
+
+
 def group_transmission(library: MultigroupLibrary, path: Tensor, materials: Optional[Sequence[int]] = None,
                        factor: Optional[Tensor] = None, filter_path: Optional[Tensor] = None,
                        filter_attenuation=None) -> Tensor:
@@ -115,19 +128,11 @@ def group_transmission(library: MultigroupLibrary, path: Tensor, materials: Opti
     Mp = int(path.shape[0])
     spatial = tuple(path.shape[1:])
     P = int(np.prod(spatial)) if spatial else 1
-    fine_mu = library.fine_mu_t if materials is None else library.fine_mu_t[list(materials)]
-    if fine_mu.shape[0] != Mp:
-        raise ValueError(f"path has {Mp} materials, the library {fine_mu.shape[0]}")
     if (filter_path is None) != (filter_attenuation is None):
         raise ValueError("filter_path and filter_attenuation go together")
-    key = ("fine", None if materials is None else tuple(int(m) for m in materials), str(device))
-    cached = library._device_cache.get(key)
-    if cached is None:
-        cached = (torch.as_tensor(np.ascontiguousarray(fine_mu), dtype=torch.float32).to(device),
-                  library.tensor("fine_weight", device),
-                  torch.as_tensor(library.fine_group.astype(np.int32)).to(device))
-        library._device_cache[key] = cached
-    mu, w, g = cached
+    mu, w, g = fine_tables(library, materials, device)
+    if mu.shape[0] != Mp:
+        raise ValueError(f"path has {Mp} materials, the library {mu.shape[0]}")
     p = path.to(torch.float32).reshape(Mp, P).contiguous()
     G = library.num_groups
     out = torch.empty(G, P, device=device, dtype=torch.float32)

@@ -268,6 +268,23 @@ int citrus_source_field(const double* field, const double* panel, const double* 
                         int64_t num_points, int32_t divide_by_distance_squared, float* out, float* filter_path_out,
                         void* stream);
 
+/* The primary image from path lengths [M, rows n, cols n] in g/cm^2 (n x n rays per pixel): the group transmission of
+ * every ray (fine tables as in citrus_group_transmission, fine_group ascending; a beam filter of thickness
+ * [thickness_rows = 1 | rows, cols] in cm times filter_density adds filter_mu [E] to the exponents), its mean over the
+ * rays, times profile / |d|^2 (fluence), the cosine of incidence (planar) and the response (per_group), each
+ * [G, rows, cols], and the sum of the last over the groups (signal [rows, cols]). columns [cols, 9] = position from the
+ * focal spot at v = 0, direction of v, inward normal; u [cols], v [rows] panel coordinates; response [G, num_theta] at
+ * the incidence angles theta_nodes [num_theta] ascending (linear, clamped). panel (host double [4]) = row pitch,
+ * channel pitch, row offset, channel offset. float64 tables on the device.
+ * Replaces primary_from_path_lengths (scatter_image.py:1395-1471). */
+int citrus_primary_image(const float* path, int64_t num_materials, int64_t num_rows, int64_t num_cols, int64_t samples,
+                         const float* fine_mu, const float* fine_weight, const int32_t* fine_group, int64_t num_fine,
+                         int64_t num_groups, const double* columns, const double* u, const double* v,
+                         const double* theta_nodes, const double* response, int64_t num_theta, const double* panel,
+                         const double* profile, const double* thickness, int64_t thickness_rows,
+                         double filter_density, const float* filter_mu, float* fluence, float* planar,
+                         float* per_group, float* signal, void* stream);
+
 /* Shared arguments of the first-collision kernels: rho [M, V] densities on the point grid, phi [G, V] uncollided
  * fluence, axes = float32 point coordinates x [cols], y [rows], z [slices] back to back, point_dims (host) = rows,
  * cols, slices, focal_spot (host double [3]), table [M, N_eta, G_out, G_in] per-steradian transfer (zero for
