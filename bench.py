@@ -612,9 +612,9 @@ def product_emission_bytes(args) -> int:
     return 4 * floats
 
 
-def downstream_bytes(args) -> int:
+def downstream_bytes(args, k_at: int = 6) -> int:
     """citrus_downstream_cumulative: the cell volume read once, the optical depths [K, C, V] written once."""
-    C, dims, K = int(args[1]), _dims(args[3]), int(args[6])
+    C, dims, K = int(args[1]), _dims(args[3]), int(args[k_at])
     V = dims[0] * dims[1] * dims[2]
     return 4 * (C * V + K * C * V)
 
@@ -634,6 +634,7 @@ def tiled_sweep_bytes(args) -> int:
 SWEEP_ENTRY_POINTS = ("citrus_sweep_tiled", "citrus_sweep_persistent_config", "citrus_sweep_persistent")
 STEP_TIMED = {"citrus_attenuated_emission_moments": emission_bytes, "citrus_attenuated_emission": product_emission_bytes,
               "citrus_downstream_cumulative": downstream_bytes, "citrus_downstream_cumulative_tables": downstream_bytes,
+              "citrus_downstream_cumulative_facing": lambda args: downstream_bytes(args, 5),
               "citrus_sweep_persistent": sweep_bytes, "citrus_sweep_persistent_config": sweep_bytes,
               "citrus_sweep_tiled": tiled_sweep_bytes,
               "citrus_oblique_project": None, "citrus_oblique_project_scratch": None, "citrus_box_blur": None,

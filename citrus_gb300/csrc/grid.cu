@@ -20,6 +20,7 @@ namespace {
 
 constexpr int kGridMaxG = 32;
 constexpr int kGridMaxSepta = 2;
+constexpr int kGridSumBlock = 64;
 
 struct PixelSepta {
   const float* theta_channels;  // [2, K, Cd] theta1 and theta2 along the first row (chunk directions from 0)
@@ -64,55 +65,58 @@ __global__ void grid_signal_sum_kernel(const float* __restrict__ img, int K, int
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (int64_t)R * C) return;
   const int r = (int)(t / C), c = (int)(t - (int64_t)r * C);
-  float sum[kGridMaxG];
-#pragma unroll
-  for (int g = 0; g < kGridMaxG; ++g) sum[g] = 0.f;
   float th1[kGridMaxSepta], th2[kGridMaxSepta];
   for (int s = 0; s < ga.num_septa; ++s) {
     th1[s] = __ldg(ga.septa[s].theta_pixels + t);
     th2[s] = __ldg(ga.septa[s].theta_pixels + (int64_t)R * C + t);
   }
-  for (int k = 0; k < K; ++k) {
-    int i10[kGridMaxSepta], i11[kGridMaxSepta], i20[kGridMaxSepta], i21[kGridMaxSepta];
-    float w1[kGridMaxSepta], w2[kGridMaxSepta];
-    for (int s = 0; s < ga.num_septa; ++s) {
-      const PixelSepta& ps = ga.septa[s];
-      const float a1 = __ldg(ps.theta_channels + (int64_t)k * C + c) + th1[s];
-      const float a2 = __ldg(ps.theta_channels + ((int64_t)K + k) * C + c) + th2[s];
-      bracket(ps.nodes1, ps.T1, fabsf(a1), i10[s], i11[s], w1[s]);
-      bracket(ps.nodes2, ps.T2, fabsf(a2), i20[s], i21[s], w2[s]);
-    }
-    const float* src = img + k * is_k + r * is_r + c * is_c;
+  // blocks of directions added to the accumulator in order, rounded as one call per block rounds
+  for (int k0 = 0; k0 < K || k0 == 0; k0 += kGridSumBlock, accumulate = 1) {
+    float sum[kGridMaxG];
 #pragma unroll
-    for (int g = 0; g < kGridMaxG; ++g) {
-      if (g >= G) break;
-      float w = __ldg(W + ((int64_t)k * G + g) * w_cols + (w_cols > 1 ? c : 0));
-      if (row_w) w *= __ldg(row_w + ((int64_t)k * G + g) * R + r);
+    for (int g = 0; g < kGridMaxG; ++g) sum[g] = 0.f;
+    for (int k = k0; k < min(k0 + kGridSumBlock, K); ++k) {
+      int i10[kGridMaxSepta], i11[kGridMaxSepta], i20[kGridMaxSepta], i21[kGridMaxSepta];
+      float w1[kGridMaxSepta], w2[kGridMaxSepta];
       for (int s = 0; s < ga.num_septa; ++s) {
         const PixelSepta& ps = ga.septa[s];
-        const float* tg = ps.table + (int64_t)g * ps.T1 * ps.T2;
-        const float a00 = __ldg(tg + i10[s] * ps.T2 + i20[s]), a01 = __ldg(tg + i10[s] * ps.T2 + i21[s]);
-        const float a10 = __ldg(tg + i11[s] * ps.T2 + i20[s]), a11 = __ldg(tg + i11[s] * ps.T2 + i21[s]);
-        const float a0 = a00 + (a01 - a00) * w2[s];
-        const float a1 = a10 + (a11 - a10) * w2[s];
-        w *= a0 + (a1 - a0) * w1[s];
+        const float a1 = __ldg(ps.theta_channels + (int64_t)k * C + c) + th1[s];
+        const float a2 = __ldg(ps.theta_channels + ((int64_t)K + k) * C + c) + th2[s];
+        bracket(ps.nodes1, ps.T1, fabsf(a1), i10[s], i11[s], w1[s]);
+        bracket(ps.nodes2, ps.T2, fabsf(a2), i20[s], i21[s], w2[s]);
       }
-      sum[g] = fmaf(w, __ldg(src + g * is_g), sum[g]);
-    }
-  }
-  if (per_group) {
+      const float* src = img + k * is_k + r * is_r + c * is_c;
 #pragma unroll
-    for (int g = 0; g < kGridMaxG; ++g) {
-      if (g >= G) break;
-      float* o = acc + (int64_t)g * R * C + t;
-      *o = accumulate ? *o + sum[g] : sum[g];
+      for (int g = 0; g < kGridMaxG; ++g) {
+        if (g >= G) break;
+        float w = __ldg(W + ((int64_t)k * G + g) * w_cols + (w_cols > 1 ? c : 0));
+        if (row_w) w *= __ldg(row_w + ((int64_t)k * G + g) * R + r);
+        for (int s = 0; s < ga.num_septa; ++s) {
+          const PixelSepta& ps = ga.septa[s];
+          const float* tg = ps.table + (int64_t)g * ps.T1 * ps.T2;
+          const float a00 = __ldg(tg + i10[s] * ps.T2 + i20[s]), a01 = __ldg(tg + i10[s] * ps.T2 + i21[s]);
+          const float a10 = __ldg(tg + i11[s] * ps.T2 + i20[s]), a11 = __ldg(tg + i11[s] * ps.T2 + i21[s]);
+          const float a0 = a00 + (a01 - a00) * w2[s];
+          const float a1 = a10 + (a11 - a10) * w2[s];
+          w *= a0 + (a1 - a0) * w1[s];
+        }
+        sum[g] = fmaf(w, __ldg(src + g * is_g), sum[g]);
+      }
     }
-  } else {
-    float total = 0.f;
+    if (per_group) {
 #pragma unroll
-    for (int g = 0; g < kGridMaxG; ++g)
-      if (g < G) total += sum[g];
-    acc[t] = accumulate ? acc[t] + total : total;
+      for (int g = 0; g < kGridMaxG; ++g) {
+        if (g >= G) break;
+        float* o = acc + (int64_t)g * R * C + t;
+        *o = accumulate ? *o + sum[g] : sum[g];
+      }
+    } else {
+      float total = 0.f;
+#pragma unroll
+      for (int g = 0; g < kGridMaxG; ++g)
+        if (g < G) total += sum[g];
+      acc[t] = accumulate ? acc[t] + total : total;
+    }
   }
 }
 

@@ -570,9 +570,20 @@ __global__ void __launch_bounds__(kThreads) from_source_kernel(Box b, const floa
 // The detector surface the downstream rays stop at, in float (rounded on the host, once).
 struct Panel {
   int curved;
+  int test_facing;             // directions that do not face the panel are told from its normal, not from `toward`
   float center[3], normal[3];  // flat panel: a point of the plane and its normal (toward the source)
   float source[3], radius2;    // curved panel: the cylinder about the vertical axis through the source
 };
+
+// whether direction k faces the panel: the caller's byte, else omega . (-n_hat) > 0 with every operation rounded on
+// its own, as tensor arithmetic evaluates it (seven small launches per call before it was done here)
+__device__ __forceinline__ bool faces_panel(const Panel& p, const uint8_t* __restrict__ toward,
+                                            const float* __restrict__ omegas, int k) {
+  if (toward != nullptr) return toward[k] != 0;
+  if (!p.test_facing) return true;
+  const float* w = omegas + 3 * k;
+  return add_rn(add_rn(mul_rn(w[0], -p.normal[0]), mul_rn(w[1], -p.normal[1])), mul_rn(w[2], -p.normal[2])) > 0.f;
+}
 
 __device__ __forceinline__ float panel_distance(const Panel& p, const float r[3], const float w[3]) {
   if (!p.curved) {
@@ -605,7 +616,7 @@ __global__ void __launch_bounds__(kThreads) downstream_kernel(Box b, const float
   if (v >= V) return;
   const int nC = kC > 0 ? kC : C;
   float* o = out + (int64_t)k * os_k + v * os_v;
-  if (toward != nullptr && toward[k] == 0) {
+  if (!faces_panel(panel, toward, omegas, k)) {
     for (int c = 0; c < nC; ++c) o[(int64_t)c * os_c] = INFINITY;
     return;
   }
@@ -703,7 +714,7 @@ __global__ void __launch_bounds__(kThreads) downstream_lattice_kernel(Box b, con
   if (v >= V) return;
   const int nC = kC > 0 ? kC : C;
   float* o = out + (int64_t)k * os_k + v * os_v;
-  if (toward != nullptr && toward[k] == 0) {
+  if (!faces_panel(panel, toward, omegas, k)) {
     for (int c = 0; c < nC; ++c) o[(int64_t)c * os_c] = INFINITY;
     return;
   }
@@ -960,7 +971,7 @@ namespace {
 int downstream(const float* volume, int64_t channels, const double* box, const int64_t* dims, const float* omegas,
                const uint8_t* toward, int64_t num_directions, const double* panel, double diagonal, float* out,
                int64_t os_k, int64_t os_c, int64_t os_v, int32_t* crossings, int64_t crossings_words, bool build,
-               void* stream);
+               bool test_facing, void* stream);
 }  // namespace
 }  // namespace citrus
 
@@ -989,7 +1000,7 @@ extern "C" int citrus_downstream_cumulative_tables(const float* volume, int64_t 
                                                    const int32_t* crossings, int64_t crossings_words, void* stream) {
   CITRUS_REQUIRE(crossings != nullptr, "citrus_downstream_cumulative_tables: null crossing tables");
   return downstream(volume, channels, box, dims, omegas, toward, num_directions, panel, diagonal, out, os_k, os_c,
-                    os_v, const_cast<int32_t*>(crossings), crossings_words, false, stream);
+                    os_v, const_cast<int32_t*>(crossings), crossings_words, false, false, stream);
 }
 
 extern "C" int citrus_downstream_cumulative(const float* volume, int64_t channels, const double* box,
@@ -998,7 +1009,16 @@ extern "C" int citrus_downstream_cumulative(const float* volume, int64_t channel
                                             float* out, int64_t os_k, int64_t os_c, int64_t os_v, int32_t* crossings,
                                             int64_t crossings_words, void* stream) {
   return downstream(volume, channels, box, dims, omegas, toward, num_directions, panel, diagonal, out, os_k, os_c,
-                    os_v, crossings, crossings_words, true, stream);
+                    os_v, crossings, crossings_words, true, false, stream);
+}
+
+extern "C" int citrus_downstream_cumulative_facing(const float* volume, int64_t channels, const double* box,
+                                                   const int64_t* dims, const float* omegas, int64_t num_directions,
+                                                   const double* panel, double diagonal, float* out, int64_t os_k,
+                                                   int64_t os_c, int64_t os_v, int32_t* crossings,
+                                                   int64_t crossings_words, int32_t build, void* stream) {
+  return downstream(volume, channels, box, dims, omegas, nullptr, num_directions, panel, diagonal, out, os_k, os_c,
+                    os_v, crossings, crossings_words, build != 0, true, stream);
 }
 
 namespace citrus {
@@ -1006,7 +1026,7 @@ namespace {
 int downstream(const float* volume, int64_t channels, const double* box, const int64_t* dims, const float* omegas,
                const uint8_t* toward, int64_t num_directions, const double* panel, double diagonal, float* out,
                int64_t os_k, int64_t os_c, int64_t os_v, int32_t* crossings, int64_t crossings_words, bool build,
-               void* stream) {
+               bool test_facing, void* stream) {
   int status = check_common(volume, channels, box, dims, out);
   if (status) return status;
   CITRUS_REQUIRE(omegas && panel, "citrus_downstream_cumulative: null directions or panel");
@@ -1014,6 +1034,7 @@ int downstream(const float* volume, int64_t channels, const double* box, const i
   if (num_directions == 0) return CITRUS_OK;
   Panel p;
   p.curved = panel[0] != 0.0;
+  p.test_facing = test_facing;
   for (int a = 0; a < 3; ++a) {
     p.center[a] = (float)panel[1 + a];
     p.normal[a] = (float)panel[4 + a];

@@ -218,8 +218,6 @@ class GB300Projectors:
         device = mu.device
         omegas = omegas.to(device=device, dtype=torch.float32).reshape(-1, 3).contiguous()
         K = omegas.shape[0]
-        n = [float(v) for v in geometry.panel_axes(angle)[2]]
-        toward = ((omegas[:, 0] * -n[0] + omegas[:, 1] * -n[1] + omegas[:, 2] * -n[2]) > 0).to(torch.uint8)
         C, V = int(mu.shape[0]), grid.num_voxels
         if voxel_major:
             out = torch.empty(K, V, C, device=device, dtype=torch.float32)
@@ -238,15 +236,13 @@ class GB300Projectors:
             if (crossings.dtype != torch.int32 or not crossings.is_contiguous()
                     or tuple(crossings.shape) != (K, 3 * E) or crossings.device != device):
                 raise ValueError(f"crossings must be the contiguous int32 [{K}, {3 * E}] tables of these directions")
-            _lib.call("citrus_downstream_cumulative_tables", vol.data_ptr(), mu.shape[0], box, dims,
-                      omegas.data_ptr(), toward.data_ptr(), K, panel_args(host, geometry, angle), diagonal,
-                      out.data_ptr(), *strides, crossings.data_ptr(), crossings.numel(), _lib.stream_handle(device))
-            return out
-        crossings = torch.empty(3 * E * K, dtype=torch.int32, device=device) if lattice else None
-        _lib.call("citrus_downstream_cumulative", vol.data_ptr(), mu.shape[0], box, dims, omegas.data_ptr(),
-                  toward.data_ptr(), K, panel_args(host, geometry, angle), diagonal, out.data_ptr(), *strides,
-                  None if crossings is None else crossings.data_ptr(), 0 if crossings is None else crossings.numel(),
-                  _lib.stream_handle(device))
+            build = False
+        else:
+            crossings = torch.empty(3 * E * K, dtype=torch.int32, device=device) if lattice else None
+            build = lattice
+        _lib.call("citrus_downstream_cumulative_facing", vol.data_ptr(), mu.shape[0], box, dims, omegas.data_ptr(), K,
+                  panel_args(host, geometry, angle), diagonal, out.data_ptr(), *strides, _lib.ptr(crossings),
+                  0 if crossings is None else crossings.numel(), int(build), _lib.stream_handle(device))
         return out
 
     # ---- (d) oblique --------------------------------------------------------------------------------------------

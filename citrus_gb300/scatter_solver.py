@@ -5,7 +5,7 @@ correction and moment source, scattering-moment source, transport sweep, source 
 scatter image, primary, ``solve_view`` — so that the per-view CITRUS step (``citrus_step``) calls the same surface.
 Every stage runs on the device through ``libcitrus_gb300.so``; the caches of the reference (transport grids, sweep
 contexts, cone direction sets, direction contexts) are kept, sized for a GB300 (an 8 GiB sweep store per chunk and
-up to 64 image directions per chunk instead of the reference's 512 MiB and 32).
+up to 512 image directions per chunk instead of the reference's 512 MiB and 32).
 """
 
 from __future__ import annotations
@@ -37,7 +37,11 @@ from .uncollided import (FirstCollisionSamplingCorrection, first_collision_means
 
 SWEEP_CHUNK_BUDGET_BYTES = 8 * 2 ** 30
 IMAGE_CHUNK_BUDGET_BYTES = 4 * 2 ** 30
-IMAGE_CHUNK_MAX_DIRECTIONS = 64
+# Directions per image chunk at most. A chunk is 17 launches and about 0.5 ms of host work, and its buffers are past L2
+# from a few directions on, so the budget is the limit that matters: with chunks of 64 the image of a 32^3 grid with
+# one group waited for the host (whole view step 5.9 ms; one chunk of 512 directions: 3.0 ms), and an image at 64^3 x 8
+# groups, whose budget is 112 directions, takes as long either way.
+IMAGE_CHUNK_MAX_DIRECTIONS = 512
 
 
 @dataclass(frozen=True)
@@ -193,7 +197,7 @@ class ScatterSolver:
         return q
 
     def image_direction_chunk(self, fields: MaterialFields) -> int:
-        """Directions per image chunk: as many as fit the budget, between ``direction_chunk`` and 64."""
+        """Directions per image chunk: as many as fit the budget, between ``direction_chunk`` and 512."""
         G = self.num_groups
         Rd, Cd = self.geometry.image_shape
         per_direction = 4 * G * (2 * fields.grid_quadrature.num_voxels + 2 * fields.grid_coarse.num_voxels

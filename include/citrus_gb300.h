@@ -212,6 +212,13 @@ int citrus_downstream_cumulative_tables(const float* volume, int64_t channels, c
                                         int64_t os_k, int64_t os_c, int64_t os_v, const int32_t* crossings,
                                         int64_t crossings_words, void* stream);
 
+/* The same with the directions that do not face the panel (omega . (-n_hat) <= 0, +inf) told from the panel's normal
+ * on the device; crossings null walks every ray by itself, else they are the tables, built here when build != 0. */
+int citrus_downstream_cumulative_facing(const float* volume, int64_t channels, const double* box, const int64_t* dims,
+                                        const float* omegas, int64_t num_directions, const double* panel,
+                                        double diagonal, float* out, int64_t os_k, int64_t os_c, int64_t os_v,
+                                        int32_t* crossings, int64_t crossings_words, int32_t build, void* stream);
+
 /* Line through every pixel centre (float64 pixels [rows, cols, 3]) along each direction, clipped to the box on both
  * sides (float64 set-up);
  * field [K or 1, V, C] with field_stride elements between directions (0: shared); out element (k, c, row, col) at
