@@ -8,9 +8,6 @@
 //     2x upsampling fused into the input staging (B is read at half resolution), and an optional ReLU. The same kernel
 //     runs the input gradient of a convolution (the transposed convolution: flipped taps, swapped channel roles,
 //     outputs split back into the A and B parts and the A part masked by its ReLU activation).
-//     A CTA computes a 4 x 8 x 8 brick of voxels x 16 output channels; per chunk of 4 input channels the haloed input
-//     brick and the chunk's weights (tap-major, 16 output channels contiguous for float4 broadcasts) are staged in
-//     shared memory.
 //   * wgrad_kernel: weight gradients as fixed-order reductions over (batch, voxel bricks), split over CTAs into
 //     partial sums that wgrad_reduce_kernel adds in split order (deterministic).
 //   * pooling (2x average), the upsampling's backward pass, MSE and Adam.
@@ -24,12 +21,9 @@ namespace citrus {
 namespace {
 
 constexpr int kConvThreads = 256;
-constexpr int kTZ = 4, kTY = 8, kTX = 8;  // voxel brick of one CTA (kTZ * kTY * kTX == kConvThreads)
-constexpr int kCoT = 16;                  // output channels of one CTA
-constexpr int kCiT = 4;                   // input channels per staging step
+constexpr int kTZ = 4, kTY = 8, kTX = 8;  // voxel brick of the weight gradient (kTZ * kTY * kTX == kConvThreads)
+constexpr int kCoT = 16;                  // output channels of one CTA of the weight gradient
 constexpr int kLearnThreads = 256;
-
-__device__ __forceinline__ float bf16_bits_to_float(uint16_t b) { return __uint_as_float((uint32_t)b << 16); }
 
 struct ConvArgs {
   const float* in_a;      // [B, ca, D, H, W]
@@ -43,92 +37,227 @@ struct ConvArgs {
   int oa, ob;
   const float* mask_a;    // out_a *= (mask_a > 0) when set
   int relu;
+  int gradient;           // an input gradient, whose sums may be taken in parts
   int B, D, H, W;
 };
 
-template <int kK>
-__global__ void __launch_bounds__(kConvThreads) conv_kernel(const ConvArgs a) {
-  constexpr int kH = kK / 2;
-  constexpr int SZ = kTZ + 2 * kH, SY = kTY + 2 * kH, SX = kTX + 2 * kH, S3 = SZ * SY * SX;
-  constexpr int K3 = kK * kK * kK;
-  __shared__ float s_in[kCiT * S3];
-  __shared__ __align__(16) float s_w[kCiT * K3 * kCoT];
+// The convolution as a product C[voxel, o] over k = (input channel, tap), the voxels of the whole batch in one row. A
+// group of kThreads threads takes kTM kThreads / 8 voxels x 32 output channels, a thread kTM x 4 of them in registers (pairs of
+// voxels, two multiply-adds an instruction). The inputs of a channel's taps stream through a ring of three
+// shared-memory tiles [k][voxel] filled by asynchronous copies (a tap outside the volume is zero from the start and
+// never copied), the weights through registers into the other of two tiles [k][o] while the current one is used.
+// Every output adds its products in the order of (input channel, tap) to its bias, one rounded multiply-add each; with
+// kSplit > 1 the CTA's groups take every kSplit-th channel and their sums are added in group order.
+// Bound by shared memory: a thread reads 4 (kTM + 4) / (4 kTM) bytes per multiply-add where the FP32 pipe's rate leaves
+// one, and in the small levels by the chain of one output's sum. The kernel before this one took bricks of 4 x 8 x 8 voxels
+// of one sample, one voxel x 16 channels a thread, and waited for four input channels at a time, 2.2 us per channel
+// whatever the size: 32 -> 32 channels at 48 x 48 x 32 in 182 us, now 108 (38 TFLOP/s); 128 + 256 -> 128 at 12 x 12 x 8 in
+// 853 us, now 321; 256 -> 256 at 6 x 6 x 4 in 555 us, now 209; its input gradient at 4 x 3 x 3 x 2 in 490 us, now 98.
+constexpr int kTN = 4;  // output channels of a thread
 
-  const int tid = threadIdx.x;
-  const int ntx = (a.W + kTX - 1) / kTX, nty = (a.H + kTY - 1) / kTY;
-  const int tile = blockIdx.x;
-  const int x0 = (tile % ntx) * kTX, y0 = ((tile / ntx) % nty) * kTY, z0 = (tile / (ntx * nty)) * kTZ;
-  const int co0 = blockIdx.y * kCoT, b = blockIdx.z;
-  const int lx = tid % kTX, ly = (tid / kTX) % kTY, lz = tid / (kTX * kTY);
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+// both lanes' fused multiply-adds, each rounded as fmaf rounds
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
+// floats of one group's tiles
+template <int kK, int kTM, int kThreads, int kCI>
+constexpr int conv_group_floats() {
+  return kCI * kK * kK * kK * (3 * (kThreads / 8) * kTM + 2 * (8 * kTN + 4));
+}
+
+template <int kK, int kTM, int kThreads, int kCI, int kSplit>
+__global__ void __launch_bounds__(kThreads * kSplit) conv_kernel(const ConvArgs a, int64_t M) {
+  constexpr int K3 = kK * kK * kK, kH = kK / 2, KC = kCI * K3;
+  constexpr int TM = (kThreads / 8) * kTM, TN = 8 * kTN, kPitch = TN + 4;
+  constexpr int kGroups = kThreads / TM;                                    // threads that share a voxel's taps
+  constexpr int kTaps = (KC + kGroups - 1) / kGroups;                           // taps a thread stages per chunk
+  constexpr int kWeights = (KC * TN + kThreads - 1) / kThreads;         // weights a thread stages per chunk
+  extern __shared__ float4 s_conv[];
+  const int tid = threadIdx.x % kThreads, part = threadIdx.x / kThreads;
+  float* s_in = reinterpret_cast<float*>(s_conv) + part * conv_group_floats<kK, kTM, kThreads, kCI>();  // [3][KC][TM]
+  float* s_w = s_in + 3 * KC * TM;                                             // [2][KC][kPitch]
+
   const int O = a.oa + a.ob, Ci = a.ca + a.cb;
-  const int64_t V = (int64_t)a.D * a.H * a.W;
-  const int Dc = a.D >> 1, Hc = a.H >> 1, Wc = a.W >> 1;
-
-  float acc[kCoT];
+  const int V = a.D * a.H * a.W, Hc = a.H >> 1, Wc = a.W >> 1;
+  const int Vb = a.b_up ? (a.D >> 1) * Hc * Wc : V;
+  // the voxel this thread stages: the offsets of its taps from a sample's channel, negative outside the volume
+  const int64_t m0 = (int64_t)blockIdx.x * TM;
+  const int ms = tid % TM, group = tid / TM;
+  const int64_t sample = m0 + ms < M ? (m0 + ms) / V : 0;
+  const int vox_s = (int)(m0 + ms - sample * V), zs = vox_s / (a.H * a.W), ys = vox_s / a.W % a.H, xs = vox_s % a.W;
+  int offset[kTaps];
+  auto tap_offsets = [&](bool up) {
 #pragma unroll
-  for (int j = 0; j < kCoT; ++j) acc[j] = (a.bias != nullptr && co0 + j < O) ? a.bias[co0 + j] : 0.f;
-
-  for (int ci0 = 0; ci0 < Ci; ci0 += kCiT) {
-    __syncthreads();
-    for (int e = tid; e < kCiT * S3; e += kConvThreads) {
-      const int c = e / S3, r = e % S3;
-      const int gz = z0 + r / (SY * SX) - kH, gy = y0 + (r / SX) % SY - kH, gx = x0 + r % SX - kH;
-      const int ci = ci0 + c;
-      float v = 0.f;
-      if (ci < Ci && gz >= 0 && gz < a.D && gy >= 0 && gy < a.H && gx >= 0 && gx < a.W) {
-        if (ci < a.ca) {
-          v = __ldg(a.in_a + ((int64_t)b * a.ca + ci) * V + ((int64_t)gz * a.H + gy) * a.W + gx);
-        } else if (a.b_up) {
-          v = __ldg(a.in_b + (((int64_t)b * a.cb + (ci - a.ca)) * Dc + (gz >> 1)) * Hc * Wc + (int64_t)(gy >> 1) * Wc +
-                    (gx >> 1));
-        } else {
-          v = __ldg(a.in_b + ((int64_t)b * a.cb + (ci - a.ca)) * V + ((int64_t)gz * a.H + gy) * a.W + gx);
-        }
+    for (int e = 0; e < kTaps; ++e) {
+      const int k = e * kGroups + group, t = k % K3;
+      const int z = zs + t / (kK * kK) - kH, y = ys + (t / kK) % kK - kH, x = xs + t % kK - kH;
+      const bool inside = k < KC && m0 + ms < M && z >= 0 && z < a.D && y >= 0 && y < a.H && x >= 0 && x < a.W;
+      const int at = up ? ((z >> 1) * Hc + (y >> 1)) * Wc + (x >> 1) : (z * a.H + y) * a.W + x;
+      offset[e] = inside ? at : -1;
+    }
+  };
+  bool in_b = a.ca == 0;
+  tap_offsets(in_b && a.b_up);
+  const int co0 = blockIdx.y * TN;
+  const int chunks = ((Ci + kCI - 1) / kCI - part + kSplit - 1) / kSplit;   // this group's: part, part + kSplit, ..
+  auto load_inputs = [&](int j) {
+    if (j < chunks) {
+      const int first = (part + j * kSplit) * kCI;
+      if (!in_b && first >= a.ca) {
+        in_b = true;
+        tap_offsets(a.b_up);
       }
-      s_in[e] = v;
+      const float* src = in_b ? a.in_b + (sample * a.cb + (first - a.ca)) * Vb : a.in_a + (sample * a.ca + first) * V;
+      const uint32_t tile = smem_u32(s_in + j % 3 * KC * TM + ms);
+      // predicated, not branched around: a branch per copy serialises the copies' address loads (60 cycles each)
+#pragma unroll
+      for (int e = 0; e < kTaps; ++e) {
+        const int k = e * kGroups + group, c = k / K3;
+        const int at = kCI == 1 || first + c < Ci ? offset[e] : -1;
+        const float* from = src + (kCI > 1 ? (int64_t)c * (in_b ? Vb : V) : 0) + offset[e];
+        asm volatile("{\n.reg .pred p;\nsetp.ge.s32 p, %2, 0;\n@p cp.async.ca.shared.global [%0], [%1], 4;\n}" ::"r"(
+                         tile + k * TM * 4),
+                     "l"(from), "r"(at));
+      }
     }
-    for (int e = tid; e < kCiT * K3 * kCoT; e += kConvThreads) {
-      const int j = e % kCoT, t = (e / kCoT) % K3, c = e / (kCoT * K3);
-      const int o = co0 + j, i = ci0 + c;
-      s_w[e] = (o < O && i < Ci) ? bf16_bits_to_float(a.w[a.w_base + o * a.w_o + i * a.w_i + t * a.w_t]) : 0.f;
+    asm volatile("cp.async.commit_group;");
+  };
+  int w_at[kWeights];                              // element of the weight at channel 0 (some valid one past the outputs)
+#pragma unroll
+  for (int u = 0; u < kWeights; ++u) {
+    const int e = u * kThreads + tid, j = e / KC, k = e - j * KC, c = k / K3, t = k - c * K3;
+    w_at[u] = (int)(a.w_base + min(co0 + j, O - 1) * a.w_o + (kCI > 1 ? c : 0) * a.w_i + t * a.w_t);
+  }
+  uint32_t w[kWeights];
+  auto load_weights = [&](int j) {
+    const int first = (part + j * kSplit) * kCI;
+    const uint16_t* src = a.w + (int64_t)first * a.w_i;
+#pragma unroll
+    for (int u = 0; u < kWeights; ++u) {
+      const int c = (u * kThreads + tid) % KC / K3;
+      w[u] = kCI == 1 || first + c < Ci ? __ldg(src + w_at[u]) : 0u;
+    }
+  };
+  auto store_weights = [&](int j) {
+#pragma unroll
+    for (int u = 0; u < kWeights; ++u) {
+      const int e = u * kThreads + tid, o = e / KC, k = e - o * KC;
+      if (e < KC * TN) s_w[((j & 1) * KC + k) * kPitch + o] = __uint_as_float(w[u] << 16);
+    }
+  };
+  auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(part + 1), "n"(kThreads) : "memory"); };
+
+  const int tn = tid % 8, tm = tid / 8;            // this thread's channels and voxels of the tile
+  uint64_t acc[kTN][kTM / 2];
+#pragma unroll
+  for (int j = 0; j < kTN; ++j) {
+    const int o = co0 + tn * kTN + j;
+    const float bias = part == 0 && a.bias != nullptr && o < O ? a.bias[o] : 0.f;
+#pragma unroll
+    for (int p = 0; p < kTM / 2; ++p) acc[j][p] = pack2(bias, bias);
+  }
+  for (int e = tid; e < 3 * KC * TM; e += kThreads) s_in[e] = 0.f;
+  __syncthreads();
+  load_inputs(0);
+  load_inputs(1);
+  if (chunks > 0) {
+    load_weights(0);
+    store_weights(0);
+  }
+  for (int j = 0; j < chunks; ++j) {
+    asm volatile("cp.async.wait_group 1;");
+    group_sync();  // this chunk's tiles are filled, and nobody reads the ones of the chunk before it any more
+    load_inputs(j + 2);
+    if (j + 1 < chunks) load_weights(j + 1);
+    const float* in = s_in + j % 3 * KC * TM + tm * kTM;
+    const float* wt = s_w + (j & 1) * KC * kPitch + tn * kTN;
+    auto multiply = [&](int k) {
+      uint64_t x[kTM / 2];
+      float wk[kTN];
+#pragma unroll
+      for (int p = 0; p < kTM / 4; ++p) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(in + k * TM + 4 * p);
+        x[2 * p] = v.x;
+        x[2 * p + 1] = v.y;
+      }
+#pragma unroll
+      for (int q = 0; q < kTN; q += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(wt + k * kPitch + q);
+        wk[q] = v.x, wk[q + 1] = v.y, wk[q + 2] = v.z, wk[q + 3] = v.w;
+      }
+#pragma unroll
+      for (int q = 0; q < kTN; ++q) {
+        const uint64_t ww = pack2(wk[q], wk[q]);
+#pragma unroll
+        for (int p = 0; p < kTM / 2; ++p) acc[q][p] = fma2(ww, x[p], acc[q][p]);
+      }
+    };
+    const int first = (part + j * kSplit) * kCI;
+    if (kCI == 1 || first + kCI <= Ci) {
+#pragma unroll 9
+      for (int k = 0; k < KC; ++k) multiply(k);
+    } else {
+      for (int k = 0; k < (Ci - first) * K3; ++k) multiply(k);
+    }
+    if (j + 1 < chunks) store_weights(j + 1);
+  }
+  if (kSplit > 1) {  // the groups' sums, added in group order by the first
+    asm volatile("cp.async.wait_all;");
+    __syncthreads();
+    uint64_t* s_sum = reinterpret_cast<uint64_t*>(s_conv);                      // [kSplit - 1][kTN kTM / 2][128]
+    constexpr int kPairs = kTN * (kTM / 2);
+    if (part > 0) {
+#pragma unroll
+      for (int q = 0; q < kPairs; ++q)
+        s_sum[((part - 1) * kPairs + q) * kThreads + tid] = acc[q / (kTM / 2)][q % (kTM / 2)];
     }
     __syncthreads();
+    if (part > 0) return;
 #pragma unroll
-    for (int c = 0; c < kCiT; ++c) {
-#pragma unroll
-      for (int tz = 0; tz < kK; ++tz)
-#pragma unroll
-        for (int ty = 0; ty < kK; ++ty)
-#pragma unroll
-          for (int tx = 0; tx < kK; ++tx) {
-            const float v = s_in[c * S3 + ((lz + tz) * SY + (ly + ty)) * SX + lx + tx];
-            const float4* w4 = reinterpret_cast<const float4*>(s_w + (c * K3 + (tz * kK + ty) * kK + tx) * kCoT);
-#pragma unroll
-            for (int q = 0; q < kCoT / 4; ++q) {
-              const float4 wq = w4[q];
-              acc[4 * q + 0] = fmaf(wq.x, v, acc[4 * q + 0]);
-              acc[4 * q + 1] = fmaf(wq.y, v, acc[4 * q + 1]);
-              acc[4 * q + 2] = fmaf(wq.z, v, acc[4 * q + 2]);
-              acc[4 * q + 3] = fmaf(wq.w, v, acc[4 * q + 3]);
-            }
-          }
+    for (int q = 0; q < kPairs; ++q) {
+      float2 sum = unpack2(acc[q / (kTM / 2)][q % (kTM / 2)]);
+      for (int g = 0; g < kSplit - 1; ++g) {
+        const float2 v = unpack2(s_sum[(g * kPairs + q) * kThreads + tid]);
+        sum.x += v.x;
+        sum.y += v.y;
+      }
+      acc[q / (kTM / 2)][q % (kTM / 2)] = pack2(sum.x, sum.y);
     }
   }
 
-  const int x = x0 + lx, y = y0 + ly, z = z0 + lz;
-  if (x >= a.W || y >= a.H || z >= a.D) return;
-  const int64_t vox = ((int64_t)z * a.H + y) * a.W + x;
 #pragma unroll
-  for (int j = 0; j < kCoT; ++j) {
-    const int o = co0 + j;
-    if (o >= O) break;
-    float r = a.relu ? fmaxf(acc[j], 0.f) : acc[j];
-    if (o < a.oa) {
-      const int64_t idx = ((int64_t)b * a.oa + o) * V + vox;
-      if (a.mask_a != nullptr && !(a.mask_a[idx] > 0.f)) r = 0.f;
-      a.out_a[idx] = r;
-    } else {
-      a.out_b[((int64_t)b * a.ob + (o - a.oa)) * V + vox] = r;
+  for (int p = 0; p < kTM; ++p) {
+    const int64_t m = m0 + tm * kTM + p;
+    if (m >= M) break;
+    const int64_t b = m / V;
+    const int vox = (int)(m - b * V);
+#pragma unroll
+    for (int j = 0; j < kTN; ++j) {
+      const int o = co0 + tn * kTN + j;
+      if (o >= O) break;
+      const float2 v = unpack2(acc[j][p / 2]);
+      float r = p % 2 ? v.y : v.x;
+      if (a.relu) r = fmaxf(r, 0.f);
+      if (o < a.oa) {
+        const int64_t idx = (b * a.oa + o) * V + vox;
+        if (a.mask_a != nullptr && !(a.mask_a[idx] > 0.f)) r = 0.f;
+        a.out_a[idx] = r;
+      } else {
+        a.out_b[(b * a.ob + (o - a.oa)) * V + vox] = r;
+      }
     }
   }
 }
@@ -620,18 +749,50 @@ int launch_conv_tc_k(const ConvArgs& a, uint32_t* error_word, cudaStream_t s) {
   return CITRUS_OK;
 }
 
+template <int kK, int kTM, int kThreads, int kCI, int kSplit>
+int launch_conv_tile(const ConvArgs& a, cudaStream_t s) {
+  constexpr int TM = (kThreads / 8) * kTM, TN = 8 * kTN;
+  const int64_t M = (int64_t)a.B * a.D * a.H * a.W;
+  constexpr size_t tiles_bytes = (size_t)kSplit * conv_group_floats<kK, kTM, kThreads, kCI>() * sizeof(float);
+  constexpr size_t sums_bytes = (size_t)(kSplit - 1) * kTM * kTN * kThreads * sizeof(float);
+  constexpr size_t smem = tiles_bytes > sums_bytes ? tiles_bytes : sums_bytes;
+  cudaError_t e = cudaFuncSetAttribute(conv_kernel<kK, kTM, kThreads, kCI, kSplit>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return set_error(CITRUS_ECUDA, "conv3d: %s", cudaGetErrorString(e));
+  const int64_t tiles = cdiv(M, TM);
+  CITRUS_REQUIRE((int64_t)(a.ca + a.cb) * (a.oa + a.ob) * kK * kK * kK < (1ll << 31), "conv3d: too many weights");
+  CITRUS_REQUIRE(tiles < (1ll << 31), "conv3d: too many voxel tiles");
+  dim3 grid((unsigned)tiles, (unsigned)cdiv(a.oa + a.ob, TN));
+  conv_kernel<kK, kTM, kThreads, kCI, kSplit><<<grid, kThreads * kSplit, smem, s>>>(a, M);
+  note_launches();
+  return CITRUS_OK;
+}
+
+template <int kK>
+int launch_conv_simt_k(const ConvArgs& a, cudaStream_t s) {
+  constexpr int kCI = kK == 3 ? 1 : 16;  // input channels of a chunk, a tap each for 1^3 kernels
+  const int64_t M = (int64_t)a.B * a.D * a.H * a.W, O = a.oa + a.ob;
+  auto tiles = [&](int tm) { return cdiv(M, tm) * cdiv(O, 32); };
+  // a chunk of several channels takes them from one input
+  if (a.cb > 0 && a.ca % kCI != 0) return launch_conv_tile<kK, 4, 128, 1, 1>(a, s);
+  // 8 voxels a thread read 1.5 bytes of shared memory per multiply-add, 4 read 2: the larger tile wherever it fills the
+  // SMs (32 -> 32 channels at 48 x 48 x 32: 108 us, 137 with 4; 64 -> 64 at 24 x 24 x 16, 144 tiles: 78 and 80), the
+  // smaller where it does not (64 -> 64 at 4 x 12 x 12 x 8, 72 and 144 tiles: 78 and 59). Below 128 tiles a gradient sums its
+  // channels in four parts, half the tile each (256 -> 256 at 4 x 3 x 3 x 2, 16 tiles: 216 and 98). An activation
+  // never does: its sign decides the ReLU's gradient, and the sum of one part gives the same bits at every size.
+  if constexpr (kK == 3) {
+    if (tiles(128) >= 128) return launch_conv_tile<kK, 8, 128, kCI, 1>(a, s);
+    if (a.gradient && tiles(64) < 128) return launch_conv_tile<kK, 4, 64, kCI, 4>(a, s);
+  }
+  return launch_conv_tile<kK, 4, 128, kCI, 1>(a, s);
+}
+
 // variant 1: the FP32 SIMT kernel; variant 2 (and 0): the tcgen05 implicit GEMM
 int launch_conv(const ConvArgs& a, int kernel_size, int variant, uint32_t* error_word, cudaStream_t s) {
   if (variant != 1) {
     return kernel_size == 3 ? launch_conv_tc_k<3>(a, error_word, s) : launch_conv_tc_k<1>(a, error_word, s);
   }
-  const int64_t tiles = cdiv(a.W, kTX) * cdiv(a.H, kTY) * cdiv(a.D, kTZ);
-  CITRUS_REQUIRE(tiles < (1ll << 31), "conv3d: too many voxel bricks");
-  dim3 grid((unsigned)tiles, (unsigned)cdiv(a.oa + a.ob, kCoT), (unsigned)a.B);
-  if (kernel_size == 3) conv_kernel<3><<<grid, kConvThreads, 0, s>>>(a);
-  else conv_kernel<1><<<grid, kConvThreads, 0, s>>>(a);
-  note_launches();
-  return CITRUS_OK;
+  return kernel_size == 3 ? launch_conv_simt_k<3>(a, s) : launch_conv_simt_k<1>(a, s);
 }
 
 }  // namespace
@@ -657,7 +818,7 @@ extern "C" int citrus_conv3d_forward_config(const float* in_a, int64_t channels_
   const int64_t k3 = (int64_t)kernel_size * kernel_size * kernel_size;
   ConvArgs a{in_a, in_b, (int)channels_a, (int)channels_b, b_upsampled ? 1 : 0,
              weight, (channels_a + channels_b) * k3, k3, 1, 0,
-             bias, out, nullptr, (int)channels_out, 0, nullptr, relu ? 1 : 0,
+             bias, out, nullptr, (int)channels_out, 0, nullptr, relu ? 1 : 0, 0,
              (int)batch, (int)depth, (int)height, (int)width};
   CITRUS_REQUIRE(variant >= 0 && variant <= 2, "citrus_conv3d_forward: variant %d (0 auto, 1 SIMT, 2 tensor cores)",
                  variant);
@@ -696,7 +857,7 @@ extern "C" int citrus_conv3d_backward_input_config(const float* grad_out, int64_
   // taps flipped
   ConvArgs a{grad_out, nullptr, (int)channels_out, 0, 0,
              weight, k3, ci * k3, -1, k3 - 1,
-             nullptr, grad_a, grad_b, (int)channels_a, (int)channels_b, mask_a, 0,
+             nullptr, grad_a, grad_b, (int)channels_a, (int)channels_b, mask_a, 0, 1,
              (int)batch, (int)depth, (int)height, (int)width};
   CITRUS_REQUIRE(variant >= 0 && variant <= 2,
                  "citrus_conv3d_backward_input: variant %d (0 auto, 1 SIMT, 2 tensor cores)", variant);

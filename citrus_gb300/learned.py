@@ -152,7 +152,8 @@ class ConvNet3D:
         from .autotune import Autotuner, tuner
 
         B, D, H, W = shape
-        key = Autotuner.key(op, self.device, B=B, D=D, H=H, W=W, ca=layer.c_a, cb=layer.c_b, co=layer.c_out,
+        # "tiles" names the float32 kernel: choices timed against the one before it are not reused
+        key = Autotuner.key(op + "_tiles", self.device, B=B, D=D, H=H, W=W, ca=layer.c_a, cb=layer.c_b, co=layer.c_out,
                             k=layer.k, up=int(layer.b_up))
         return int(tuner().choose(key, [2, 1], run, 2))
 
