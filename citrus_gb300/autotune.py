@@ -132,7 +132,8 @@ def small_k_gemm_config(A, B, C, M: int, K: int, J: int, batch: int, sb: int, sc
                         tensor_cores=None) -> list:
     """(variant, tile rows) of the small-K product for this shape, tuned into a scratch output: the float32 forms,
     and the tensor-core product ([3, 0]) when ``tensor_cores(out, ld_out, stride_out)`` runs it."""
-    key = Autotuner.key("small_k_gemm" + ("_bf16x3" if tensor_cores else ""), A.device, M=M, K=K, J=J, batch=batch,
+    # "quads" names the streaming forms: choices timed against those of two columns per thread are not reused
+    key = Autotuner.key("small_k_gemm_quads" + ("_bf16x3" if tensor_cores else ""), A.device, M=M, K=K, J=J, batch=batch,
                         acc=int(bool(accumulate)),
                         aligned=int(J % 4 == 0 and B.stride(1) % 4 == 0 and C.stride(1) % 4 == 0))
     entry = tuner().table.get(key)

@@ -31,6 +31,25 @@ void note_launches(int n = 1);
     if (!(cond)) return ::citrus::set_error(CITRUS_EINVAL, __VA_ARGS__); \
   } while (0)
 
+// ---- pairs of floats in one 64-bit register --------------------------------------------------------------------
+// fma.rn.f32x2 rounds each lane as fmaf does; it has the FP32 pipe's rate (75 TFLOP/s measured, as scalar multiply-adds)
+// at half the issue slots, which leaves the others to loads and address arithmetic.
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
 // ---- memory-ordering helpers ----------------------------------------------------------------------------------
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
   unsigned v;

@@ -296,6 +296,171 @@ __global__ void __launch_bounds__(kStreamThreads) gemm_rows_kernel(const float* 
   }
 }
 
+// The streaming forms over four columns per thread, in pairs (fma2). A value of A read from shared memory as part of a
+// float4 costs a wavefront per 128 bytes delivered, broadcast or not, so two columns a thread spend twice the
+// cycles on reading A that the FP32 pipe spends on its products; four balance them. The columns or outputs of four columns
+// are 4 K or 4 M registers, hence K, M <= 36. The sums are those of the forms above, bit for bit. 120 x 36 on 8.4 M
+// columns (64^3 cells, 8 groups; 5.2 GB, 36 G multiply-adds): the expansion 1.64 -> 1.51 ms
+// (with means 2.31 -> 1.88), the accumulation 2.09 -> 1.55.
+template <int kKP, int kMode>
+__global__ void __launch_bounds__(kStreamThreads) gemm_cols4_kernel(const float* __restrict__ A, int64_t lda,
+                                                                   const float* __restrict__ B, int64_t ldb,
+                                                                   float* __restrict__ C, int64_t ldc, int M, int K,
+                                                                   int64_t J, int64_t stride_b, int64_t stride_c,
+                                                                   const float* __restrict__ F, int64_t ldf,
+                                                                   int64_t stride_f) {
+  extern __shared__ float4 s_a4[];
+  float (*As)[kKP] = reinterpret_cast<float (*)[kKP]>(s_a4);  // [kStreamRows + 3][kKP], zero past the tile
+  const int row0 = blockIdx.y * kStreamRows;
+  const int rows = min(kStreamRows, M - row0);
+  for (int i = threadIdx.x; i < (kStreamRows + 3) * kKP; i += kStreamThreads) {
+    const int r = i / kKP, k = i % kKP;
+    As[r][k] = (r < rows && k < K) ? A[(int64_t)(row0 + r) * lda + k] : 0.f;
+  }
+  const int64_t col = ((int64_t)blockIdx.x * kStreamThreads + threadIdx.x) * 4;
+  const bool valid = col < J;
+  B += blockIdx.z * stride_b + col;
+  C += blockIdx.z * stride_c + col;
+  if (kMode == 2) F += blockIdx.z * stride_f + (col >> 2);
+  uint64_t b01[kKP], b23[kKP];
+#pragma unroll
+  for (int k = 0; k < kKP; ++k) {
+    ulonglong2 v = make_ulonglong2(0, 0);
+    if (valid && k < K) v = *reinterpret_cast<const ulonglong2*>(B + (int64_t)k * ldb);
+    b01[k] = v.x;
+    b23[k] = v.y;
+  }
+  __syncthreads();
+  if (!valid) return;
+  // the means of the next four rows are in flight during the products of the current ones
+  float next[4] = {0.f, 0.f, 0.f, 0.f};
+  auto load_means = [&](int r0) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) next[q] = r0 + q < rows ? __ldg(F + (int64_t)(row0 + r0 + q) * ldf) : 0.f;
+  };
+  if (kMode == 2) load_means(0);
+  for (int r0 = 0; r0 < rows; r0 += 4) {
+    uint64_t a01[4] = {0, 0, 0, 0}, a23[4] = {0, 0, 0, 0};
+    float f[4] = {next[0], next[1], next[2], next[3]};
+    if (kMode == 2) load_means(r0 + 4);
+#pragma unroll
+    for (int k = 0; k < kKP; k += 4) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float4 a = *reinterpret_cast<const float4*>(&As[r0 + q][k]);  // rows past the tile are zero
+        const float av[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint64_t aa = pack2(av[i], av[i]);
+          a01[q] = fma2(aa, b01[k + i], a01[q]);
+          a23[q] = fma2(aa, b23[k + i], a23[q]);
+        }
+      }
+    }
+    float* out = C + (int64_t)(row0 + r0) * ldc;
+    float4 o[4];
+    if (kMode == 1) {  // the four loads before the first store
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        o[q] = r0 + q < rows ? *reinterpret_cast<const float4*>(out + (int64_t)q * ldc) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (r0 + q >= rows) break;
+      const float2 lo = unpack2(a01[q]), hi = unpack2(a23[q]);
+      float4 v = make_float4(lo.x, lo.y, hi.x, hi.y);
+      if (kMode == 1) v = make_float4(v.x + o[q].x, v.y + o[q].y, v.z + o[q].z, v.w + o[q].w);
+      if (kMode == 2) v.x += f[q];
+      *reinterpret_cast<float4*>(out + (int64_t)q * ldc) = v;
+    }
+  }
+}
+
+template <int kMP, bool kAccumulate>
+__global__ void __launch_bounds__(kStreamThreads) gemm_rows4_kernel(const float* __restrict__ A, int64_t lda,
+                                                                   const float* __restrict__ B, int64_t ldb,
+                                                                   float* __restrict__ C, int64_t ldc, int M, int K,
+                                                                   int64_t J, int64_t stride_b, int64_t stride_c) {
+  extern __shared__ float4 s_at4[];
+  float* At = reinterpret_cast<float*>(s_at4);  // [K][kMP], A transposed, zero rows past M
+  for (int i = threadIdx.x; i < K * kMP; i += kStreamThreads) {
+    const int k = i / kMP, r = i % kMP;
+    At[i] = r < M ? A[(int64_t)r * lda + k] : 0.f;
+  }
+  const int64_t col = ((int64_t)blockIdx.x * kStreamThreads + threadIdx.x) * 4;
+  B += blockIdx.z * stride_b + col;
+  C += blockIdx.z * stride_c + col;
+  __syncthreads();
+  if (col >= J) return;
+  uint64_t c[kMP / 2][4];  // pairs of rows, so that a pair of A needs no packing
+#pragma unroll
+  for (int r = 0; r < kMP / 2; ++r)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) c[r][j] = 0;
+  auto product = [&](int k, float4 x) {
+    const ulonglong2* at = reinterpret_cast<const ulonglong2*>(At + k * kMP);
+    const uint64_t xx[4] = {pack2(x.x, x.x), pack2(x.y, x.y), pack2(x.z, x.z), pack2(x.w, x.w)};
+#pragma unroll
+    for (int r = 0; r < kMP / 2; r += 2) {
+      const ulonglong2 a = at[r / 2];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) c[r][j] = fma2(a.x, xx[j], c[r][j]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) c[r + 1][j] = fma2(a.y, xx[j], c[r + 1][j]);
+    }
+  };
+  // the loads of the next kU rows of B are in flight during the products of the current ones
+  constexpr int kU = 4;
+  float4 x[kU];
+#pragma unroll
+  for (int u = 0; u < kU; ++u)
+    x[u] = u < K ? __ldg(reinterpret_cast<const float4*>(B + (int64_t)u * ldb)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int k = 0; k < K; k += kU) {
+    float4 next[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u)
+      next[u] = k + kU + u < K ? __ldg(reinterpret_cast<const float4*>(B + (int64_t)(k + kU + u) * ldb))
+                               : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      if (k + u < K) product(k + u, x[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < kU; ++u) x[u] = next[u];
+  }
+#pragma unroll
+  for (int r4 = 0; r4 < kMP; r4 += 4) {
+    float4 o[4];
+    if (kAccumulate) {  // four rows' loads before their stores
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        o[q] = r4 + q < M ? *reinterpret_cast<const float4*>(C + (int64_t)(r4 + q) * ldc)
+                          : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (r4 + q >= M) break;
+      float v[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 pair = unpack2(c[(r4 + q) / 2][j]);
+        v[j] = q % 2 ? pair.y : pair.x;
+      }
+      float4 w = make_float4(v[0], v[1], v[2], v[3]);
+      if (kAccumulate) w = make_float4(w.x + o[q].x, w.y + o[q].y, w.z + o[q].z, w.w + o[q].w);
+      *reinterpret_cast<float4*>(C + (int64_t)(r4 + q) * ldc) = w;
+    }
+  }
+}
+
+// Four columns per thread: whole float4s of B and C, and enough columns for the two blocks that an SM holds
+constexpr int kQuadMax = 36;
+inline bool quad_columns(const float* B, const float* C, int64_t ldb, int64_t ldc, int64_t stride_b, int64_t stride_c,
+                         int64_t J) {
+  return J % 4 == 0 && ldb % 4 == 0 && ldc % 4 == 0 && stride_b % 4 == 0 && stride_c % 4 == 0 &&
+         ((uintptr_t)B % 16) == 0 && ((uintptr_t)C % 16) == 0 && J >= 4 * kStreamThreads * 2 * (int64_t)num_sms();
+}
+
 template <int kKP, bool kPair, int kMode>
 int launch_cols(const float* A, int64_t lda, const float* B, int64_t ldb, float* C, int64_t ldc, int M, int K,
                 int64_t J, int64_t batch, int64_t stride_b, int64_t stride_c, cudaStream_t s,
@@ -306,6 +471,15 @@ int launch_cols(const float* A, int64_t lda, const float* B, int64_t ldb, float*
     cudaError_t e = cudaFuncSetAttribute(gemm_cols_kernel<kKP, kPair, kMode>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return set_error(CITRUS_ECUDA, "citrus_small_k_gemm: %s", cudaGetErrorString(e));
+  }
+  if constexpr (kKP <= kQuadMax && kPair) {
+    if (quad_columns(B, C, ldb, ldc, stride_b, stride_c, J)) {
+      dim3 quads((unsigned)cdiv(J, 4 * kStreamThreads), (unsigned)cdiv(M, kStreamRows), (unsigned)batch);
+      gemm_cols4_kernel<kKP, kMode><<<quads, kStreamThreads, smem, s>>>(A, lda, B, ldb, C, ldc, M, K, J, stride_b,
+                                                                        stride_c, F, ldf, stride_f);
+      note_launches();
+      return launch_status("citrus_small_k_gemm");
+    }
   }
   dim3 grid((unsigned)cdiv(J, cols_per_block), (unsigned)cdiv(M, kStreamRows), (unsigned)batch);
   gemm_cols_kernel<kKP, kPair, kMode><<<grid, kStreamThreads, smem, s>>>(A, lda, B, ldb, C, ldc, M, K, J, stride_b,
@@ -318,6 +492,20 @@ template <int kMP, bool kPair, bool kAcc>
 int launch_rows(const float* A, int64_t lda, const float* B, int64_t ldb, float* C, int64_t ldc, int M, int K,
                 int64_t J, int64_t batch, int64_t stride_b, int64_t stride_c, cudaStream_t s) {
   const size_t smem = (size_t)K * kMP * sizeof(float);
+  if constexpr (kMP <= kQuadMax && kPair) {
+    if (quad_columns(B, C, ldb, ldc, stride_b, stride_c, J)) {
+      if (smem > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_rows4_kernel<kMP, kAcc>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return set_error(CITRUS_ECUDA, "citrus_small_k_gemm: %s", cudaGetErrorString(e));
+      }
+      dim3 quads((unsigned)cdiv(J, 4 * kStreamThreads), 1, (unsigned)batch);
+      gemm_rows4_kernel<kMP, kAcc><<<quads, kStreamThreads, smem, s>>>(A, lda, B, ldb, C, ldc, M, K, J, stride_b,
+                                                                       stride_c);
+      note_launches();
+      return launch_status("citrus_small_k_gemm");
+    }
+  }
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(gemm_rows_kernel<kMP, kPair, kAcc>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

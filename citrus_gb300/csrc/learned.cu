@@ -55,23 +55,6 @@ struct ConvArgs {
 // 853 us, now 321; 256 -> 256 at 6 x 6 x 4 in 555 us, now 209; its input gradient at 4 x 3 x 3 x 2 in 490 us, now 98.
 constexpr int kTN = 4;  // output channels of a thread
 
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ float2 unpack2(uint64_t v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-// both lanes' fused multiply-adds, each rounded as fmaf rounds
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-
 // floats of one group's tiles
 template <int kK, int kTM, int kThreads, int kCI>
 constexpr int conv_group_floats() {
