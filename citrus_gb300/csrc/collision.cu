@@ -396,8 +396,8 @@ __global__ void fc_sums_kernel(FCInputs in, Table tb, PointGrid pg, const float*
 // all of the block's directions, and the transfer rows of the eta nodes that the block's points and directions touch are staged
 // in shared memory (the window). S_MC is either read ([K, G, NC], the reference's interface) or formed from the
 // scattering-source moments of the point's cell held in registers, T[n, g, cell] for n < N_sh, and the harmonics of
-// the block's directions in shared memory. The per-block sums are a fixed-order warp butterfly and a fixed-order sum
-// over the groups: deterministic.
+// the block's directions in shared memory. The per-block sums are a butterfly over the groups and one over the points:
+// deterministic.
 constexpr int kEmitPoints = 32;
 constexpr int kMaxMoments = 64;
 constexpr int kRegMoments = 36;  // scattering-source moments held in registers (P5); more are read per direction
@@ -425,21 +425,27 @@ __device__ __forceinline__ float row_dot(const float* __restrict__ row, const fl
 }
 
 // The window of table nodes a block needs: its points' cosines with its directions span a few dozen of the eta nodes,
-// so the rows of those nodes ([node][m][g][g'], each (node, m) block padded by 4 floats against bank conflicts) are
-// staged in shared memory once and every interpolation of the block reads them there.
+// so the rows of those nodes ([node][m][g][g']) are staged in shared memory once and every interpolation of the block
+// reads them there. The lanes' nodes are neighbours: a node's stride is 16 bytes (4 where rows are read as floats) past a
+// multiple of all banks, so that eight neighbouring nodes are read without conflicts (16 bytes per (node, m) let four).
 constexpr int kWindowBytes = 32 * 1024;
 
-__host__ __device__ inline int window_row_stride(int G) { return G * G + 4; }
+__host__ __device__ inline int window_node_stride(int M, int G) {
+  return (M * G * G + 31) / 32 * 32 + (G % 4 == 0 ? 4 : 1);
+}
 __host__ __device__ inline int window_nodes(int M, int G, int bytes = kWindowBytes) {
-  const int n = bytes / (4 * M * window_row_stride(G));
-  return n < 96 ? n : 96;
+  const int n = bytes / (4 * window_node_stride(M, G));
+  return n < 128 ? n : 128;
 }
 
 
 // Stages the table window of a block for the directions s_om[0..n): the eta nodes [lo, hi + 1] that its valid points
 // touch, if they fit, else s_window[0] = -1 (rows read from global memory). Each thread evaluates the directions
 // first_dir, first_dir + dir_step, ... for its point; s_range holds one (lo, hi) per warp. Ends with a block barrier;
-// every thread of the block must call it.
+// every thread of the block must call it. kG: the groups when they are known at compile time (else 0): the copy is
+// then shifts and asynchronous 16-byte copies, all in flight together; a division per (node, material) and a load waited
+// for at a time were a third of the sampling correction's instructions.
+template <int kG = 0>
 __device__ void stage_window(const Table& tb, bool valid, float ux, float uy, float uz, const float (*s_om)[3], int n,
                              int first_dir, int dir_step, int warp, int nwarps, int tid, int nthreads,
                              int (*s_range)[32], int* s_window, float* s_tab, int window_bytes = kWindowBytes) {
@@ -475,57 +481,82 @@ __device__ void stage_window(const Table& tb, bool valid, float ux, float uy, fl
   }
   __syncthreads();
   const int win_lo = s_window[0], win_n = s_window[1];
-  if (win_lo >= 0 && G % 4 == 0 && ((uintptr_t)tb.t % 16) == 0) {
-    // whole (node, material) blocks of G x G floats as float4, one block per warp at a time: no index division per
-    // element (the padded stride G G + 4 keeps every block 16-byte aligned)
-    const int RS = window_row_stride(G), GG4 = G * G / 4;
-    for (int nm = warp; nm < win_n * tb.M; nm += nwarps) {
-      const int node = nm / tb.M, m = nm - node * tb.M;
-      const float4* src = reinterpret_cast<const float4*>(tb.t + ((int64_t)m * tb.N + win_lo + node) * G * G);
-      float4* dst = reinterpret_cast<float4*>(s_tab + (node * tb.M + m) * RS);
-      for (int r = tid & 31; r < GG4; r += 32) dst[r] = __ldg(src + r);
+  if (kG > 0 && kG % 4 == 0 && win_lo >= 0 && ((uintptr_t)tb.t % 16) == 0) {
+    constexpr int GG4 = kG > 0 ? kG * kG / 4 : 1;
+    const int NS = window_node_stride(tb.M, G);
+    for (int m = 0; m < tb.M; ++m) {
+      const float4* src = reinterpret_cast<const float4*>(tb.t + ((int64_t)m * tb.N + win_lo) * (kG * kG));
+      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_tab + m * kG * kG);
+      for (int i = tid; i < win_n * GG4; i += nthreads)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (i / GG4) * NS * 4 + (i % GG4) * 16),
+                     "l"(src + i));
     }
-  } else if (win_lo >= 0) {
-    const int RS = window_row_stride(G);
-    const int per = tb.M * G * G;
-    for (int q = tid; q < win_n * per; q += nthreads) {
-      const int node = q / per, rem = q - node * per;
-      const int m = rem / (G * G), r = rem - m * G * G;
-      s_tab[(node * tb.M + m) * RS + r] = __ldg(tb.t + ((int64_t)m * tb.N + win_lo + node) * G * G + r);
-    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  } else if (win_lo >= 0) {  // a warp per node: no division per element here either
+    const int NS = window_node_stride(tb.M, G), GG = G * G, lane = tid & 31;
+    for (int m = 0; m < tb.M; ++m)
+      for (int node = warp; node < win_n; node += nwarps) {
+        const float* src = tb.t + ((int64_t)m * tb.N + win_lo + node) * GG;
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_tab + node * NS + m * GG);
+        for (int r = lane; r < GG; r += 32)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 4 * r), "l"(src + r));
+      }
+    asm volatile("cp.async.wait_all;" ::: "memory");
   }
   __syncthreads();
 }
 
+// the source between two nodes whose sums over the materials are f0 and f1
+__device__ __forceinline__ float interpolate_nodes(float f0, float f1, float w) {
+  return fmaf(__fsub_rn(f1, f0), w, f0);
+}
+
 // S_FC of group g at one point for one direction, rows from the window (win_lo >= 0) or from global memory
-// kWindow: 1 the rows are in the block's shared-memory window, 2 in global memory, 0 decided by win_lo >= 0
-template <int kGP, int kMM, int kWindow = 0>
+// kWindow: 1 the rows are in the block's shared-memory window, 2 in global memory, 0 decided by win_lo >= 0. kNodes: the
+// materials are summed at each node before the interpolation (as emission_warps_kernel's ring holds them), else after
+template <int kGP, int kMM, int kWindow = 0, bool kNodes = false>
 __device__ __forceinline__ float fc_group(const Table& tb, const float* s_tab, int win_lo, int i0, float w, int g,
                                           const float* rho, const float* phi) {
-  const int G = tb.G, RS = window_row_stride(G);
-  float src = 0.f;
+  const int G = tb.G, NS = window_node_stride(tb.M, G);
+  float f0 = 0.f, f1 = 0.f;
 #pragma unroll
   for (int m = 0; m < kMM; ++m) {
     const float r = rho[m];
     if (m >= tb.M || r == 0.f) continue;
     float a0, a1;
     if (kWindow == 1 || (kWindow == 0 && win_lo >= 0)) {
-      const float* row0 = s_tab + ((i0 - win_lo) * tb.M + m) * RS + g * G;
+      const float* row0 = s_tab + (i0 - win_lo) * NS + (m * G + g) * G;
       a0 = row_dot<kGP, true>(row0, phi, G);
-      a1 = row_dot<kGP, true>(row0 + tb.M * RS, phi, G);
+      a1 = row_dot<kGP, true>(row0 + NS, phi, G);
     } else {
       const float* row0 = tb.t + (((int64_t)m * tb.N + i0) * G + g) * G;
       a0 = row_dot<kGP, false>(row0, phi, G);
       a1 = row_dot<kGP, false>(row0 + (int64_t)G * G, phi, G);
     }
-    src = fmaf(r, a0 + (a1 - a0) * w, src);
+    if (kNodes) {
+      f0 = fmaf(r, a0, f0);
+      f1 = fmaf(r, a1, f1);
+    } else {
+      f0 = fmaf(r, a0 + (a1 - a0) * w, f0);
+    }
   }
-  return src;
+  return kNodes ? interpolate_nodes(f0, f1, w) : f0;
 }
 
 // window bytes of an emission block with kDirs directions (more directions span more table nodes)
 __host__ __device__ constexpr int emission_window_bytes(int dirs) {
   return dirs > 32 ? 64 * 1024 : dirs > 16 ? 48 * 1024 : kWindowBytes;
+}
+
+// x[0] + ... + x[n-1] in the order of an xor butterfly over n lanes read at lane 0: pairwise halves, each addition
+// rounded on its own (a butterfly's shuffles keep a product from fusing into the next addition; here __fadd_rn does)
+template <int n>
+__device__ __forceinline__ float tree_sum(const float* x) {
+  if constexpr (n == 1) {
+    return x[0];
+  } else {
+    return __fadd_rn(tree_sum<n / 2>(x), tree_sum<n / 2>(x + n / 2));
+  }
 }
 
 template <int kGP, int kMM, bool kFused, int kDirs>
@@ -626,7 +657,7 @@ __global__ void __launch_bounds__(kEmitPoints * kGP) emission_kernel(
         float w;
         table_position(tb, cosine, i0, w);
         const float offset = pg.f > 1 ? oy * offy + ox * offx + oz * offz : 0.f;  // one point per cell: its centre
-        const float src = fc_group<kGP, kMM, kWin ? 1 : 2>(tb, s_tab, win_lo, i0, w, g, rho, phi);
+        const float src = fc_group<kGP, kMM, kWin ? 1 : 2, true>(tb, s_tab, win_lo, i0, w, g, rho, phi);
         float smc = 0.f;
         if (kFused) {
 #pragma unroll
@@ -684,36 +715,38 @@ __global__ void __launch_bounds__(kEmitPoints * kGP) emission_kernel(
   if (win_lo >= 0) directions(std::true_type{});
   else directions(std::false_type{});
   __syncthreads();
-  if (tid < 2 * nd) {
-    const int dd = tid / 2, which = tid % 2;
-    float acc = 0.f;
-    for (int q = 0; q < kWarps; ++q) acc += s_sum[dd][q][which];
-    partial[((int64_t)(d0 + dd) * gridDim.x + blockIdx.x) * 2 + which] = acc;
+  for (int i = tid; i < 2 * nd; i += nthreads) {  // one or two groups have fewer threads than sums
+    const int dd = i / 2, which = i % 2;
+    float part[kWarps];
+#pragma unroll
+    for (int q = 0; q < kWarps; ++q) part[q] = s_sum[dd][q][which];
+    partial[((int64_t)(d0 + dd) * gridDim.x + blockIdx.x) * 2 + which] = tree_sum<kWarps>(part);  // the butterfly goes on
   }
 }
 
 // ---- attenuated emission, one thread per (point, direction) with all of its groups ---------------------------------
 // A block is 32 points (the lanes, consecutive points and, for one point per cell, consecutive cells) by kEmitWarps
-// warps; warp w takes the block's directions w, w + kEmitWarps, ... . The cosine, the table position, the traced path
-// lengths, the signal sum and the write happen once per (point, direction), where the group lanes of emission_kernel
-// repeat them G times; the multiple-collision source (and per-group optical depths) of a cell are G contiguous floats,
-// read as float4 and coalesced over the warp. Only the transfer entries of incoming groups at or above the outgoing
-// one enter the sum (the reference's first-collision table is downscatter only, uncollided_kernels.py:488-550).
-// Every group value, the group sums and the per-block partial sums are formed in emission_kernel's order (its
-// sequential incoming-group sums, its xor-butterfly group sums, its warp-then-block point sums), so the two kernels
-// give the same bits on a table without upscatter entries.
+// warps; a warp takes one direction at a time. The multiple-collision source (and per-group optical depths) of a cell
+// are G contiguous floats, read as float4 and coalesced over the warp.
+// A point's first-collision source depends on the direction through the scattering cosine alone, and the panel's directions
+// see few of the table's nodes: the block forms F[node][group], the sum over materials and incoming groups, once per
+// node and point (node_sums), and a direction only interpolates between two nodes. The directions run in the order of their
+// cosine with the block's middle direction, and F is a ring of nodes in shared memory that moves with them, so
+// that every node is formed once per block. A row of the table read for a whole warp costs four shared-memory or L1
+// wavefronts per float4; with both rows read per direction that was 192 wavefronts for 8 groups and two materials, the
+// kernel's bound, against 16 for the interpolation and 96 per node formed. 64^3 points, 8 groups,
+// 512 directions: 3.46 -> 1.80 ms (2.56 with the numbers of groups and materials checked at run time, hence kExact); 32^3,
+// one group: 213 -> 152 us.
+// Only the transfer entries of incoming groups at or above the outgoing one enter the sum (the reference's
+// first-collision table is downscatter only, uncollided_kernels.py:488-550). Every group value, the group sums and the
+// per-block partial sums are formed in emission_kernel's order (its sequential incoming-group sums, its butterflies
+// over groups and points), so the two kernels give the same bits on a table without upscatter entries.
 constexpr int kEmitWarps = 8;
+constexpr int kEmitDirs = 256;  // directions of a block
+constexpr int kEmitBins = 512;  // bins of the sort by cosine
 
-// x[0] + ... + x[n-1] in the order of an xor butterfly over n lanes read at lane 0: pairwise halves, each addition
-// rounded on its own (a butterfly's shuffles keep a product from fusing into the next addition; here __fadd_rn does)
-template <int n>
-__device__ __forceinline__ float tree_sum(const float* x) {
-  if constexpr (n == 1) {
-    return x[0];
-  } else {
-    return __fadd_rn(tree_sum<n / 2>(x), tree_sum<n / 2>(x + n / 2));
-  }
-}
+// nodes of the ring: a power of two, 64 KB of float[kGP][32] per node for up to 8 groups (3 blocks per SM), 128 KB for 16
+__host__ __device__ constexpr int ring_nodes(int gp) { return gp > 8 ? 64 : 512 / gp; }
 
 // sum_{gi <= g} row[gi] phi[gi], in incoming-group order; the row in shared or global memory, float4 reads when the
 // rows are 16-byte aligned (kVec)
@@ -762,62 +795,90 @@ __device__ __forceinline__ void load_groups(const float* __restrict__ p, int G, 
   }
 }
 
+// F of one node at this lane's point: sum_m rho_m sum_{g' <= g} T_m[node][g][g'] phi_g', materials without density left
+// out, into f
+// (rows [material][G][G] in shared memory, kStaged, or the table's in global memory)
+template <int kGP, int kMM, bool kVec, bool kExact, bool kStaged>
+__device__ __forceinline__ void node_sums(const Table& tb, const float* rows, int64_t material_stride,
+                                          const float* rho, const float* phi, float* f) {
+  const int G = kExact ? kGP : tb.G;
+#pragma unroll
+  for (int g = 0; g < kGP; ++g) f[g] = 0.f;
+#pragma unroll
+  for (int m = 0; m < kMM; ++m) {
+    if (!kExact && m >= tb.M) break;
+    const float* row = rows + m * material_stride;
+#pragma unroll
+    for (int g = 0; g < kGP; ++g) {
+      if (g >= G) break;
+      const float a = dot_lower<kGP, kVec, kStaged>(row + g * G, phi, g);
+      if (rho[m] != 0.f) f[g] = fmaf(rho[m], a, f[g]);
+    }
+  }
+}
+
+// kN values of a ring slot at this lane from group g on: float4s of consecutive groups [group / 4][lane], or floats
+// [group][lane] for 1 or 2 groups
+template <int kN>
+__device__ __forceinline__ void load_ring(const float* __restrict__ slot, int g, int lane, float* f) {
+  if constexpr (kN == 4) {
+    const float4 t = *reinterpret_cast<const float4*>(slot + (g * 32 + 4 * lane));
+    f[0] = t.x;
+    f[1] = t.y;
+    f[2] = t.z;
+    f[3] = t.w;
+  } else {
+#pragma unroll
+    for (int q = 0; q < kN; ++q) f[q] = slot[(g + q) * 32 + lane];
+  }
+}
+
 // kQ1: one point per cell (the point is the cell's centre: no in-cell offsets, no cell attenuation needed). A warp's
-// loads of its next direction's multiple-collision source and path lengths are issued before the table sums of the
-// current one, so their latency hides behind that arithmetic; 3 blocks of 256 threads per SM (80 registers, the
-// 64 KB table window).
-template <int kGP, int kMM, int kDirs, bool kVec, bool kQ1>
-__global__ void __launch_bounds__(32 * kEmitWarps, 3) emission_warps_kernel(
+// loads of its next direction's multiple-collision source and path lengths are issued before the interpolation of the
+// current one, so their latency hides behind that arithmetic; 3 blocks of 256 threads per SM (80 registers).
+// kExact: kGP groups and kMM materials, with traced lengths of kMM materials: the group and material tests of every
+// direction drop out (a third of the instructions).
+template <int kGP, int kMM, bool kVec, bool kQ1, bool kExact>
+__global__ void __launch_bounds__(32 * kEmitWarps, kGP > 8 ? 1 : 3) emission_warps_kernel(
     FCInputs in, Table tb, PointGrid pg, const float* __restrict__ omegas, int K,
     const float* __restrict__ tau /*[K, NC, G], or [K, NC, TM] path lengths with tau_mu*/,
-    const float* __restrict__ tau_mu /*[TM, G] or null*/, int TM, const float* __restrict__ mu /*[G, NC]*/,
+    const float* __restrict__ tau_mu /*[TM, G] or null*/, int traced_materials, const float* __restrict__ mu /*[G, NC]*/,
     const float* __restrict__ multiple /*[K, NC, G]*/, const float* __restrict__ heights,
     const float* __restrict__ signal_weight /*[K, G] or null*/, float dx, float dy, float dz,
     float* __restrict__ out, float* __restrict__ partial /*[K, nblocks, 2]*/) {
-  constexpr int kPW = 32 / kGP;  // points per warp of emission_kernel, whose partial-sum order is kept
   constexpr int nthreads = 32 * kEmitWarps;
+  constexpr int kRing = ring_nodes(kGP);
   extern __shared__ float4 s_dyn4[];
-  float* s_tab = reinterpret_cast<float*>(s_dyn4);
-  __shared__ float s_om[kDirs][3];
-  __shared__ float s_sw[kDirs][kGP];
-  __shared__ float s_tmu[kMM][kGP];
-  __shared__ int s_range[2][32];
-  __shared__ int s_window[2];
-  const int G = tb.G;
+  float* s_ring = reinterpret_cast<float*>(s_dyn4);   // [kRing][kGP][32]
+  __shared__ float s_om[kEmitDirs][3];
+  __shared__ __align__(16) float s_tmu[kMM][kGP];
+  __shared__ int s_first[kEmitBins + 1];              // directions before each bin
+  __shared__ short s_order[kEmitDirs], s_bin[kEmitDirs];
+  const int G = kExact ? kGP : tb.G, TM = kExact ? kMM : traced_materials;
+  const int M = kExact ? kMM : tb.M;
+  const bool traced = kExact || tau_mu != nullptr;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int d0 = blockIdx.y * kDirs;
-  const int nd = min(kDirs, K - d0);
-  for (int i = tid; i < kDirs * 3; i += nthreads) s_om[i / 3][i % 3] = i < nd * 3 ? omegas[3 * d0 + i] : 0.f;
-  if (signal_weight != nullptr)
-    for (int i = tid; i < kDirs * kGP; i += nthreads) {
-      const int dd = i / kGP, q = i % kGP;
-      s_sw[dd][q] = (dd < nd && q < G) ? signal_weight[(int64_t)(d0 + dd) * G + q] : 0.f;
-    }
+  const int d0 = blockIdx.y * kEmitDirs;
+  const int nd = min(kEmitDirs, K - d0);
+  for (int i = tid; i < nd * 3; i += nthreads) s_om[i / 3][i % 3] = omegas[3 * d0 + i];
   for (int i = tid; i < kMM * kGP; i += nthreads) {
     const int m = i / kGP, q = i % kGP;
-    s_tmu[m][q] = (tau_mu != nullptr && m < TM && q < G) ? tau_mu[m * G + q] : 0.f;
+    s_tmu[m][q] = (traced && m < TM && q < G) ? tau_mu[m * G + q] : 0.f;
   }
+  for (int i = tid; i <= kEmitBins; i += nthreads) s_first[i] = 0;
 
   const int64_t v = (int64_t)blockIdx.x * 32 + lane;
   const bool valid = v < in.V;
   const int64_t NC = (int64_t)pg.Rc * pg.Cc * pg.Sc;
-  float rho[kMM], phi[kGP], muc[kGP];
+  float muc[kGP];
   float ux = 0.f, uy = 0.f, uz = 0.f, h = 0.f, offx = 0.f, offy = 0.f, offz = 0.f;
   int64_t cell = 0;
 #pragma unroll
-  for (int q = 0; q < kGP; ++q) phi[q] = muc[q] = 0.f;
-#pragma unroll
-  for (int m = 0; m < kMM; ++m) rho[m] = 0.f;
+  for (int q = 0; q < kGP; ++q) muc[q] = 0.f;
   if (valid) {
     int i, j, k;
     point_rcs(v, pg, i, j, k);
     primary_direction(__ldg(in.ax_x + j), __ldg(in.ax_y + i), __ldg(in.ax_z + k), in.r0x, in.r0y, in.r0z, ux, uy, uz);
-#pragma unroll
-    for (int m = 0; m < kMM; ++m)
-      if (m < tb.M) rho[m] = __ldg(in.rho + (int64_t)m * in.V + v);
-#pragma unroll
-    for (int q = 0; q < kGP; ++q)
-      if (q < G) phi[q] = __ldg(in.phi + (int64_t)q * in.V + v);
     const int F = pg.f, ic = i / F, jc = j / F, kc = k / F;
     cell = ((int64_t)ic * pg.Cc + jc) * pg.Sc + kc;
     const float half = (F - 1) * 0.5f;
@@ -831,27 +892,90 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 3) emission_warps_kernel(
         if (q < G) muc[q] = __ldg(mu + (int64_t)q * NC + cell);
     }
   }
-  __syncthreads();  // s_om, s_sw and s_tmu are complete
-  stage_window(tb, valid, ux, uy, uz, s_om, nd, warp, kEmitWarps, warp, kEmitWarps, tid, nthreads, s_range, s_window,
-               s_tab, emission_window_bytes(kDirs));
-  const int win_lo = s_window[0];
-  const int RS = window_row_stride(G);
-
-  auto directions = [&](auto windowed) {
-    constexpr bool kWin = decltype(windowed)::value;
-    float smc_n[kGP], P_n[kMM];
-    auto fetch = [&](int dd) {
-      if (valid && dd < nd) {
-        const int64_t dc = (d0 + dd) * NC + cell;
-        load_groups<kGP, kVec>(multiple + dc * G, G, smc_n);
-        if (tau_mu != nullptr) {
+  // the middle of the block's primary directions, and the farthest of them in nodes of the table (every warp holds all
+  // 32 points): a direction's nodes at the block's points lie that far around its node at the middle
+  float c[3] = {ux, uy, uz}, margin = 0.f;
 #pragma unroll
-          for (int m = 0; m < kMM; ++m) P_n[m] = m < TM ? __ldg(tau + dc * TM + m) : 0.f;
+  for (int a = 0; a < 3; ++a) {
+    float lo = valid ? c[a] : INFINITY, hi = valid ? c[a] : -INFINITY;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, off));
+      hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, off));
+    }
+    const float mid = 0.5f * (lo + hi);
+    if (valid) margin = fmaf(c[a] - mid, c[a] - mid, margin);
+    c[a] = mid;
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) margin = fmaxf(margin, __shfl_xor_sync(0xffffffffu, margin, off));
+  // a unit direction's length and the cosines are rounded: one node more covers far more than that
+  const float nodes_away = 1.01f * sqrtf(margin) * (float)(tb.N - 1) / (tb.eta_hi - tb.eta_lo) + 1.f;
+  const int reach = nodes_away < 4096.f ? (int)nodes_away + 1 : 4096;
+  int shift = 0;                                      // nodes per bin, as a power of two
+  while (((tb.N - 1) >> shift) >= kEmitBins) ++shift;
+  // nodes [first of a bin - reach, last of the bin + reach + 1] have to fit the ring
+  const bool ring = 2 * reach + 1 + (1 << shift) <= kRing;
+  __syncthreads();  // s_om, s_tmu and the zeroed bins are complete
+  for (int i = tid; i < nd; i += nthreads) {
+    int node;
+    float w;
+    table_position(tb, c[0] * s_om[i][0] + c[1] * s_om[i][1] + c[2] * s_om[i][2], node, w);
+    s_bin[i] = (short)(node >> shift);
+    atomicAdd(&s_first[(node >> shift) + 1], 1);
+  }
+  __syncthreads();
+  if (warp == 0) {  // running sums over the bins, 16 a lane
+    constexpr int kPer = kEmitBins / 32;
+    int count = 0;
+    for (int q = 0; q < kPer; ++q) count += s_first[1 + lane * kPer + q];
+    int before = count;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int other = __shfl_up_sync(0xffffffffu, before, off);
+      if (lane >= off) before += other;
+    }
+    before -= count;
+    for (int q = 0; q < kPer; ++q) {
+      before += s_first[1 + lane * kPer + q];
+      s_first[1 + lane * kPer + q] = before;
+    }
+  }
+  __syncthreads();
+  // directions by bin; their order within one changes nothing, every direction's result is its own. A bin's first
+  // place moves up to the next bin's.
+  for (int i = tid; i < nd; i += nthreads) s_order[atomicAdd(&s_first[s_bin[i]], 1)] = (short)i;
+  __syncthreads();
+  // the point's densities and fluence, read where nodes are formed (registers short in the direction loop)
+  auto load_inputs = [&](float* rho, float* phi) {
+#pragma unroll
+    for (int m = 0; m < kMM; ++m) rho[m] = valid && m < M ? __ldg(in.rho + (int64_t)m * in.V + v) : 0.f;
+#pragma unroll
+    for (int q = 0; q < kGP; ++q) phi[q] = valid && q < G ? __ldg(in.phi + (int64_t)q * in.V + v) : 0.f;
+  };
+
+  const float* multiple_c = multiple + (d0 * NC + cell) * G;  // of the block's first direction
+  const float* tau_c = tau + (d0 * NC + cell) * (traced ? TM : G);
+  const int64_t multiple_step = NC * G, tau_step = NC * (traced ? TM : G);
+  float* out_v = out + (d0 * in.V + v) * (signal_weight != nullptr ? 1 : G);
+  const int64_t out_step = in.V * (signal_weight != nullptr ? 1 : G);
+  // directions s_order[from .. to) of this warp, their nodes in the ring, or the table's rows in global memory
+  auto directions = [&](auto ringed, int from, int to) {
+    constexpr bool kRinged = decltype(ringed)::value;
+    float smc_n[kGP], P_n[kMM];
+    auto fetch = [&](int at) {
+      if (valid && at < to) {
+        const int dd = s_order[at];
+        load_groups<kGP, kVec>(multiple_c + dd * multiple_step, G, smc_n);
+        if (traced) {
+#pragma unroll
+          for (int m = 0; m < kMM; ++m) P_n[m] = m < TM ? __ldg(tau_c + dd * tau_step + m) : 0.f;
         }
       }
     };
-    fetch(warp);
-    for (int dd = warp; dd < nd; dd += kEmitWarps) {
+    fetch(from + warp);
+    for (int at = from + warp; at < to; at += kEmitWarps) {
+      const int dd = s_order[at];
       const int64_t d = d0 + dd;
       float e[kGP];
 #pragma unroll
@@ -861,61 +985,70 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 3) emission_warps_kernel(
       for (int q = 0; q < kGP; ++q) smc[q] = smc_n[q];
 #pragma unroll
       for (int m = 0; m < kMM; ++m) P[m] = P_n[m];
-      fetch(dd + kEmitWarps);  // the next direction's loads in flight during this one's table sums
+      fetch(at + kEmitWarps);  // the next direction's loads in flight during this one's arithmetic
       if (valid) {
-        const int64_t dc = d * NC + cell;
-        float t[kGP];
-        if (tau_mu != nullptr) {  // sum_m mu[m, g] P_m, in material order
-#pragma unroll
-          for (int q = 0; q < kGP; ++q) t[q] = 0.f;
-#pragma unroll
-          for (int m = 0; m < kMM; ++m)
-            if (m < TM) {
-#pragma unroll
-              for (int q = 0; q < kGP; ++q) t[q] = fmaf(s_tmu[m][q], P[m], t[q]);
-            }
-        } else {
-          load_groups<kGP, kVec>(tau + dc * G, G, t);
-        }
         const float ox = s_om[dd][0], oy = s_om[dd][1], oz = s_om[dd][2];
         const float cosine = ux * ox + uy * oy + uz * oz;
         int i0;
         float w;
         table_position(tb, cosine, i0, w);
         const float offset = kQ1 ? 0.f : oy * offy + ox * offx + oz * offz;
-        float src[kGP];
-#pragma unroll
-        for (int q = 0; q < kGP; ++q) src[q] = 0.f;
-#pragma unroll
-        for (int m = 0; m < kMM; ++m) {
-          const float r = rho[m];
-          if (m >= tb.M || r == 0.f) continue;
-          const float* row0 = kWin ? s_tab + ((i0 - win_lo) * tb.M + m) * RS
-                                   : tb.t + ((int64_t)m * tb.N + i0) * G * G;
-          const float* row1 = row0 + (kWin ? tb.M * RS : G * G);
-#pragma unroll
-          for (int g = 0; g < kGP; ++g) {
-            if (g >= G) break;
-            const float a0 = dot_lower<kGP, kVec, kWin>(row0 + g * G, phi, g);
-            const float a1 = dot_lower<kGP, kVec, kWin>(row1 + g * G, phi, g);
-            src[g] = fmaf(r, a0 + (a1 - a0) * w, src[g]);
-          }
+        const float *slot0, *slot1;
+        float rho[kRinged ? 1 : kMM], phi[kRinged ? 1 : kGP], f_all[2][kRinged ? 1 : kGP];
+        if constexpr (kRinged) {
+          slot0 = s_ring + (i0 & (kRing - 1)) * kGP * 32;
+          slot1 = s_ring + ((i0 + 1) & (kRing - 1)) * kGP * 32;
+        } else {
+          load_inputs(rho, phi);
+          const float* row0 = tb.t + (int64_t)i0 * G * G;
+          node_sums<kGP, kMM, kVec, kExact, false>(tb, row0, (int64_t)tb.N * G * G, rho, phi, f_all[0]);
+          node_sums<kGP, kMM, kVec, kExact, false>(tb, row0 + G * G, (int64_t)tb.N * G * G, rho, phi, f_all[1]);
         }
+        constexpr int kN = kGP < 4 ? kGP : 4;
 #pragma unroll
-        for (int g = 0; g < kGP; ++g) {
-          if (g >= G) break;
-          const float depth = kQ1 ? fmaxf(t[g], 0.f) : fmaxf(t[g] - muc[g] * offset, 0.f);
-          e[g] = (src[g] + smc[g]) * __expf(-depth);  // the fast exponential: within a few ulp for these depths
+        for (int q = 0; q < kGP; q += kN) {
+          if (q >= G) break;
+          float t[kN], f0[kN], f1[kN];
+          if (traced) {  // sum_m mu[m, g] P_m, in material order
+#pragma unroll
+            for (int g = 0; g < kN; ++g) t[g] = 0.f;
+#pragma unroll
+            for (int m = 0; m < kMM; ++m) {  // materials past TM: zero lengths
+              if (kMM <= 2 || m < TM) {
+#pragma unroll
+                for (int g = 0; g < kN; ++g) t[g] = fmaf(s_tmu[m][q + g], P[m], t[g]);
+              }
+            }
+          } else {
+            load_groups<kN, kVec>(tau_c + dd * tau_step + q, G - q, t);
+          }
+          if constexpr (kRinged) {
+            load_ring<kN>(slot0, q, lane, f0);
+            load_ring<kN>(slot1, q, lane, f1);
+          } else {
+#pragma unroll
+            for (int g = 0; g < kN; ++g) {
+              f0[g] = f_all[0][q + g];
+              f1[g] = f_all[1][q + g];
+            }
+          }
+#pragma unroll
+          for (int g = 0; g < kN; ++g) {  // groups past G: zero sources and depths
+            const float depth = kQ1 ? fmaxf(t[g], 0.f) : fmaxf(t[g] - muc[q + g] * offset, 0.f);
+            // the fast exponential: within a few ulp for these depths
+            e[q + g] = (interpolate_nodes(f0[g], f1[g], w) + smc[q + g]) * __expf(-depth);
+          }
         }
       }
       const float tot = tree_sum<kGP>(e);
       if (signal_weight != nullptr) {
         float sg[kGP];
+        load_groups<kGP, kVec>(signal_weight + d * G, G, sg);
 #pragma unroll
-        for (int q = 0; q < kGP; ++q) sg[q] = __fmul_rn(s_sw[dd][q], e[q]);
-        if (valid) out[d * in.V + v] = tree_sum<kGP>(sg);
+        for (int q = 0; q < kGP; ++q) sg[q] = __fmul_rn(sg[q], e[q]);
+        if (valid) out_v[dd * out_step] = tree_sum<kGP>(sg);
       } else if (valid) {
-        float* o = out + (d * in.V + v) * G;
+        float* o = out_v + dd * out_step;
         if (kVec) {
 #pragma unroll
           for (int q = 0; q < kGP / 4; ++q)
@@ -926,27 +1059,76 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 3) emission_warps_kernel(
             if (q < G) o[q] = e[q];
         }
       }
-      // emission_kernel's order: a butterfly over its kPW points per warp, then its warps in sequence
+      // a butterfly over the block's points
       float a = tot, b = __fmul_rn(tot, h);
 #pragma unroll
-      for (int off = 1; off < kPW; off <<= 1) {
+      for (int off = 1; off < 32; off <<= 1) {
         a += __shfl_xor_sync(0xffffffffu, a, off);
         b += __shfl_xor_sync(0xffffffffu, b, off);
       }
-      float sa = 0.f, sb = 0.f;
-#pragma unroll
-      for (int q = 0; q < kGP; ++q) {
-        sa += __shfl_sync(0xffffffffu, a, q * kPW);
-        sb += __shfl_sync(0xffffffffu, b, q * kPW);
-      }
       if (lane == 0) {
-        partial[(d * gridDim.x + blockIdx.x) * 2] = sa;
-        partial[(d * gridDim.x + blockIdx.x) * 2 + 1] = sb;
+        partial[(d * gridDim.x + blockIdx.x) * 2] = a;
+        partial[(d * gridDim.x + blockIdx.x) * 2 + 1] = b;
       }
     }
   };
-  if (win_lo >= 0) directions(std::true_type{});
-  else directions(std::false_type{});
+  if (!ring) {  // points too far apart for the ring (uniform over the block)
+    directions(std::false_type{}, 0, nd);
+    return;
+  }
+  // this warp's rows of one node, [material][G][G], and where its lanes find them in the table
+  constexpr int kLoads = (kMM * kGP * kGP + 31) / 32;
+  float* s_rows = s_ring + kRing * kGP * 32 + warp * kLoads * 32;
+  int64_t row_at[kLoads];
+#pragma unroll
+  for (int q = 0; q < kLoads; ++q) {
+    const int e = q * 32 + lane, m = e / (G * G);
+    row_at[q] = m < M ? (int64_t)m * tb.N * G * G + (e - m * G * G) : -1;
+  }
+  int built = 0;  // nodes below this are in the ring or behind it
+  for (int from = 0; from < nd;) {
+    const int lo = (s_bin[s_order[from]] << shift) - reach;
+    // the bins whose nodes all lie below lo + kRing: node + reach + 1 <= lo + kRing - 1 for the last node of the bin
+    const int bins = min((lo + kRing - 1 - reach) >> shift, kEmitBins);
+    const int to = s_first[bins - 1];
+    const int hi = min(tb.N - 1, (s_bin[s_order[to - 1]] << shift) + (1 << shift) + reach);
+    if (max(lo, built) <= hi) {
+      float rho[kMM], phi[kGP];
+      load_inputs(rho, phi);
+      int node = max(max(lo, 0), built) + warp;
+      // the warp's rows of its next node are loaded while it sums the current one's from its shared memory
+      float next[kLoads];
+      auto load_rows = [&](int n) {
+#pragma unroll
+        for (int q = 0; q < kLoads; ++q) next[q] = row_at[q] >= 0 && n <= hi ? __ldg(tb.t + (int64_t)n * G * G + row_at[q]) : 0.f;
+      };
+      load_rows(node);
+      for (; node <= hi; node += kEmitWarps) {
+        float f[kGP];
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < kLoads; ++q)
+          if (row_at[q] >= 0) s_rows[q * 32 + lane] = next[q];
+        __syncwarp();
+        load_rows(node + kEmitWarps);
+        node_sums<kGP, kMM, kVec, kExact, true>(tb, s_rows, G * G, rho, phi, f);
+        float* slot = s_ring + (node & (kRing - 1)) * kGP * 32;
+        if constexpr (kGP >= 4) {
+#pragma unroll
+          for (int q = 0; q < kGP; q += 4)
+            *reinterpret_cast<float4*>(slot + q * 32 + 4 * lane) = make_float4(f[q], f[q + 1], f[q + 2], f[q + 3]);
+        } else {
+#pragma unroll
+          for (int q = 0; q < kGP; ++q) slot[q * 32 + lane] = f[q];
+        }
+      }
+    }
+    built = hi + 1;
+    __syncthreads();
+    directions(std::true_type{}, from, to);
+    __syncthreads();  // the ring moves on
+    from = to;
+  }
 }
 
 // ---- sampling correction over the sweep directions, with the source values kept -----------------------------------
@@ -1095,15 +1277,20 @@ __global__ void __launch_bounds__(kEmitPoints * kGP) fc_correction_kernel(
 // factors formed as fc_correction_kernel forms them. The sums differ from fc_correction_kernel's at rounding level
 // (another order of the same terms).
 // 3 blocks of 256 threads per SM (80 registers): at 2 (128 registers) the table gathers' latency went unhidden
+// Directions of a batch, and the bytes of its window: a batch of the sorted directions has to fit its window, or every
+// row is gathered from global memory. 120 directions over the sphere take 401 nodes, 24 of them 80, and the points of
+// a block spread a node over up to 28 more: 120 nodes of two materials and 8 groups are 64 KB. (32 directions in 48
+// KB, 88 nodes, never fitted: 1.77 ms at 64^3 points, 8 groups and 120 directions, now 0.75.)
 constexpr int kFcWarps = 8;
-constexpr int kFcDirBatch = 32;
+__host__ __device__ constexpr int fc_batch(int gp) { return gp > 8 ? 16 : 24; }
+__host__ __device__ constexpr int fc_window_bytes(int gp) { return gp > 8 ? 176 * 1024 : 64 * 1024; }
 
-template <int kGP, int kMM, bool kVec>
-__global__ void __launch_bounds__(32 * kFcWarps, 3) fc_correction_warps_kernel(
+template <int kGP, int kMM, bool kVec, bool kExact>  // kExact: kGP groups and kMM materials
+__global__ void __launch_bounds__(32 * kFcWarps, kGP > 8 ? 1 : 3) fc_correction_warps_kernel(
     FCInputs in, Table tb, PointGrid pg, const float* __restrict__ omegas, const float* __restrict__ weights, int K,
     const float* __restrict__ moments /*[M, 2, G, G]*/, float* __restrict__ sums /*[5, G, V] or null*/,
     float* __restrict__ scale, float* __restrict__ beta, float* __restrict__ cache /*[K, G, V] or null*/) {
-  constexpr int nthreads = 32 * kFcWarps;
+  constexpr int nthreads = 32 * kFcWarps, kFcDirBatch = fc_batch(kGP);
   extern __shared__ float4 s_dyn4[];
   float* s_tab = reinterpret_cast<float*>(s_dyn4);
   __shared__ float s_key[kMaxSorted];
@@ -1115,8 +1302,8 @@ __global__ void __launch_bounds__(32 * kFcWarps, 3) fc_correction_warps_kernel(
   __shared__ int s_window[2];
   __shared__ float s_u0[3];
   // after the direction loop the window's shared memory holds the warps' partial sums [kFcWarps][3][kGP][32]
-  static_assert(kFcWarps * 3 * kGP * 32 * 4 <= emission_window_bytes(kFcDirBatch), "partial sums exceed the window");
-  const int G = tb.G;
+  static_assert(kFcWarps * 3 * kGP * 32 * 4 <= fc_window_bytes(kGP), "partial sums exceed the window");
+  const int G = kExact ? kGP : tb.G, M = kExact ? kMM : tb.M;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t v = (int64_t)blockIdx.x * 32 + lane;
   const bool valid = v < in.V;
@@ -1132,7 +1319,7 @@ __global__ void __launch_bounds__(32 * kFcWarps, 3) fc_correction_warps_kernel(
     primary_direction(__ldg(in.ax_x + j), __ldg(in.ax_y + i), __ldg(in.ax_z + k), in.r0x, in.r0y, in.r0z, ux, uy, uz);
 #pragma unroll
     for (int m = 0; m < kMM; ++m)
-      if (m < tb.M) rho[m] = __ldg(in.rho + (int64_t)m * in.V + v);
+      if (m < M) rho[m] = __ldg(in.rho + (int64_t)m * in.V + v);
 #pragma unroll
     for (int q = 0; q < kGP; ++q)
       if (q < G) phi[q] = __ldg(in.phi + (int64_t)q * in.V + v);
@@ -1163,7 +1350,7 @@ __global__ void __launch_bounds__(32 * kFcWarps, 3) fc_correction_warps_kernel(
   float I0[kGP], I1[kGP], I2[kGP];
 #pragma unroll
   for (int q = 0; q < kGP; ++q) I0[q] = I1[q] = I2[q] = 0.f;
-  const int RS = window_row_stride(G);
+  const int NS = window_node_stride(M, G);
   for (int b0 = 0; b0 < K; b0 += kFcDirBatch) {
     const int nb = min(kFcDirBatch, K - b0);
     if (tid < nb) {
@@ -1175,10 +1362,12 @@ __global__ void __launch_bounds__(32 * kFcWarps, 3) fc_correction_warps_kernel(
       s_w[tid] = __ldg(weights + d);
     }
     __syncthreads();
-    stage_window(tb, valid, ux, uy, uz, s_om, nb, warp, kFcWarps, warp, kFcWarps, tid, nthreads, s_range, s_window,
-                 s_tab, emission_window_bytes(kFcDirBatch));
+    stage_window<kExact ? kGP : 0>(tb, valid, ux, uy, uz, s_om, nb, warp, kFcWarps, warp, kFcWarps, tid, nthreads,
+                                   s_range, s_window, s_tab, fc_window_bytes(kGP));
     const int win_lo = s_window[0];
-    if (valid) {
+    // one body per place of the rows: a pointer to either is a generic one, whose loads are no shared-memory loads
+    auto batch = [&](auto windowed) {
+      constexpr bool kWin = decltype(windowed)::value;
       for (int i = warp; i < nb; i += kFcWarps) {
         const float cosine = ux * s_om[i][0] + uy * s_om[i][1] + uz * s_om[i][2];
         int i0;
@@ -1187,24 +1376,17 @@ __global__ void __launch_bounds__(32 * kFcWarps, 3) fc_correction_warps_kernel(
         float S[kGP];
 #pragma unroll
         for (int q = 0; q < kGP; ++q) S[q] = 0.f;
-        const bool win = win_lo >= 0;
 #pragma unroll
         for (int m = 0; m < kMM; ++m) {
           const float r = rho[m];
-          if (m >= tb.M || r == 0.f) continue;
-          const float* row0 = win ? s_tab + ((i0 - win_lo) * tb.M + m) * RS : tb.t + ((int64_t)m * tb.N + i0) * G * G;
-          const float* row1 = row0 + (win ? tb.M * RS : G * G);
+          if (m >= M || r == 0.f) continue;
+          const float* row0 = kWin ? s_tab + (i0 - win_lo) * NS + m * G * G : tb.t + ((int64_t)m * tb.N + i0) * G * G;
+          const float* row1 = row0 + (kWin ? NS : G * G);
 #pragma unroll
           for (int g = 0; g < kGP; ++g) {
             if (g >= G) break;
-            float a0, a1;
-            if (win) {
-              a0 = dot_lower<kGP, kVec, true>(row0 + g * G, phi, g);
-              a1 = dot_lower<kGP, kVec, true>(row1 + g * G, phi, g);
-            } else {
-              a0 = dot_lower<kGP, kVec, false>(row0 + g * G, phi, g);
-              a1 = dot_lower<kGP, kVec, false>(row1 + g * G, phi, g);
-            }
+            const float a0 = dot_lower<kGP, kVec, kWin>(row0 + g * G, phi, g);
+            const float a1 = dot_lower<kGP, kVec, kWin>(row1 + g * G, phi, g);
             S[g] = fmaf(r, a0 + (a1 - a0) * w, S[g]);
           }
         }
@@ -1220,6 +1402,10 @@ __global__ void __launch_bounds__(32 * kFcWarps, 3) fc_correction_warps_kernel(
           if (cache != nullptr) cache[(d * G + g) * in.V + v] = S[g];
         }
       }
+    };
+    if (valid) {
+      if (win_lo >= 0) batch(std::true_type{});
+      else batch(std::false_type{});
     }
     __syncthreads();  // the batch's directions and window are replaced next
   }
@@ -1243,7 +1429,7 @@ __global__ void __launch_bounds__(32 * kFcWarps, 3) fc_correction_warps_kernel(
     }
     // exact l = 0, 1 moments of the source (downscatter rows of the moment table)
     float E0 = 0.f, E1 = 0.f;
-    for (int m = 0; m < tb.M && m < kMM; ++m) {
+    for (int m = 0; m < M && m < kMM; ++m) {
       const float* r0 = moments + (((int64_t)m * 2 + 0) * G + g) * G;
       const float* r1 = moments + (((int64_t)m * 2 + 1) * G + g) * G;
       float a0 = 0.f, a1 = 0.f;
@@ -1603,18 +1789,31 @@ int launch_fc_correction_m(dim3 grid, int G, cudaStream_t s, const FCInputs& in,
   return CITRUS_OK;
 }
 
+template <int kGP, int kMM, bool kVec, bool kExact>
+int launch_fc_correction_warps_e(dim3 grid, cudaStream_t s, const FCInputs& in, const Table& tb, const PointGrid& pg,
+                               const float* omegas, const float* weights, int K, const float* moments, float* sums,
+                               float* scale, float* beta, float* cache) {
+  constexpr int bytes = fc_window_bytes(kGP);
+  cudaError_t e = cudaFuncSetAttribute(fc_correction_warps_kernel<kGP, kMM, kVec, kExact>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e != cudaSuccess) return set_error(CITRUS_ECUDA, "first-collision window: %s", cudaGetErrorString(e));
+  fc_correction_warps_kernel<kGP, kMM, kVec, kExact><<<grid, 32 * kFcWarps, bytes, s>>>(in, tb, pg, omegas, weights, K,
+                                                                                moments, sums, scale, beta, cache);
+  note_launches();
+  return CITRUS_OK;
+}
+
 template <int kGP, int kMM, bool kVec>
 int launch_fc_correction_warps(dim3 grid, cudaStream_t s, const FCInputs& in, const Table& tb, const PointGrid& pg,
                                const float* omegas, const float* weights, int K, const float* moments, float* sums,
                                float* scale, float* beta, float* cache) {
-  constexpr int bytes = emission_window_bytes(kFcDirBatch);
-  cudaError_t e = cudaFuncSetAttribute(fc_correction_warps_kernel<kGP, kMM, kVec>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e != cudaSuccess) return set_error(CITRUS_ECUDA, "first-collision window: %s", cudaGetErrorString(e));
-  fc_correction_warps_kernel<kGP, kMM, kVec><<<grid, 32 * kFcWarps, bytes, s>>>(in, tb, pg, omegas, weights, K,
-                                                                                moments, sums, scale, beta, cache);
-  note_launches();
-  return CITRUS_OK;
+  if constexpr (kMM == 2 && (kVec || kGP < 4)) {
+    if (tb.G == kGP && tb.M == kMM)
+      return launch_fc_correction_warps_e<kGP, kMM, kVec, true>(grid, s, in, tb, pg, omegas, weights, K, moments, sums,
+                                                                scale, beta, cache);
+  }
+  return launch_fc_correction_warps_e<kGP, kMM, kVec, false>(grid, s, in, tb, pg, omegas, weights, K, moments, sums,
+                                                             scale, beta, cache);
 }
 
 // CITRUS_FC_KERNEL=groups selects the group-lane correction kernel (fc_correction_kernel); read at every call
@@ -1840,34 +2039,21 @@ int launch_emission(dim3 grid, int G, cudaStream_t s, const FCInputs& in, const 
                                                harmonics, moments, NS, heights, signal_weight, deltas, out, partial);
 }
 
-template <int kGP, int kMM, int kDirs, bool kVec, bool kQ1>
+template <int kGP, int kMM, bool kVec, bool kQ1, bool kExact>
 int launch_emission_warps_q(dim3 grid, cudaStream_t s, const FCInputs& in, const Table& tb, const PointGrid& pg,
                             const float* omegas, int K, const float* tau, const float* tau_mu, int TM,
                             const float* mu, const float* multiple, const float* heights, const float* signal_weight,
                             const double* deltas, float* out, float* partial) {
-  constexpr int bytes = emission_window_bytes(kDirs);
-  cudaError_t e = cudaFuncSetAttribute(emission_warps_kernel<kGP, kMM, kDirs, kVec, kQ1>,
+  constexpr int bytes = (ring_nodes(kGP) * kGP + kEmitWarps * ((kMM * kGP * kGP + 31) / 32)) * 32 * 4;
+  cudaError_t e = cudaFuncSetAttribute(emission_warps_kernel<kGP, kMM, kVec, kQ1, kExact>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e != cudaSuccess) return set_error(CITRUS_ECUDA, "emission window: %s", cudaGetErrorString(e));
-  grid.y = (unsigned)cdiv(K, kDirs);
-  emission_warps_kernel<kGP, kMM, kDirs, kVec, kQ1><<<grid, 32 * kEmitWarps, bytes, s>>>(
+  if (e != cudaSuccess) return set_error(CITRUS_ECUDA, "emission ring: %s", cudaGetErrorString(e));
+  grid.y = (unsigned)cdiv(K, kEmitDirs);
+  emission_warps_kernel<kGP, kMM, kVec, kQ1, kExact><<<grid, 32 * kEmitWarps, bytes, s>>>(
       in, tb, pg, omegas, K, tau, tau_mu, TM, mu, multiple, heights, signal_weight, (float)deltas[0],
       (float)deltas[1], (float)deltas[2], out, partial);
   note_launches();
   return CITRUS_OK;
-}
-
-template <int kGP, int kMM, int kDirs, bool kVec>
-int launch_emission_warps_d(dim3 grid, cudaStream_t s, const FCInputs& in, const Table& tb, const PointGrid& pg,
-                            const float* omegas, int K, const float* tau, const float* tau_mu, int TM,
-                            const float* mu, const float* multiple, const float* heights, const float* signal_weight,
-                            const double* deltas, float* out, float* partial) {
-  if (pg.f == 1)
-    return launch_emission_warps_q<kGP, kMM, kDirs, kVec, true>(grid, s, in, tb, pg, omegas, K, tau, tau_mu, TM, mu,
-                                                                multiple, heights, signal_weight, deltas, out,
-                                                                partial);
-  return launch_emission_warps_q<kGP, kMM, kDirs, kVec, false>(grid, s, in, tb, pg, omegas, K, tau, tau_mu, TM, mu,
-                                                               multiple, heights, signal_weight, deltas, out, partial);
 }
 
 template <int kGP, int kMM, bool kVec>
@@ -1875,11 +2061,15 @@ int launch_emission_warps_v(dim3 grid, cudaStream_t s, const FCInputs& in, const
                             const float* omegas, int K, const float* tau, const float* tau_mu, int TM,
                             const float* mu, const float* multiple, const float* heights, const float* signal_weight,
                             const double* deltas, float* out, float* partial) {
-  if (K >= 64)
-    return launch_emission_warps_d<kGP, kMM, 64, kVec>(grid, s, in, tb, pg, omegas, K, tau, tau_mu, TM, mu, multiple,
-                                                       heights, signal_weight, deltas, out, partial);
-  return launch_emission_warps_d<kGP, kMM, 32, kVec>(grid, s, in, tb, pg, omegas, K, tau, tau_mu, TM, mu, multiple,
-                                                     heights, signal_weight, deltas, out, partial);
+#define CITRUS_EWQ(Q1, EXACT)                                                                                         \
+  launch_emission_warps_q<kGP, kMM, kVec, Q1, EXACT>(grid, s, in, tb, pg, omegas, K, tau, tau_mu, TM, mu, multiple,   \
+                                                     heights, signal_weight, deltas, out, partial)
+  if constexpr (kMM == 2 && (kVec || kGP < 4)) {
+    if (tb.G == kGP && tb.M == kMM && tau_mu != nullptr && TM == kMM)
+      return pg.f == 1 ? CITRUS_EWQ(true, true) : CITRUS_EWQ(false, true);
+  }
+  return pg.f == 1 ? CITRUS_EWQ(true, false) : CITRUS_EWQ(false, false);
+#undef CITRUS_EWQ
 }
 
 // the (point, direction) kernel for G <= 16 with the multiple-collision source read (not fused); float4 group rows
@@ -1891,7 +2081,7 @@ int launch_emission_warps(dim3 grid, cudaStream_t s, const FCInputs& in, const T
                           const double* deltas, float* out, float* partial) {
   const auto aligned = [](const void* p) { return ((uintptr_t)p % 16) == 0; };
   const bool vec = tb.G % 4 == 0 && aligned(tb.t) && aligned(multiple) && (tau_mu != nullptr || aligned(tau)) &&
-                   (signal_weight != nullptr || aligned(out));
+                   (signal_weight != nullptr ? aligned(signal_weight) : aligned(out));
   constexpr bool kCanVec = kGP >= 4;  // G < 4 has no float4 rows
 #define CITRUS_EW(MM, VEC)                                                                                         \
   launch_emission_warps_v<kGP, MM, VEC>(grid, s, in, tb, pg, omegas, K, tau, tau_mu, TM, mu, multiple, heights,    \

@@ -36,11 +36,12 @@ from .uncollided import (FirstCollisionSamplingCorrection, first_collision_means
                          present_materials, uncollided_fluence)
 
 SWEEP_CHUNK_BUDGET_BYTES = 8 * 2 ** 30
-IMAGE_CHUNK_BUDGET_BYTES = 4 * 2 ** 30
+IMAGE_CHUNK_BUDGET_BYTES = 8 * 2 ** 30
 # Directions per image chunk at most. A chunk is 17 launches and about 0.5 ms of host work, and its buffers are past L2
 # from a few directions on, so the budget is the limit that matters: with chunks of 64 the image of a 32^3 grid with
-# one group waited for the host (whole view step 5.9 ms; one chunk of 512 directions: 3.0 ms), and an image at 64^3 x 8
-# groups, whose budget is 112 directions, takes as long either way.
+# one group waited for the host (whole view step 5.9 ms; one chunk of 512 directions: 3.0 ms). The emission takes up to
+# 256 directions per block and forms a point's sums at the table nodes once for them, so 64^3 x 8 groups gets two equal
+# chunks of 256 (4 GiB would make four of 128).
 IMAGE_CHUNK_MAX_DIRECTIONS = 512
 
 
@@ -197,13 +198,15 @@ class ScatterSolver:
         return q
 
     def image_direction_chunk(self, fields: MaterialFields) -> int:
-        """Directions per image chunk: as many as fit the budget, between ``direction_chunk`` and 512."""
+        """Directions per image chunk: as many as fit the budget, in equal chunks of ``direction_chunk`` to 512."""
         G = self.num_groups
         Rd, Cd = self.geometry.image_shape
-        per_direction = 4 * G * (2 * fields.grid_quadrature.num_voxels + 2 * fields.grid_coarse.num_voxels
-                                 + 3 * Rd * Cd)
-        return int(max(self.config.direction_chunk,
-                       min(IMAGE_CHUNK_MAX_DIRECTIONS, IMAGE_CHUNK_BUDGET_BYTES // max(1, per_direction))))
+        # the emission at the points, optical depths and multiple-collision source of the cells, three panel images
+        per_direction = 4 * G * (fields.grid_quadrature.num_voxels + 2 * fields.grid_coarse.num_voxels + 3 * Rd * Cd)
+        most = min(IMAGE_CHUNK_MAX_DIRECTIONS, IMAGE_CHUNK_BUDGET_BYTES // max(1, per_direction))
+        directions = self.config.cone_num_polar * self.config.cone_num_azimuthal
+        chunks = -(-directions // max(1, int(most)))
+        return int(max(self.config.direction_chunk, -(-directions // chunks)))
 
     def sweep_direction_chunk(self, fields: MaterialFields) -> int:
         """Directions per octant of a sweep chunk: as many as fit the store budget, in equal chunks."""
