@@ -555,7 +555,8 @@ def step_config(args, views: int, batch: int) -> dict:
 
 
 def sweep_form_name(solver, w, rho_dev) -> str:
-    """The accumulator sweep's form the autotuner chose for this grid (plane wavefront or tiled schedule)."""
+    """The accumulator sweep's form the autotuner chose for this grid (pencil schedule, plane wavefront or tiled
+    schedule)."""
     from citrus_gb300.batched import sweep_launch_config
     fields = solver.material_fields(rho_dev, w.grid)
     _, form, dc = sweep_launch_config(solver, fields, 60, 0)
@@ -563,6 +564,9 @@ def sweep_form_name(solver, w, rho_dev) -> str:
     if form.tile > 0:
         return (f"tiled: {form.tile}^3-cell tiles, {form.dirs_per_block} directions per task, thread form "
                 f"{form.thread_form}{chunks}")
+    if form.tile < 0:
+        return (f"pencils: tiles of {-form.tile}^2, {form.dirs_per_block} directions per task, {form.thread_form} views "
+                f"per thread{chunks}")
     return f"plane wavefront, thread form {form.thread_form}{chunks}"
 
 
@@ -631,12 +635,18 @@ def tiled_sweep_bytes(args) -> int:
     return 32 * views * 8 * Dc * N * G
 
 
-SWEEP_ENTRY_POINTS = ("citrus_sweep_tiled", "citrus_sweep_persistent_config", "citrus_sweep_persistent")
+def pencil_sweep_bytes(args) -> int:
+    """citrus_sweep_pencils: the same 32 B per update as the plane wavefront."""
+    cells, G, Dc, views = int(args[3]) * int(args[4]) * int(args[5]), int(args[6]), int(args[7]), int(args[8])
+    return 32 * views * 8 * Dc * cells * G
+
+
+SWEEP_ENTRY_POINTS = ("citrus_sweep_pencils", "citrus_sweep_tiled", "citrus_sweep_persistent_config", "citrus_sweep_persistent")
 STEP_TIMED = {"citrus_attenuated_emission_moments": emission_bytes, "citrus_attenuated_emission": product_emission_bytes,
               "citrus_downstream_cumulative": downstream_bytes, "citrus_downstream_cumulative_tables": downstream_bytes,
               "citrus_downstream_cumulative_facing": lambda args: downstream_bytes(args, 5),
               "citrus_sweep_persistent": sweep_bytes, "citrus_sweep_persistent_config": sweep_bytes,
-              "citrus_sweep_tiled": tiled_sweep_bytes,
+              "citrus_sweep_tiled": tiled_sweep_bytes, "citrus_sweep_pencils": pencil_sweep_bytes,
               "citrus_oblique_project": None, "citrus_oblique_project_scratch": None, "citrus_box_blur": None,
               "citrus_small_k_gemm": None,
               "citrus_small_k_gemm_config": None, "citrus_small_k_gemm_bf16x3": None, "citrus_first_collision_moments": None,

@@ -163,31 +163,50 @@ VIEW_CANDIDATES = (1, 2, 4, 8)
 # registers capped for 5 (form 1), 6 (form 3) or 4 (form 5) blocks of 256 threads per SM, or the loads of 2 (form 2)
 # or 4 (form 4) views issued before their solves
 UNROLL_CANDIDATES = (1, 3, 5, 2, 4)
-# the tiled schedule (one grid barrier per tile diagonal) in the forms that came closest to the plane wavefront on the
-# 64^3 x 120-direction grid: (thread form, tile edge, directions per task); directions per task are capped by the chunk
-TILED_CANDIDATES = ((2, 4, 5), (2, 8, 3), (1, 4, 5), (1, 8, 3))
+# lanes of a pencil (directions of a task x groups) of the pencil schedule: few for the most tasks, or a warp's share
+PENCIL_LANES = (1, 2, 8)
 
 
-def sweep_config(ctx, mu_cells, num_groups: int, views: int, default=(4, 2, 0, 1), dc: int = 0) -> tuple:
+def pencil_forms(num_groups: int, dc: int) -> list:
+    """The candidates of the pencil schedule as [views per thread, -tile, directions per task]: as many directions as
+    the lanes hold, in equal tasks; empty where a block cannot hold the groups."""
+    from .kernels import PENCIL_THREADS, pencil_tile
+
+    tile = pencil_tile(num_groups)
+    forms = []
+    for lanes in PENCIL_LANES:
+        d = -(-dc // -(-dc // max(1, min(dc, lanes // num_groups))))
+        for u in (1, 2):
+            if tile and tile * tile * d * num_groups <= PENCIL_THREADS and [u, -tile, d] not in forms:
+                forms.append([u, -tile, d])
+    return forms
+
+
+def sweep_config(ctx, mu_cells, num_groups: int, views: int, default=None, dc: int = 0) -> tuple:
     """(views per sweep launch, ``kernels.SweepForm``) for ``views`` views on this grid and chunks of ``dc``
     directions per octant (0: all): the per-view time of the sweep on a store of ones of 1, 2, 4 or 8 views (those
-    whose store takes at most a quarter of the free device memory) in each form (the plane wavefront in each
-    lanes-per-thread form, the tiled schedule per tile edge, thread form and directions per task); the first (fewest
-    views) within 3 % of the fastest."""
+    whose store takes at most a quarter of the free device memory) in each form: the pencil schedule per views per
+    thread and directions per task, or, for more groups than its blocks hold, the plane wavefront per thread form. The
+    pencil schedule was 1.3 to 11 times as fast as the plane wavefront (which the tiled schedule did not beat) on grids
+    of 8^3 to 64^3, 8 x 8 x 200 and 200 x 8 x 8 cells with 1 to 100 groups, so those are not timed beside it. The first
+    (fewest views) within 3 % of the fastest."""
     from . import kernels
 
     N, Q = ctx.num_cells, 4 * num_groups
     D8 = ctx.directions_per_octant if dc <= 0 else min(int(dc), ctx.directions_per_octant)
     c_chunk = ctx.c if D8 == ctx.directions_per_octant else ctx.c[:, :D8].contiguous()
     device = ctx.device
-    # "form" names the forms' meaning: entries timed before the tiled schedule existed are not reused
+    if default is None:
+        tile = kernels.pencil_tile(num_groups)
+        default = (2, 2, -tile, 1) if tile else (4, 2, 0, 1)
+    # "form" names the forms' meaning: entries timed before the pencil schedule existed are not reused
     key = Autotuner.key("sweep", device, N=N, D8=D8, G=num_groups, shape="x".join(map(str, ctx.shape)),
-                        form="views-per-thread+tiles")
+                        form="views-per-thread+tiles+pencils")
     entry = tuner().table.get(key)
     if entry is None and not torch.cuda.is_current_stream_capturing():
         free, _ = torch.cuda.mem_get_info(device)
         per_view = 8 * D8 * N * Q * 4
-        forms = [[u, 0, 1] for u in UNROLL_CANDIDATES] + [[u, t, min(d, D8)] for u, t, d in TILED_CANDIDATES]
+        forms = pencil_forms(num_groups, D8) or [[u, 0, 1] for u in UNROLL_CANDIDATES]
         candidates = [[b, *f] for b in VIEW_CANDIDATES if b * per_view <= free // 4 for f in forms]
         candidates = candidates or [[1, *f] for f in forms]
         stores = {}

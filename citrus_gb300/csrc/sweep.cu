@@ -35,7 +35,56 @@ struct LaneCoef {
   float qsx, qsy, qsz;  // s_a c_a / d_a
   float rden;           // 1 / (sum_a c_a + m + 3 sum_a c_a q_a)
   uint32_t at, ax, ay, az;
+  bool plain;  // the direction's c_a are 0 or within [kPlainMin, kPlainMax]
 };
+
+// c_a and m between these (or 0) keep d_a, its reciprocal, c_a / d_a and the remainder of quotient() normal numbers
+constexpr float kPlainMin = 1e-18f, kPlainMax = 1e18f;
+
+__device__ __forceinline__ bool plain_c(float c) { return c == 0.f || (c >= kPlainMin && c <= kPlainMax); }
+
+// a / b from the correctly rounded reciprocal r of b, which the lane needs as well: the product a r corrected once by its
+// exact remainder (Markstein, Computation of elementary functions on the IBM RISC System/6000 processor, 1990), the
+// rounding of an IEEE division for normal numbers (no other result in 6e8 random pairs). Three such quotients are nine
+// instructions; three divisions were a quarter of a lane's.
+__device__ __forceinline__ float quotient(float a, float b, float r) {
+  const float q = __fmul_rn(a, r);
+  return __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
+}
+
+// The part of a lane that its octant and direction give. Every operation here and below is rounded on its own (no
+// multiply-add contraction), so every kernel computes the same bits.
+__device__ __forceinline__ void direction_coef(int o, float cx, float cy, float cz, LaneCoef& k) {
+  const float sx = (o & 4) ? -1.f : 1.f, sy = (o & 2) ? -1.f : 1.f, sz = (o & 1) ? -1.f : 1.f;
+  k.sx = sx, k.sy = sy, k.sz = sz, k.cx = cx, k.cy = cy, k.cz = cz;
+  k.plain = plain_c(cx) && plain_c(cy) && plain_c(cz);
+  k.k3x = __fmul_rn(__fmul_rn(3.f, sx), cx);
+  k.k3y = __fmul_rn(__fmul_rn(3.f, sy), cy);
+  k.k3z = __fmul_rn(__fmul_rn(3.f, sz), cz);
+}
+
+// The part that the cell's attenuation m gives for that direction
+__device__ __forceinline__ void cell_coef(float m, LaneCoef& k) {
+  const float cx = k.cx, cy = k.cy, cz = k.cz;
+  const float csum = __fadd_rn(__fadd_rn(cx, cy), cz);
+  const float dx = __fadd_rn(__fadd_rn(__fmul_rn(3.f, cx), __fsub_rn(csum, cx)), m);
+  const float dy = __fadd_rn(__fadd_rn(__fmul_rn(3.f, cy), __fsub_rn(csum, cy)), m);
+  const float dz = __fadd_rn(__fadd_rn(__fmul_rn(3.f, cz), __fsub_rn(csum, cz)), m);
+  k.rdx = __frcp_rn(dx);
+  k.rdy = __frcp_rn(dy);
+  k.rdz = __frcp_rn(dz);
+  float qx, qy, qz;
+  if (k.plain && m >= 0.f && m <= kPlainMax) {
+    qx = quotient(cx, dx, k.rdx), qy = quotient(cy, dy, k.rdy), qz = quotient(cz, dz, k.rdz);
+  } else {
+    qx = __fdiv_rn(cx, dx), qy = __fdiv_rn(cy, dy), qz = __fdiv_rn(cz, dz);
+  }
+  const float qsum = __fadd_rn(__fadd_rn(__fmul_rn(cx, qx), __fmul_rn(cy, qy)), __fmul_rn(cz, qz));
+  k.rden = __frcp_rn(__fadd_rn(__fadd_rn(csum, m), __fmul_rn(3.f, qsum)));
+  k.qsx = __fmul_rn(k.sx, qx);
+  k.qsy = __fmul_rn(k.sy, qy);
+  k.qsz = __fmul_rn(k.sz, qz);
+}
 
 // The lane of entry e, direction d and group g; every float4 position of a view is below 2^31 (checked on the host)
 template <int kG>
@@ -56,25 +105,8 @@ __device__ __forceinline__ void lane_coef_edg(uint32_t e, uint32_t d, uint32_t g
   k.ax = ux < N ? (base + ux) * G + g : kVacuum;
   k.ay = uy < N ? (base + uy) * G + g : kVacuum;
   k.az = uz < N ? (base + uz) * G + g : kVacuum;
-  // every operation is rounded on its own (no multiply-add contraction), so every kernel computes the same bits
-  const float sx = (o & 4) ? -1.f : 1.f, sy = (o & 2) ? -1.f : 1.f, sz = (o & 1) ? -1.f : 1.f;
-  k.sx = sx, k.sy = sy, k.sz = sz, k.cx = cx, k.cy = cy, k.cz = cz;
-  k.k3x = __fmul_rn(__fmul_rn(3.f, sx), cx);
-  k.k3y = __fmul_rn(__fmul_rn(3.f, sy), cy);
-  k.k3z = __fmul_rn(__fmul_rn(3.f, sz), cz);
-  const float csum = __fadd_rn(__fadd_rn(cx, cy), cz);
-  const float dx = __fadd_rn(__fadd_rn(__fmul_rn(3.f, cx), __fsub_rn(csum, cx)), m);
-  const float dy = __fadd_rn(__fadd_rn(__fmul_rn(3.f, cy), __fsub_rn(csum, cy)), m);
-  const float dz = __fadd_rn(__fadd_rn(__fmul_rn(3.f, cz), __fsub_rn(csum, cz)), m);
-  const float qx = __fdiv_rn(cx, dx), qy = __fdiv_rn(cy, dy), qz = __fdiv_rn(cz, dz);
-  const float qsum = __fadd_rn(__fadd_rn(__fmul_rn(cx, qx), __fmul_rn(cy, qy)), __fmul_rn(cz, qz));
-  k.rden = __frcp_rn(__fadd_rn(__fadd_rn(csum, m), __fmul_rn(3.f, qsum)));
-  k.rdx = __frcp_rn(dx);
-  k.rdy = __frcp_rn(dy);
-  k.rdz = __frcp_rn(dz);
-  k.qsx = __fmul_rn(sx, qx);
-  k.qsy = __fmul_rn(sy, qy);
-  k.qsz = __fmul_rn(sz, qz);
+  direction_coef(o, cx, cy, cz, k);
+  cell_coef(m, k);
 }
 
 // lane = (e - start) Dc G + d G + g of a plane starting at entry start
@@ -103,9 +135,8 @@ __device__ __forceinline__ void gather_view(const LaneCoef& k, const float4* vie
   in.Z = k.az != kVacuum ? load4<kCoherent>(view + k.az) : zero;
 }
 
-// The closed-form cell solve of the equations of linear_discontinuous_cell.py:14-87 in one view, stored over the
-// source.
-__device__ __forceinline__ void solve_view(const LaneCoef& k, const LaneIn& in, float4* view) {
+// The closed-form cell solve of the equations of linear_discontinuous_cell.py:14-87 in one view
+__device__ __forceinline__ float4 solve_cell(const LaneCoef& k, const LaneIn& in) {
   const float4 s = in.s, X = in.X, Y = in.Y, Z = in.Z;
   // face-averaged inflow psibar_a = psi_0[N_a] + s_a psi_a[N_a]
   const float pbx = __fadd_rn(X.x, __fmul_rn(k.sx, X.y));
@@ -126,7 +157,12 @@ __device__ __forceinline__ void solve_view(const LaneCoef& k, const LaneIn& in, 
   out.y = __fmul_rn(__fadd_rn(rx, __fmul_rn(k.k3x, p0)), k.rdx);
   out.z = __fmul_rn(__fadd_rn(ry, __fmul_rn(k.k3y, p0)), k.rdy);
   out.w = __fmul_rn(__fadd_rn(rz, __fmul_rn(k.k3z, p0)), k.rdz);
-  view[k.at] = out;
+  return out;
+}
+
+// ... stored over the source
+__device__ __forceinline__ void solve_view(const LaneCoef& k, const LaneIn& in, float4* view) {
+  view[k.at] = solve_cell(k, in);
 }
 
 // One plane, one lane (view v, entry, direction, group) per thread: the reference's launch plan.
@@ -233,6 +269,200 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) tiled_kernel(
   }
 }
 
+// ---- pencils ------------------------------------------------------------------------------------------------------
+// The wavefront without grid barriers. In each octant's sweep frame the (row, column) plane is cut into tiles of T x T
+// pencils; a task is one tile of one (octant, block of dpb directions, block of kVB views), and a block walks its pencils
+// along the slices, a thread per (pencil, direction, group), pencil (i, j) of the tile i + j steps behind the first. A
+// thread keeps its own last cell (the z inflow) in registers and hands its outputs to the pencils (i + 1, j) and
+// (i, j + 1) of the tile through shared memory one step later; only the tile's faces read what another block wrote.
+// Shared memory is a ring of kPencilSlots steps of (T + 1) x (T + 1) pencils, the first row and column being the inflow
+// through the faces. The sources and face inflows of the next kPencilAhead steps are on their way to it (cp.async, each
+// thread into places that it alone reads), and a step's output takes its source's place, so a step costs one block
+// barrier, every inflow is read at the same offset, and no thread waits for memory.
+// Tasks come from a counter, by views and then by tile diagonal over all octants and directions; a task waits, with a
+// limit, for the flags of its two upstream tiles, which earlier tasks set. A block holds one task at a time and the
+// earliest unfinished task never waits, so every wait ends, however many blocks are resident.
+// Against the plane wavefront it reads a cell's source once and its own outputs not at all (three neighbours per cell
+// came from L2), loads no entry tables, and needs no grid barrier: 64^3 cells, 8 groups, 120 directions 3.81 -> 2.31 ms,
+// in pairs of views 2.92 -> 1.77 ms per view; 32^3, one group 0.57 -> 0.21 ms. Its issue slots are 70 % busy (about 200
+// instructions per cell, half of them the coefficients that two views share); HBM's floor at 64^3 is 1.19 ms.
+constexpr int kPencilSlots = 5;
+constexpr int kPencilAhead = kPencilSlots - 2;  // a slot is refilled a barrier after the neighbours read its outputs
+constexpr int kPencilThreads = 512;
+constexpr int kPencilFlag = 4;  // the first flag among the sync words: 0 the task counter, 2 the error word
+
+struct Pencils {
+  uint32_t R, C, S, G, Dc, dpb, T;  // grid, groups, directions of an octant and of a task, tile edge
+  uint32_t tiles_r, tiles_c, dir_blocks, sequences, total;  // tiles along rows and columns; (octant, directions) pairs
+};
+
+// 16 bytes to shared memory if `issue`: those at src, or zeros if bytes is 0 (predicated: a branch per copy costs more)
+__device__ __forceinline__ void cp_async16_if(bool issue, uint32_t dst, const void* src, int bytes = 16) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %0, 0;\n\t"
+      "@p cp.async.cg.shared.global [%1], [%2], 16, %3;\n\t}" ::"r"((int)issue), "r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+
+__device__ __forceinline__ float4 load_shared4(uint32_t at) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at));
+  return v;
+}
+
+__device__ __forceinline__ void store_shared4(uint32_t at, float4 v) {
+  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(at), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+
+// The next task of the block as (sequence, tile row, tile column, flag index), its inflow complete; false when there is
+// none or a wait ran out. One thread.
+__device__ __forceinline__ bool next_pencil_task(const Pencils& p, unsigned* sync, uint64_t timeout_ns, uint32_t out[4]) {
+  const uint32_t id = atomicAdd(&sync[0], 1u);
+  if (id >= p.total) return false;
+  const uint32_t tiles = p.tiles_r * p.tiles_c, per_view = p.sequences * tiles;
+  const uint32_t v = id / per_view, rem = id - v * per_view;
+  const uint32_t rank = rem / p.sequences;
+  const uint32_t q = v * p.sequences + (rem - rank * p.sequences);
+  // the tile of that rank by diagonals: they grow to n = min(tiles_r, tiles_c) tiles, stay so and shrink again
+  const uint32_t n = min(p.tiles_r, p.tiles_c), wide = max(p.tiles_r, p.tiles_c) - n + 1;
+  const uint32_t grow = (uint32_t)((uint64_t)n * (n - 1) / 2);
+  uint32_t D, place;
+  if (rank >= grow && rank - grow < n * wide) {
+    D = n - 1 + (rank - grow) / n;
+    place = (rank - grow) % n;
+  } else {
+    const bool shrinking = rank >= grow;
+    const uint32_t r = shrinking ? tiles - 1 - rank : rank;
+    uint32_t e = (uint32_t)((sqrt(8.0 * r + 1.0) - 1.0) * 0.5);  // the last e with e (e + 1) / 2 <= r
+    while ((uint64_t)e * (e + 1) / 2 > r) --e;
+    while ((uint64_t)(e + 1) * (e + 2) / 2 <= r) ++e;
+    place = r - (uint32_t)((uint64_t)e * (e + 1) / 2);
+    if (shrinking) place = e - place;
+    D = shrinking ? p.tiles_r + p.tiles_c - 2 - e : e;
+  }
+  const uint32_t I = (D >= p.tiles_c ? D - p.tiles_c + 1 : 0) + place, J = D - I;
+  const uint32_t flag = q * tiles + I * p.tiles_c + J;
+  const unsigned* flags = sync + kPencilFlag;
+  const uint64_t t0 = global_timer_ns();
+  for (int a = 0; a < 2; ++a) {
+    if ((a == 0 ? I : J) == 0) continue;
+    const unsigned* f = flags + flag - (a == 0 ? p.tiles_c : 1);
+    while (ld_acquire_u32(f) == 0u) {
+      if (ld_acquire_u32(&sync[2]) != 0u) return false;
+      if (global_timer_ns() - t0 > timeout_ns) {
+        atomicExch(&sync[2], 1u);
+        return false;
+      }
+      __nanosleep(64);
+    }
+  }
+  __threadfence();
+  out[0] = q, out[1] = I, out[2] = J, out[3] = flag;
+  return true;
+}
+
+template <int kG, int kVB>
+__global__ void __launch_bounds__(kPencilThreads, 2) pencil_kernel(float4* __restrict__ store,
+                                                                   const float* __restrict__ mu,
+                                                                   const float* __restrict__ c, Pencils p, int views,
+                                                                   int64_t view_stride, unsigned* sync,
+                                                                   uint64_t timeout_ns, int skip) {
+  extern __shared__ float4 s_pencil[];  // [kPencilSlots][kVB][T + 1][T + 1][L]
+  __shared__ uint32_t s_task[4];
+  __shared__ int s_go;
+  const uint32_t G = kG > 0 ? kG : p.G, L = p.dpb * G, T = p.T;
+  const uint32_t tid = threadIdx.x, l = tid % L, col = tid / L, tj = col % T, ti = col / T, dd = l / G, g = l - dd * G;
+  const uint32_t to_x = 16 * L, to_y = (T + 1) * to_x, view_bytes = (T + 1) * to_y, slot_bytes = kVB * view_bytes;
+  const uint32_t mine = (uint32_t)__cvta_generic_to_shared(s_pencil) + (ti + 1) * to_y + (tj + 1) * to_x + 16 * l;
+  const int lag = (int)(ti + tj);
+  for (;;) {
+    if (tid == 0) s_go = next_pencil_task(p, sync, timeout_ns, s_task);
+    __syncthreads();
+    if (!s_go) return;
+    const uint32_t q = s_task[0], I = s_task[1], J = s_task[2];
+    const uint32_t vb = q / p.sequences, od = q - vb * p.sequences, o = od / p.dir_blocks;
+    const uint32_t d = (od - o * p.dir_blocks) * p.dpb + dd;
+    const uint32_t ip = I * T + ti, jp = J * T + tj;  // the pencil in the octant's sweep frame
+    const bool valid = ip < p.R && jp < p.C && d < p.Dc;
+    const int v0 = (int)vb * kVB, nv = min(kVB, views - v0);
+    const int steps = (int)(p.S + min(T, p.R - I * T) + min(T, p.C - J * T)) - 2;
+    const uint32_t S = valid ? p.S : 0u;  // cells of this thread's pencil
+    const int dk = (o & 1) ? -(int)G : (int)G;  // float4 (and attenuation) stride to the next cell of the pencil
+    // ... and to the x and y upstream cells (0 at a vacuum face, which reads zeros)
+    const int up_x = jp == 0 ? 0 : (o & 4) ? (int)(p.S * G) : -(int)(p.S * G);
+    const int up_y = ip == 0 ? 0 : (o & 2) ? (int)(p.C * p.S * G) : -(int)(p.C * p.S * G);
+    const bool at_face = __any_sync(__activemask(), tj == 0 || ti == 0);  // the warp's pencils at the tile's faces
+    const int bytes_x = jp > 0 ? 16 : 0, bytes_y = ip > 0 ? 16 : 0;
+    LaneCoef k;
+    direction_coef((int)o, 0.f, 0.f, 0.f, k);
+    k.at = 0;
+    int64_t at = 0;  // the cell that is loaded, as a float4 position; kPencilAhead cells on from the one that is solved
+    const float* m_next_at = mu;
+    if (valid) {
+      const uint32_t i = (o & 2) ? p.R - 1 - ip : ip, j = (o & 4) ? p.C - 1 - jp : jp, k0 = (o & 1) ? p.S - 1 : 0;
+      const uint32_t n = (i * p.C + j) * p.S + k0, odir = o * p.Dc + d;
+      direction_coef((int)o, __ldg(c + 3 * odir), __ldg(c + 3 * odir + 1), __ldg(c + 3 * odir + 2), k);
+      at = v0 * view_stride + ((int64_t)odir * (p.R * p.C * p.S) + n) * G + g - (int64_t)lag * dk;
+      m_next_at = mu + ((int64_t)n * G + g) - (int64_t)(lag + kPencilAhead - 1) * dk;
+    }
+    float4 Z[kVB];
+#pragma unroll
+    for (int v = 0; v < kVB; ++v) Z[v] = make_float4(0.f, 0.f, 0.f, 0.f);
+    float m_next = 0.f;
+    // Step t runs in slot (t + kPencilAhead) % kPencilSlots; the inflow of a step is in the slot before it
+    for (int t0 = -kPencilAhead; t0 < steps; t0 += kPencilSlots) {
+#pragma unroll
+      for (int q5 = 0; q5 < kPencilSlots; ++q5) {
+        constexpr int kA = kPencilAhead, kP = kPencilSlots;
+        const int t = t0 + q5, here = t - lag;
+        if (t >= steps) break;
+        const bool load = (uint32_t)(here + kA) < S;
+#pragma unroll
+        for (int v = 0; v < kVB; ++v) {
+          const bool some = load && (kVB == 1 || v < nv);
+          const float4* src = store + at + v * view_stride;
+          const uint32_t to = mine + v * view_bytes, before = to + (q5 + kA - 1) % kP * slot_bytes;
+          cp_async16_if(some, to + (q5 + kA) % kP * slot_bytes, src);
+          if (at_face) {
+            cp_async16_if(some && tj == 0, before - to_x, src + up_x, bytes_x);
+            cp_async16_if(some && ti == 0, before - to_y, src + up_y, bytes_y);
+          }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const float m = m_next;
+        if ((uint32_t)(here + 1) < S) m_next = __ldg(m_next_at);
+        m_next_at += dk;
+        if (t >= 0) {
+          asm volatile("cp.async.wait_group %0;" ::"n"(kA) : "memory");
+          if ((uint32_t)here < S) {
+            cell_coef(m, k);
+            float4* out = store + at - kA * dk;
+#pragma unroll
+            for (int v = 0; v < kVB; ++v) {
+              if (kVB > 1 && v >= nv) break;
+              const uint32_t slot = mine + v * view_bytes + q5 * slot_bytes;
+              const uint32_t last = mine + v * view_bytes + (q5 + kP - 1) % kP * slot_bytes;
+              LaneIn in;
+              in.s = load_shared4(slot);
+              in.X = load_shared4(last - to_x);
+              in.Y = load_shared4(last - to_y);
+              in.Z = Z[v];
+              Z[v] = solve_cell(k, in);
+              out[v * view_stride] = Z[v];
+              store_shared4(slot, Z[v]);
+            }
+          }
+          __syncthreads();
+        }
+        at += dk;
+      }
+    }
+    if (tid == 0) {  // the last step's barrier put the block's stores before this
+      __threadfence();
+      if ((int)blockIdx.x != skip) st_release_u32(sync + kPencilFlag + s_task[3], 1u);
+    }
+  }
+}
+
 template <int kG>
 int launch_planes(float* store, const float* mu, const float* c, const int* octant, const int* cell,
                   const int* upstream, const int64_t* offsets, int64_t num_planes, int64_t N, int G, int64_t Dc,
@@ -320,6 +550,37 @@ int launch_tiled(float* store, const float* mu, const float* c, const int* octan
                                     num_diagonals, num_sub, N, G, Dc, dpb, views, sync, max_blocks, timeout_ns, skip,
                                     stream);
   return set_error(CITRUS_EINVAL, "citrus_sweep_tiled: thread form %d (1 or 2)", form);
+}
+
+template <int kG, int kVB>
+int launch_pencils(float* store, const float* mu, const float* c, Pencils p, int64_t views, unsigned* sync,
+                   int64_t sync_words, int64_t max_blocks, uint64_t timeout_ns, int skip, cudaStream_t stream) {
+  const int64_t view_blocks = cdiv(views, kVB), tiles = (int64_t)p.tiles_r * p.tiles_c;
+  const int64_t total = view_blocks * p.sequences * tiles;
+  CITRUS_REQUIRE(total < (1ll << 30), "citrus_sweep_pencils: too many tasks (%lld)", (long long)total);
+  CITRUS_REQUIRE(sync_words >= kPencilFlag + total, "citrus_sweep_pencils: %lld sync words for %lld tasks",
+                 (long long)sync_words, (long long)total);
+  p.total = (uint32_t)total;
+  const int lanes = (int)(p.dpb * p.G), threads = (int)(p.T * p.T) * lanes;
+  const int smem = kPencilSlots * kVB * (int)((p.T + 1) * (p.T + 1)) * lanes * (int)sizeof(float4);
+  CITRUS_REQUIRE(smem <= 226 * 1024, "citrus_sweep_pencils: %d bytes of shared memory for tiles of %d^2 pencils of %d "
+                 "lanes", smem, (int)p.T, lanes);
+  cudaError_t e = cudaFuncSetAttribute(pencil_kernel<kG, kVB>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  int per_sm = 0;
+  if (e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pencil_kernel<kG, kVB>, threads, smem);
+  if (e != cudaSuccess || per_sm < 1) return set_error(CITRUS_ECUDA, "citrus_sweep_pencils: occupancy query failed");
+  int64_t blocks = (int64_t)per_sm * num_sms();
+  if (max_blocks > 0 && max_blocks < blocks) blocks = max_blocks;
+  if (blocks > total) blocks = total;
+  if (skip >= blocks) skip = (int)blocks - 1;
+  e = cudaMemsetAsync(sync, 0, (kPencilFlag + total) * sizeof(unsigned), stream);
+  if (e != cudaSuccess) return set_error(CITRUS_ECUDA, "citrus_sweep_pencils: %s", cudaGetErrorString(e));
+  const int64_t view_stride = 8 * (int64_t)p.Dc * p.R * p.C * p.S * p.G;  // float4 per view
+  pencil_kernel<kG, kVB><<<(unsigned)blocks, threads, smem, stream>>>(reinterpret_cast<float4*>(store), mu, c, p,
+                                                                      (int)views, view_stride, sync, timeout_ns, skip);
+  note_launches();
+  return launch_status("citrus_sweep_pencils");
 }
 
 constexpr int kDefaultUnroll = 1;
@@ -476,6 +737,54 @@ extern "C" int citrus_sweep_tiled(float* store, const float* mu_cells, const flo
 #undef CITRUS_TILED
   if (status) return status;
   return launch_status("citrus_sweep_tiled");
+}
+
+extern "C" int citrus_sweep_pencils(float* store, const float* mu_cells, const float* c, int64_t rows, int64_t cols,
+                                    int64_t slices, int64_t num_groups, int64_t dc, int64_t views, int64_t tile,
+                                    int64_t dirs_per_block, int64_t views_per_thread, uint32_t* sync,
+                                    int64_t sync_words, int64_t max_blocks, int64_t timeout_ns, int64_t skip_block,
+                                    void* stream) {
+  CITRUS_REQUIRE(store && mu_cells && c && sync, "citrus_sweep_pencils: null pointer argument");
+  CITRUS_REQUIRE(rows >= 1 && cols >= 1 && slices >= 1 && num_groups >= 1 && dc >= 1 && views >= 1,
+                 "citrus_sweep_pencils: sizes must be positive");
+  const int64_t cells_max = (1ll << 31) / 8;
+  CITRUS_REQUIRE(rows < cells_max && cols < cells_max && slices < cells_max && rows * cols < cells_max &&
+                     rows * cols * slices < cells_max,
+                 "citrus_sweep_pencils: the grid's cells exceed the 32-bit positions");
+  const int64_t cells = rows * cols * slices;
+  CITRUS_REQUIRE(views < (1ll << 31), "citrus_sweep_pencils: too many views (%lld)", (long long)views);
+  CITRUS_REQUIRE(num_groups <= 4096 && dc < (1ll << 28) && 8 * cells * num_groups < (1ll << 31) &&
+                     8 * cells * num_groups * dc < (1ll << 31),
+                 "citrus_sweep_pencils: one view's store exceeds the 32-bit lane positions; sweep fewer directions per "
+                 "chunk");
+  CITRUS_REQUIRE(((uintptr_t)store % 16) == 0, "citrus_sweep_pencils: store must be 16-byte aligned");
+  CITRUS_REQUIRE(dirs_per_block >= 1 && dirs_per_block <= dc, "citrus_sweep_pencils: directions per task %lld outside "
+                 "[1, %lld]", (long long)dirs_per_block, (long long)dc);
+  CITRUS_REQUIRE(tile >= 1 && tile <= 16 && tile * tile * dirs_per_block * num_groups <= kPencilThreads,
+                 "citrus_sweep_pencils: a tile of %lld^2 pencils of %lld lanes exceeds %d threads", (long long)tile,
+                 (long long)(dirs_per_block * num_groups), kPencilThreads);
+  CITRUS_REQUIRE(views_per_thread == 1 || views_per_thread == 2,
+                 "citrus_sweep_pencils: views per thread %lld (1 or 2)", (long long)views_per_thread);
+  CITRUS_REQUIRE(timeout_ns > 0, "citrus_sweep_pencils: timeout_ns must be positive");
+  Pencils p;
+  p.R = (uint32_t)rows, p.C = (uint32_t)cols, p.S = (uint32_t)slices, p.G = (uint32_t)num_groups, p.Dc = (uint32_t)dc;
+  p.dpb = (uint32_t)dirs_per_block, p.T = (uint32_t)tile;
+  p.tiles_r = (uint32_t)cdiv(rows, tile), p.tiles_c = (uint32_t)cdiv(cols, tile);
+  p.dir_blocks = (uint32_t)cdiv(dc, dirs_per_block), p.sequences = 8 * p.dir_blocks, p.total = 0;
+  const uint64_t t = (uint64_t)timeout_ns;
+  const int skip = skip_block < 0 ? -1 : (int)skip_block;
+  unsigned* sy = reinterpret_cast<unsigned*>(sync);
+  cudaStream_t s = as_stream(stream);
+#define CITRUS_PENCILS(KG)                                                                                        \
+  (views_per_thread == 2                                                                                          \
+       ? launch_pencils<KG, 2>(store, mu_cells, c, p, views, sy, sync_words, max_blocks, t, skip, s)              \
+       : launch_pencils<KG, 1>(store, mu_cells, c, p, views, sy, sync_words, max_blocks, t, skip, s))
+  switch (num_groups) {
+    case 1: return CITRUS_PENCILS(1);
+    case 8: return CITRUS_PENCILS(8);
+    default: return CITRUS_PENCILS(0);
+  }
+#undef CITRUS_PENCILS
 }
 
 // ---- allocation-free persistent sweep ----------------------------------------------------------------------------

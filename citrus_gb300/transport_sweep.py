@@ -295,7 +295,9 @@ def sweep(ctx: SweepContext, mu_t: Tensor, source_function, direction_chunk: Opt
             ``[Dsel, R, C, S, G, 4]`` into ``out`` (``cell_major = True``), or returning ``[Dsel, G, 4, R, C, S]``.
         direction_chunk: directions per octant swept together (None: all D8).
         return_psi: also return the angular fluence ``[M, G, 4, R, C, S]`` (tests).
-        method: plane driver of ``kernels.sweep_planes``.
+        method: "persistent" (one launch per chunk: the pencil schedule of ``kernels.sweep_pencils`` for up to 128
+            groups, which was faster at every size measured, else the plane wavefront) or "planes" (one launch per
+            plane).
         check: read back the barrier words and raise on a timeout (one host synchronization per sweep).
         precision: arithmetic of the moment accumulation ``Yw^T psi`` (``kernels.small_k_gemm``).
 
@@ -323,7 +325,10 @@ def sweep(ctx: SweepContext, mu_t: Tensor, source_function, direction_chunk: Opt
         c = ctx.c[:, d0:d1].contiguous()
         store = torch.empty(8, chunk, N, Q, device=device, dtype=torch.float32)
         _fill_source(ctx, source_function, d0, d1, G, store)
-        sync = kernels.sweep_planes(ctx.flat_index, store, mu_cells, c, method=method)
+        if method == "persistent" and kernels.pencil_tile(G):
+            sync = kernels.sweep_pencils(ctx.shape, store, mu_cells, c, tile=kernels.pencil_tile(G))
+        else:
+            sync = kernels.sweep_planes(ctx.flat_index, store, mu_cells, c, method=method)
         if sync is not None:
             syncs.append(sync)
         weights = ctx.Y_weighted.index_select(0, index).t().contiguous()  # [N_sh, 8 dc]

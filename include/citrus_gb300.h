@@ -90,6 +90,19 @@ int citrus_sweep_tiled(float* store, const float* mu_cells, const float* c, cons
                        int64_t views, int64_t dirs_per_block, uint32_t* sync, int64_t max_blocks, int64_t thread_form,
                        int64_t timeout_ns, int64_t skip_block, void* stream);
 
+/* The accumulator sweep of one chunk in the pencil schedule (no counterpart in the reference): the same store as
+ * citrus_sweep_planes, bit for bit, in one launch without grid barriers. In each octant's sweep frame the (row, column)
+ * plane is cut into tiles of tile x tile pencils (1..16); a block walks the pencils of one tile along the slices for
+ * dirs_per_block directions (1..dc) and views_per_thread views (1 or 2) once the tile's two upstream tiles are done.
+ * tile^2 dirs_per_block num_groups is at most 512 threads. sync: sync_words device words, 4 and one per task (tiles x
+ * 8 ceil(dc / dirs_per_block) x ceil(views / views_per_thread)), cleared by the call itself; sync[2] != 0 after the
+ * launch: a wait ran past timeout_ns and the store is invalid. max_blocks caps the grid (0: as many as fit); skip_block
+ * >= 0 is a test hook (that block never reports its tasks as done). */
+int citrus_sweep_pencils(float* store, const float* mu_cells, const float* c, int64_t rows, int64_t cols,
+                         int64_t slices, int64_t num_groups, int64_t dc, int64_t views, int64_t tile,
+                         int64_t dirs_per_block, int64_t views_per_thread, uint32_t* sync, int64_t sync_words,
+                         int64_t max_blocks, int64_t timeout_ns, int64_t skip_block, void* stream);
+
 /* The persistent sweep without any allocation: no counterpart in the reference, which always runs the sweep through
  * torch's allocator. The barrier words and the plane offsets live in a static device array of this library (33 KB
  * per device, at most 8191 planes, i.e. R + C + S - 2 <= 8191; more planes return CITRUS_EINVAL). The call clears
