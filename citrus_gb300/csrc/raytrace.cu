@@ -682,6 +682,65 @@ __global__ void crossing_table_kernel(Box b, const float* __restrict__ omegas, i
   }
 }
 
+// The crossing table of direction k in shared memory: the steps (segment length, flat index step x scale) as int2 [E] (E
+// rounded up to even, so that two steps are one 16-byte load), then t [E] and first [E]. Ends with a block barrier.
+struct LatticeTable {
+  const int2* step;
+  const float* t;
+  const int32_t* first;
+};
+
+__device__ __forceinline__ LatticeTable stage_lattice(int4* s_tab4, const int32_t* __restrict__ table, int k, int E,
+                                                      int scale) {
+  const int E2 = (E + 1) & ~1;
+  int2* s_step = reinterpret_cast<int2*>(s_tab4);
+  int32_t* s_words = reinterpret_cast<int32_t*>(s_tab4) + 2 * E2;
+  const int32_t* src = table + (int64_t)k * 3 * E;
+  for (int i = threadIdx.x; i < E; i += kThreads) {
+    // the length of the segment that ends at crossing i: t[i] - t[i - 1] (t[-1] = 0), as the walk forms it
+    const float tj = __int_as_float(src[i]), tp = i > 0 ? __int_as_float(src[i - 1]) : 0.f;
+    s_step[i] = make_int2(__float_as_int(tj - tp), src[E + i] * scale);
+    s_words[i] = src[i];
+    s_words[E + i] = src[2 * E + i];
+  }
+  if (threadIdx.x == 0 && E2 > E) s_step[E] = make_int2(0, 0);
+  __syncthreads();
+  return {s_step, reinterpret_cast<const float*>(s_words), s_words + E};
+}
+
+// The segments of the ray from voxel (ix, iy, iz) along w: the first J end at crossings 0 .. J - 1 and are whole
+// (t_j <= t_end); when the ray ends before its exit crossing there is one more, cut at t_end.
+__device__ __forceinline__ void lattice_ray(const Box& b, const Panel& panel, const LatticeTable& tab, const float w[3],
+                                            float diagonal, int ix, int iy, int iz, int& J, bool& cut, float& t_end) {
+  const int E = b.n[0] + b.n[1] + b.n[2];
+  const float r[3] = {voxel_centre(b, 0, ix), voxel_centre(b, 1, iy), voxel_centre(b, 2, iz)};
+  t_end = fminf(fmaxf(panel_distance(panel, r, w), 0.f), diagonal);
+  // the crossing that leaves the box: along axis a after the voxels left between i_a and the face ahead
+  const int idx[3] = {ix, iy, iz};
+  const int off[3] = {0, b.n[0], b.n[0] + b.n[1]};
+  int exit_j = E;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    if (w[a] == 0.f) continue;
+    const int left = w[a] > 0.f ? b.n[a] - 1 - idx[a] : idx[a];
+    exit_j = min(exit_j, tab.first[off[a] + left]);
+  }
+  if (exit_j < E) t_end = fminf(t_end, tab.t[exit_j]);
+  // the first j with t_j > t_end, by bisection of the sorted table
+  J = min(exit_j + 1, E);
+  cut = false;
+  if (J > 0 && tab.t[J - 1] > t_end) {
+    int lo = 0, hi = J - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (tab.t[mid] > t_end) hi = mid;
+      else lo = mid + 1;
+    }
+    J = lo;
+    cut = true;
+  }
+}
+
 template <int kC>
 __global__ void __launch_bounds__(kThreads) downstream_lattice_kernel(Box b, const float* __restrict__ vol, int C,
                                                                       const float* __restrict__ omegas,
@@ -690,26 +749,9 @@ __global__ void __launch_bounds__(kThreads) downstream_lattice_kernel(Box b, con
                                                                       const int32_t* __restrict__ table,
                                                                       float* __restrict__ out, int64_t os_k,
                                                                       int64_t os_c, int64_t os_v) {
-  // [4E] words of this direction: the steps (segment length, flat index step) as int2 [E] (E rounded up to even, so
-  // that two steps are one 16-byte load), then t [E] and first [E]
   extern __shared__ int4 s_tab4[];
   const int k = blockIdx.y;
-  const int E = b.n[0] + b.n[1] + b.n[2];
-  const int E2 = (E + 1) & ~1;
-  int2* s_step = reinterpret_cast<int2*>(s_tab4);
-  int32_t* s_words = reinterpret_cast<int32_t*>(s_tab4) + 2 * E2;
-  const int32_t* src = table + (int64_t)k * 3 * E;
-  for (int i = threadIdx.x; i < E; i += kThreads) {
-    // the length of the segment that ends at crossing i: t[i] - t[i - 1] (t[-1] = 0), as the walk forms it
-    const float tj = __int_as_float(src[i]), tp = i > 0 ? __int_as_float(src[i - 1]) : 0.f;
-    s_step[i] = make_int2(__float_as_int(tj - tp), src[E + i]);
-    s_words[i] = src[i];
-    s_words[E + i] = src[2 * E + i];
-  }
-  if (threadIdx.x == 0 && E2 > E) s_step[E] = make_int2(0, 0);
-  __syncthreads();
-  const float* t_cross = reinterpret_cast<const float*>(s_words);
-  const int32_t* first = s_words + E;
+  const LatticeTable tab = stage_lattice(s_tab4, table, k, b.n[0] + b.n[1] + b.n[2], 1);
   const int64_t v = (int64_t)blockIdx.x * kThreads + threadIdx.x;
   if (v >= V) return;
   const int nC = kC > 0 ? kC : C;
@@ -723,68 +765,20 @@ __global__ void __launch_bounds__(kThreads) downstream_lattice_kernel(Box b, con
   const int64_t rem = v - (int64_t)iy * nzx;
   const int ix = (int)(rem / b.n[2]);
   const int iz = (int)(rem - (int64_t)ix * b.n[2]);
-  const float r[3] = {voxel_centre(b, 0, ix), voxel_centre(b, 1, iy), voxel_centre(b, 2, iz)};
   const float w[3] = {omegas[3 * k], omegas[3 * k + 1], omegas[3 * k + 2]};
-  float t_end = fminf(fmaxf(panel_distance(panel, r, w), 0.f), diagonal);
-  // the crossing that leaves the box: along axis a after the voxels left between i_a and the face ahead
-  const int idx[3] = {ix, iy, iz};
-  const int off[3] = {0, b.n[0], b.n[0] + b.n[1]};
-  int exit_j = E;
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    if (w[a] == 0.f) continue;
-    const int left = w[a] > 0.f ? b.n[a] - 1 - idx[a] : idx[a];
-    exit_j = min(exit_j, first[off[a] + left]);
-  }
-  if (exit_j < E) t_end = fminf(t_end, t_cross[exit_j]);
-  // the segments ending at crossings 0 .. J - 1 are whole (t_j <= t_end); the one ending at crossing J, when the ray
-  // ends before its exit crossing, is cut at t_end (the first j with t_j > t_end, by bisection of the sorted table)
-  int J = min(exit_j + 1, E);
-  bool cut = false;
-  if (J > 0 && t_cross[J - 1] > t_end) {
-    int lo = 0, hi = J - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if (t_cross[mid] > t_end) hi = mid;
-      else lo = mid + 1;
-    }
-    J = lo;
-    cut = true;
-  }
+  int J;
+  bool cut;
+  float t_end;
+  lattice_ray(b, panel, tab, w, diagonal, ix, iy, iz, J, cut, t_end);
   float acc[kC > 0 ? kC : kMaxChannels];
   for (int c = 0; c < nC; ++c) acc[c] = 0.f;
   int cur = (int)v;
-  int j = 0;
-  if (kC == 2) {
-    // four segments at a time: the four gathers are issued before their sums (the crossing table gives every step's
-    // voxel in advance)
-    for (; j + 4 <= J; j += 4) {
-      const int4 e01 = s_tab4[j >> 1], e23 = s_tab4[(j >> 1) + 1];  // steps j .. j + 3 (j even)
-      const int c1 = cur + e01.y, c2 = c1 + e01.w, c3 = c2 + e23.y;
-      const float2 q0 = __ldg(reinterpret_cast<const float2*>(vol) + cur);
-      const float2 q1 = __ldg(reinterpret_cast<const float2*>(vol) + c1);
-      const float2 q2 = __ldg(reinterpret_cast<const float2*>(vol) + c2);
-      const float2 q3 = __ldg(reinterpret_cast<const float2*>(vol) + c3);
-      const float s0 = __int_as_float(e01.x), s1 = __int_as_float(e01.z), s2 = __int_as_float(e23.x),
-                  s3 = __int_as_float(e23.z);
-      acc[0] = fmaf(s0, q0.x, acc[0]);
-      acc[kC > 1 ? 1 : 0] = fmaf(s0, q0.y, acc[kC > 1 ? 1 : 0]);
-      acc[0] = fmaf(s1, q1.x, acc[0]);
-      acc[kC > 1 ? 1 : 0] = fmaf(s1, q1.y, acc[kC > 1 ? 1 : 0]);
-      acc[0] = fmaf(s2, q2.x, acc[0]);
-      acc[kC > 1 ? 1 : 0] = fmaf(s2, q2.y, acc[kC > 1 ? 1 : 0]);
-      acc[0] = fmaf(s3, q3.x, acc[0]);
-      acc[kC > 1 ? 1 : 0] = fmaf(s3, q3.y, acc[kC > 1 ? 1 : 0]);
-      cur = c3 + e23.w;
-    }
-  }
-  // the remaining whole segments, then the cut one (step j == J)
-  for (; j <= J; ++j) {
+  for (int j = 0; j <= J; ++j) {  // the whole segments, then the cut one (j == J)
     float seg;
     if (j < J) {
-      seg = __int_as_float(s_step[j].x);
+      seg = __int_as_float(tab.step[j].x);
     } else {
-      const float prev = j > 0 ? t_cross[j - 1] : 0.f;
+      const float prev = j > 0 ? tab.t[j - 1] : 0.f;
       if (!cut || !(prev < t_end)) break;
       seg = t_end - prev;
     }
@@ -798,14 +792,10 @@ __global__ void __launch_bounds__(kThreads) downstream_lattice_kernel(Box b, con
         acc[c + 2] = fmaf(seg, q.z, acc[c + 2]);
         acc[c + 3] = fmaf(seg, q.w, acc[c + 3]);
       }
-    } else if (kC == 2) {
-      const float2 q = __ldg(reinterpret_cast<const float2*>(vox));
-      acc[0] = fmaf(seg, q.x, acc[0]);
-      acc[kC > 1 ? 1 : 0] = fmaf(seg, q.y, acc[kC > 1 ? 1 : 0]);
     } else {
       for (int c = 0; c < nC; ++c) acc[c] = fmaf(seg, __ldg(vox + c), acc[c]);
     }
-    if (j < J) cur += s_step[j].y;
+    if (j < J) cur += tab.step[j].y;
   }
   if ((kC == 8 || kC == 4) && os_c == 1 && os_v == nC) {  // voxel-major out: the channels of a ray in float4s
 #pragma unroll
@@ -813,6 +803,92 @@ __global__ void __launch_bounds__(kThreads) downstream_lattice_kernel(Box b, con
       *reinterpret_cast<float4*>(o + c) = make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]);
   } else {
     for (int c = 0; c < nC; ++c) o[(int64_t)c * os_c] = acc[c];
+  }
+}
+
+// Two channels, kRays neighbouring rays per thread along x. The rays of a direction take the same steps, so the table's
+// lengths and the flat offset are read and added once for all of them; their bases differ by whole rows. Whole segments
+// run four at a time (four steps x kRays gathers in flight) up to the shortest ray, the rest and the cut segments one
+// at a time. Each ray's sums run in the order of its segments, two channels per packed multiply-add.
+// One ray per thread was bound by the load-store pipe (76 % busy: a 16-byte broadcast of the table is four wavefronts, a
+// gather of 32 float2 at any offset three or four) and by issue (75 %); the gathers remain. 512 directions: 64^3 voxels
+// 3.87 -> 3.51 ms, 32^3 372 -> 281 us.
+template <int kRays>
+__global__ void __launch_bounds__(kThreads) downstream_lattice_rays_kernel(
+    Box b, const float2* __restrict__ vol, const float* __restrict__ omegas, const uint8_t* __restrict__ toward,
+    Panel panel, float diagonal, const int32_t* __restrict__ table, float* __restrict__ out, int64_t os_k, int64_t os_c,
+    int64_t os_v) {
+  extern __shared__ int4 s_tab4[];
+  const int k = blockIdx.y, nx = b.n[0], nz = b.n[2], ng = (nx + kRays - 1) / kRays;
+  const LatticeTable tab = stage_lattice(s_tab4, table, k, nx + b.n[1] + nz, (int)sizeof(float2));
+  const int64_t id = (int64_t)blockIdx.x * kThreads + threadIdx.x, per_row = (int64_t)ng * nz;
+  const int iy = (int)(id / per_row);
+  if (iy >= b.n[1]) return;
+  const int rem = (int)(id - iy * per_row), ix = rem / nz * kRays, iz = rem - rem / nz * nz;
+  const int64_t v = ((int64_t)iy * nx + ix) * nz + iz;
+  float* o = out + (int64_t)k * os_k + v * os_v;
+  if (!faces_panel(panel, toward, omegas, k)) {
+    for (int r = 0; r < kRays && ix + r < nx; ++r) {
+      o[r * nz * os_v] = INFINITY;
+      o[r * nz * os_v + os_c] = INFINITY;
+    }
+    return;
+  }
+  const float w[3] = {omegas[3 * k], omegas[3 * k + 1], omegas[3 * k + 2]};
+  int J[kRays];        // whole segments
+  float last[kRays];   // length of the cut segment, 0 for none
+  const char* base[kRays];
+  uint64_t acc[kRays];
+  int common = 1 << 30, most = 0;
+#pragma unroll
+  for (int r = 0; r < kRays; ++r) {
+    const int rr = ix + r < nx ? r : 0;  // past the row: the first ray again, not stored
+    bool cut;
+    float t_end;
+    lattice_ray(b, panel, tab, w, diagonal, ix + rr, iy, iz, J[r], cut, t_end);
+    const float prev = J[r] > 0 ? tab.t[J[r] - 1] : 0.f;
+    last[r] = cut && prev < t_end ? t_end - prev : 0.f;
+    base[r] = reinterpret_cast<const char*>(vol + (int64_t)rr * nz);
+    acc[r] = 0;
+    common = min(common, J[r]);
+    most = max(most, J[r] + (last[r] > 0.f ? 1 : 0));
+  }
+  // signed: past the end of the first ray it may lie before the volume, where a later ray's base still adds a row
+  int cur = (int)v * (int)sizeof(float2);
+  int j = 0;
+  for (; j + 4 <= common; j += 4) {
+    const int4 e01 = s_tab4[j >> 1], e23 = s_tab4[(j >> 1) + 1];  // steps j .. j + 3 (j even)
+    const int c[4] = {cur, cur + e01.y, cur + e01.y + e01.w, cur + e01.y + e01.w + e23.y};
+    const int len[4] = {e01.x, e01.z, e23.x, e23.z};
+    uint64_t q[4][kRays];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int r = 0; r < kRays; ++r) q[i][r] = __ldg(reinterpret_cast<const unsigned long long*>(base[r] + c[i]));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint64_t s = pack2(__int_as_float(len[i]), __int_as_float(len[i]));
+#pragma unroll
+      for (int r = 0; r < kRays; ++r) acc[r] = fma2(s, q[i][r], acc[r]);
+    }
+    cur = c[3] + e23.w;
+  }
+  for (; j < most; ++j) {
+    const int2 e = tab.step[j];  // j <= J <= E: the table is padded to E rounded up to even, or holds t after it
+#pragma unroll
+    for (int r = 0; r < kRays; ++r) {
+      const float seg = j < J[r] ? __int_as_float(e.x) : j == J[r] ? last[r] : 0.f;
+      if (j < J[r] || (j == J[r] && seg > 0.f))
+        acc[r] = fma2(pack2(seg, seg), __ldg(reinterpret_cast<const unsigned long long*>(base[r] + cur)), acc[r]);
+    }
+    cur += e.y;
+  }
+#pragma unroll
+  for (int r = 0; r < kRays; ++r) {
+    if (ix + r >= nx) break;
+    const float2 a = unpack2(acc[r]);
+    o[r * nz * os_v] = a.x;
+    o[r * nz * os_v + os_c] = a.y;
   }
 }
 
@@ -1066,12 +1142,22 @@ int downstream(const float* volume, int64_t channels, const double* box, const i
     note_launches();
   }
   const size_t smem = (size_t)(2 * ((E + 1) & ~1) + 2 * E) * sizeof(int32_t);
+  // two channels up to 1 GiB: byte offsets, one step beyond the volume included, fit 32 signed bits
+  if (C == 2 && V <= (1ll << 27)) {
+    constexpr int kRays = 2;  // 4: 1 % slower at 64^3, 3 % at 32^3
+    const int64_t threads = (dims[0] + kRays - 1) / kRays * dims[1] * dims[2];
+    grid.x = (unsigned)cdiv(threads, kThreads);
+    downstream_lattice_rays_kernel<kRays><<<grid, kThreads, smem, s>>>(b, reinterpret_cast<const float2*>(volume), omegas,
+                                                                       toward, p, (float)diagonal, crossings, out, os_k,
+                                                                       os_c, os_v);
+    note_launches();
+    return launch_status("citrus_downstream_cumulative");
+  }
 #define CITRUS_LATTICE(KC)                                                                                        \
   downstream_lattice_kernel<KC><<<grid, kThreads, smem, s>>>(b, volume, C, omegas, toward, p, (float)diagonal, V, \
                                                             crossings, out, os_k, os_c, os_v)
   switch (C) {
     case 1: CITRUS_LATTICE(1); break;
-    case 2: CITRUS_LATTICE(2); break;
     case 4: CITRUS_LATTICE(4); break;
     case 8: CITRUS_LATTICE(8); break;
     default: CITRUS_LATTICE(0); break;
