@@ -201,7 +201,7 @@ def sweep_config(ctx, mu_cells, num_groups: int, views: int, default=None, dc: i
         default = (2, 2, -tile, 1) if tile else (4, 2, 0, 1)
     # "form" names the forms' meaning: entries timed before the pencil schedule existed are not reused
     key = Autotuner.key("sweep", device, N=N, D8=D8, G=num_groups, shape="x".join(map(str, ctx.shape)),
-                        form="views-per-thread+tiles+pencils")
+                        form="views-per-thread+pencils-16")
     entry = tuner().table.get(key)
     if entry is None and not torch.cuda.is_current_stream_capturing():
         free, _ = torch.cuda.mem_get_info(device)

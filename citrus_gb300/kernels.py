@@ -142,10 +142,11 @@ PENCIL_THREADS = 512  # threads of a block of the pencil schedule at most
 
 
 def pencil_tile(num_groups: int) -> int:
-    """Edge of the pencil schedule's tiles: the largest of 8, 4 and 2 whose block holds every group of a direction, 0
-    for none. Larger tiles read fewer faces and wait less often (48^3 cells, 120 directions: 12 groups 1.52 ms in
-    tiles of 4, 1.99 in tiles of 2; 40^3, 6 groups, 128 directions: 0.59 ms in tiles of 8, 0.71 in tiles of 4)."""
-    return next((t for t in (8, 4, 2) if t * t * num_groups <= PENCIL_THREADS), 0)
+    """Edge of the pencil schedule's tiles, 0 for none: the largest of 16, 12, 8, 4, 3 and 2 whose block holds every
+    group of a direction. Larger tiles read fewer faces and wait less often, but 5, 7 and 11 fill their warps badly.
+    120 directions: 32^3 cells, 1 group 0.21 ms in tiles of 8, 0.16 in tiles of 16; 48^3, 3 groups 0.63 (8), 0.57 (12);
+    4 groups 0.67 (8), 0.74 (11); 12 groups 1.99 (2), 1.55 (4), 1.57 (6); 16 groups 1.82 (4), 2.09 (5)."""
+    return next((t for t in (16, 12, 8, 4, 3, 2) if t * t * num_groups <= PENCIL_THREADS), 0)
 
 
 def sweep_pencils(shape, store: Tensor, mu_cells: Tensor, c: Tensor, *, tile: int = 8, dirs_per_block: int = 1,

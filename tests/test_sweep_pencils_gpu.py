@@ -23,6 +23,7 @@ pytestmark = pytest.mark.gpu
     ((33, 2, 9), 16, 2, 4, 2),       # 512 threads
     ((3, 20, 5), 1, 2, 16, 2),       # the largest tile
     ((6, 6, 6), 170, 1, 1, 1),       # one pencil per block
+    ((13, 25, 4), 3, 1, 12, 1),      # a last warp of 16 threads
     ((20, 11, 3), 1, 2, 2, 2),       # 10 x 6 tiles: diagonals that grow, stay and shrink
     ((7, 22, 3), 2, 1, 2, 1),        # 4 x 11 tiles
 ])
