@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(kTcThreads) gemm_tc_kernel(const float* __rest
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar_addr)
                    : "memory");
     }
-    const bool ok = mbar_wait(mbar_addr, phase, global_timer_ns());
+    const bool ok = mbar_wait(mbar_addr, phase);
     phase ^= 1u;
     if (!ok) {
       if (error_word != nullptr) atomicExch(error_word, 1u);
@@ -196,29 +196,40 @@ __global__ void __launch_bounds__(kTcThreads) gemm_tc_kernel(const float* __rest
 // ---- the warp-specialised form ------------------------------------------------------------------------------------
 // The same product as gemm_tc_kernel with its stages overlapped, one CTA per SM walking its tiles in order:
 //
-//   * loader (one thread of warp 13): the [K x 128] float32 tile of B comes in one tensor copy (cp.async.bulk.tensor
+//   * loader (one thread of warp 21): the [K x 128] float32 tile of B comes in one tensor copy (cp.async.bulk.tensor
 //     through a tensor map of B as [batch][K][J], completing on the stage's mbarrier with the box's byte count;
 //     columns past J read as zeros), or, where the map cannot be made, as K bulk copies of its 512-byte row runs, into
 //     a ring of float32 stages (as many as the shared memory holds, up to kWsRawMax). One request per tile instead of
 //     K: the per-request cost of K small copies held the loads near 1.3 TB/s;
-//   * converters (warps 8 to 11): thread t splits column t of a raw stage into the bfloat16 high and low operand
+//   * converters (warps 16 to 19): thread t splits column t of a raw stage into the bfloat16 high and low operand
 //     tiles in the K-major core-matrix layout (kWsOps stages), then frees the raw stage;
-//   * MMA issuer (one thread of warp 12): 3 x (K / 16) tcgen05.mma per tile into one of two float32 accumulators in
+//   * MMA issuer (one thread of warp 20): 3 x (K / 16) tcgen05.mma per tile into one of two float32 accumulators in
 //     tensor memory, committed to the operand stage (freed once read) and to the accumulator (full);
-//   * epilogue (warps 0 to 7): warp w reads accumulator lanes 32 (w % 4) .. + 31 (columns of C) and every other
+//   * epilogue (warps 0 to 15): warp w reads accumulator lanes 32 (w % 4) .. + 31 (columns of C) and every fourth
 //     16 of its rows, and writes (or adds to) C, so that the stores of one tile overlap the loads, splits and MMAs
-//     of the next; the means come from their own two-stage ring (one tensor copy of [M][32] per tile).
+//     of the next; the rows of C that it adds to are loaded before it waits for the accumulator; the means come from
+//     their own two-stage ring (one tensor copy of [M][32] per tile).
+//
+// An inner dimension above 64 goes through the rings in two parts of at most 64 rows, each with an accumulator of its
+// own; the epilogue adds them in order, which is what two calls that accumulate give, bit for bit, without writing and
+// reading C in between.
+//
+// What bounds it is memory: 12.6 M columns, 120 x 64 2.43 -> 1.50 ms (91 % of a copy's bandwidth), 64 x 64 accumulating
+// 2.65 -> 1.60 ms (89 %), 64 x 120 accumulating 5.29 -> 2.37 ms (78 %). Before, converting in integer arithmetic (20
+// instructions a pair) beside polling warps took as long as the loads, and eight epilogue warps held too few rows of C in
+// flight (8: 1.88 ms, 12: 1.67 ms at 120 x 64); eight converter warps gained nothing (1.57 ms).
 //
 // The MMAs run in gemm_tc_kernel's order and the epilogue adds in its order: the two forms give the same bits. Every
 // mbarrier wait is bounded by kTcTimeoutNs; a role whose wait runs out records the error and stops, the others then
 // stop at their own bounded waits, the issuer waits (bounded) for its last MMAs, and the CTA frees its tensor memory.
 constexpr int kWsRawMax = 3;              // float32 stages of B (deeper rings measured no faster with tensor copies)
 constexpr int kWsOps = 2;                 // bf16 hi/lo operand stages
-constexpr int kWsThreads = 14 * 32;       // 8 epilogue, 4 converter, 1 MMA and 1 loader warps
-constexpr int kWsEpilogueWarps = 8;
-constexpr int kWsConverterWarp0 = 8;
-constexpr int kWsMmaWarp = 12;
-constexpr int kWsLoaderWarp = 13;
+constexpr int kWsPartK = 64;              // inner rows of a part
+constexpr int kWsThreads = 22 * 32;       // 16 epilogue, 4 converter, 1 MMA and 1 loader warps
+constexpr int kWsEpilogueWarps = 16;
+constexpr int kWsConverterWarp0 = 16;
+constexpr int kWsMmaWarp = 20;
+constexpr int kWsLoaderWarp = 21;
 constexpr size_t kWsMeansBytes = 2 * kTcM * 32 * 4;  // two [M <= 128][32] float32 tiles of the means
 
 __device__ __forceinline__ void mbar_init(uint32_t mbar, uint32_t count) {
@@ -253,15 +264,16 @@ __global__ void __launch_bounds__(kWsThreads, 1) gemm_ws_kernel(const float* __r
                                                                 const __grid_constant__ CUtensorMap f_map,
                                                                 int use_f_map) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  const int KS = (K + 15) / 16;
+  const int KS = (K + 15) / 16, parts = (K + kWsPartK - 1) / kWsPartK;
+  const int part_rows = K < kWsPartK ? K : kWsPartK, part_steps = (part_rows + 15) / 16;
   const uint32_t a_step = kTcM * 16 * 2, b_step = kTcN * 16 * 2;
-  const uint32_t raw_bytes = (uint32_t)K * kTcN * 4;
+  const uint32_t raw_bytes = (uint32_t)part_rows * kTcN * 4;
   const uint32_t raw_stride = (raw_bytes + 1023u) & ~1023u;
   uint8_t* a_hi = smem;
   uint8_t* a_lo = a_hi + KS * a_step;
   uint8_t* ops = a_lo + KS * a_step;                                 // kWsOps x (hi, lo)
-  const uint32_t op_bytes = 2u * KS * b_step;
-  float* raw = reinterpret_cast<float*>(ops + kWsOps * op_bytes);   // raw_stages x [K][128]
+  const uint32_t op_bytes = 2u * part_steps * b_step;
+  float* raw = reinterpret_cast<float*>(ops + kWsOps * op_bytes);   // raw_stages x [part_rows][128]
   __shared__ __align__(8) uint64_t bar[2 * kWsRawMax + 2 * kWsOps + 9];
   __shared__ uint32_t tmem_base;
   __shared__ volatile int abort_flag;
@@ -320,11 +332,11 @@ __global__ void __launch_bounds__(kWsThreads, 1) gemm_ws_kernel(const float* __r
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   const int n_t = ((M + 15) / 16) * 16;
-  const uint32_t acc_cols = n_t <= 64 ? 64u : 128u;  // one accumulator; two are allocated
+  const uint32_t acc_cols = n_t <= 64 ? 64u : 128u;  // one accumulator; two per part are allocated
   const uint32_t idesc = idesc_bf16(n_t);
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
-                 "r"(2 * acc_cols)
+                 "r"(2 * parts * acc_cols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -343,7 +355,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) gemm_ws_kernel(const float* __r
     if (lane == 1 && f_tma) {  // the means: one tensor copy of [M][32] per tile, two stages ahead of the epilogue
       for (int64_t i = 0; i < my_tiles && !abort_flag; ++i) {
         const int fs = (int)(i & 1);
-        if (!mbar_wait(smem_u32(f_empty + fs), (uint32_t)((i >> 1) & 1) ^ 1u, global_timer_ns())) {
+        if (!mbar_wait(smem_u32(f_empty + fs), (uint32_t)((i >> 1) & 1) ^ 1u)) {
           fail();
           break;
         }
@@ -360,12 +372,14 @@ __global__ void __launch_bounds__(kWsThreads, 1) gemm_ws_kernel(const float* __r
       }
     }
     if (lane == 0) {
-      for (int64_t i = 0; i < my_tiles && !abort_flag; ++i) {
-        const int st = (int)(i % raw_stages);
-        if (!mbar_wait(smem_u32(raw_empty + st), (uint32_t)((i / raw_stages) & 1) ^ 1u, global_timer_ns())) {
+      for (int64_t u = 0; u < my_tiles * parts && !abort_flag; ++u) {
+        const int st = (int)(u % raw_stages);
+        if (!mbar_wait(smem_u32(raw_empty + st), (uint32_t)((u / raw_stages) & 1) ^ 1u)) {
           fail();
           break;
         }
+        const int64_t i = u / parts;
+        const int k0 = (int)(u - i * parts) * kWsPartK, rows = K - k0 < kWsPartK ? K - k0 : kWsPartK;
         const int64_t tile = blockIdx.x + i * gridDim.x;
         const int64_t bz = tile / tiles_per_batch;
         const int64_t n0 = (tile - bz * tiles_per_batch) * kTcN;
@@ -373,38 +387,40 @@ __global__ void __launch_bounds__(kWsThreads, 1) gemm_ws_kernel(const float* __r
         const uint32_t mb = smem_u32(raw_full + st);
         const uint32_t dst = smem_u32(reinterpret_cast<uint8_t*>(raw) + st * raw_stride);
         if (use_map) {
-          mbar_expect_tx(mb, (uint32_t)K * kTcN * 4);  // the whole box, its columns past J filled with zeros
+          mbar_expect_tx(mb, raw_bytes);  // the whole box, its columns past J and rows past K filled with zeros
           asm volatile(
               "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, "
               "%4}], [%5];" ::"r"(dst),
-              "l"(reinterpret_cast<uint64_t>(&b_map)), "r"((int)n0), "r"(0), "r"((int)bz), "r"(mb)
+              "l"(reinterpret_cast<uint64_t>(&b_map)), "r"((int)n0), "r"(k0), "r"((int)bz), "r"(mb)
               : "memory");
         } else {
-          mbar_expect_tx(mb, bytes * (uint32_t)K);
-          const float* src = B + bz * stride_b + n0;
-          for (int k = 0; k < K; ++k) bulk_copy_g2s(dst + (uint32_t)k * kTcN * 4, src + (int64_t)k * ldb, bytes, mb);
+          mbar_expect_tx(mb, bytes * (uint32_t)rows);
+          const float* src = B + bz * stride_b + n0 + (int64_t)k0 * ldb;
+          for (int k = 0; k < rows; ++k) bulk_copy_g2s(dst + (uint32_t)k * kTcN * 4, src + (int64_t)k * ldb, bytes, mb);
         }
       }
     }
   } else if (warp >= kWsConverterWarp0 && warp < kWsConverterWarp0 + 4) {
     const int t = tid - kWsConverterWarp0 * 32;  // the tile column this thread splits
-    for (int64_t i = 0; i < my_tiles && !abort_flag; ++i) {
-      const int st = (int)(i % raw_stages), op = (int)(i % kWsOps);
-      if (!mbar_wait(smem_u32(raw_full + st), (uint32_t)((i / raw_stages) & 1), global_timer_ns()) ||
-          !mbar_wait(smem_u32(op_empty + op), (uint32_t)((i / kWsOps) & 1) ^ 1u, global_timer_ns())) {
+    for (int64_t u = 0; u < my_tiles * parts && !abort_flag; ++u) {
+      const int st = (int)(u % raw_stages), op = (int)(u % kWsOps);
+      const int k0 = (int)(u % parts) * kWsPartK, rows = K - k0 < kWsPartK ? K - k0 : kWsPartK;
+      if (!mbar_wait(smem_u32(raw_full + st), (uint32_t)((u / raw_stages) & 1)) ||
+          !mbar_wait(smem_u32(op_empty + op), (uint32_t)((u / kWsOps) & 1) ^ 1u)) {
         fail();
         break;
       }
       const float* col = reinterpret_cast<const float*>(reinterpret_cast<uint8_t*>(raw) + st * raw_stride) + t;
       uint8_t* o_hi = ops + op * op_bytes;
-      uint8_t* o_lo = o_hi + KS * b_step;
-      for (int s = 0; s < KS; ++s)
+      uint8_t* o_lo = o_hi + part_steps * b_step;
+      const int steps = (rows + 15) / 16;
+      for (int s = 0; s < steps; ++s)
         for (int k8 = 0; k8 < 16; k8 += 8) {
           float x[8];
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
             const int k = s * 16 + k8 + q;
-            x[q] = k < K ? col[k * kTcN] : 0.f;
+            x[q] = k < rows ? col[k * kTcN] : 0.f;
           }
           uint4 hi, lo;
           split_pair(x[0], x[1], hi.x, lo.x);
@@ -421,95 +437,99 @@ __global__ void __launch_bounds__(kWsThreads, 1) gemm_ws_kernel(const float* __r
     }
   } else if (warp == kWsMmaWarp) {
     if (lane == 0) {
-      for (int64_t i = 0; i < my_tiles && !abort_flag; ++i) {
-        const int op = (int)(i % kWsOps), ac = (int)(i & 1);
-        if (!mbar_wait(smem_u32(op_full + op), (uint32_t)((i / kWsOps) & 1), global_timer_ns()) ||
-            !mbar_wait(smem_u32(acc_empty + ac), (uint32_t)((i >> 1) & 1) ^ 1u, global_timer_ns())) {
+      for (int64_t u = 0; u < my_tiles * parts && !abort_flag; ++u) {
+        const int64_t i = u / parts;
+        const int part = (int)(u - i * parts), op = (int)(u % kWsOps), ac = (int)(i & 1);
+        if (!mbar_wait(smem_u32(op_full + op), (uint32_t)((u / kWsOps) & 1)) ||
+            (part == 0 && !mbar_wait(smem_u32(acc_empty + ac), (uint32_t)((i >> 1) & 1) ^ 1u))) {
           fail();
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t d = tmem + (uint32_t)ac * acc_cols;
+        const uint32_t d = tmem + (uint32_t)(ac * parts + part) * acc_cols;
         uint8_t* o_hi = ops + op * op_bytes;
-        uint8_t* o_lo = o_hi + KS * b_step;
-        for (int s = 0; s < KS; ++s) {
+        uint8_t* o_lo = o_hi + part_steps * b_step;
+        const int s0 = part * (kWsPartK / 16), s1 = KS - s0 < kWsPartK / 16 ? KS : s0 + kWsPartK / 16;
+        for (int s = s0; s < s1; ++s) {
           const uint64_t ah = smem_desc(smem_u32(a_hi + s * a_step), 128, 256);
           const uint64_t al = smem_desc(smem_u32(a_lo + s * a_step), 128, 256);
-          const uint64_t bh = smem_desc(smem_u32(o_hi + s * b_step), 128, 256);
-          const uint64_t bl = smem_desc(smem_u32(o_lo + s * b_step), 128, 256);
-          mma_bf16(d, bh, ah, idesc, s > 0 ? 1u : 0u);
+          const uint64_t bh = smem_desc(smem_u32(o_hi + (s - s0) * b_step), 128, 256);
+          const uint64_t bl = smem_desc(smem_u32(o_lo + (s - s0) * b_step), 128, 256);
+          mma_bf16(d, bh, ah, idesc, s > s0 ? 1u : 0u);
           mma_bf16(d, bh, al, idesc, 1u);
           mma_bf16(d, bl, ah, idesc, 1u);
         }
         tc_commit(smem_u32(op_empty + op));
-        tc_commit(smem_u32(acc_full + ac));
+        if (part == parts - 1) tc_commit(smem_u32(acc_full + ac));
       }
       tc_commit(smem_u32(mma_done));  // tracks every MMA issued above
-      if (!mbar_wait(smem_u32(mma_done), 0u, global_timer_ns())) fail();
+      if (!mbar_wait(smem_u32(mma_done), 0u)) fail();
     }
-  } else {  // epilogue warps 0 .. 7
-    const int quarter = warp % 4, half = warp / 4;
+  } else {  // epilogue warps
+    const int quarter = warp % 4, m_first = warp / 4 * 16;
     for (int64_t i = 0; i < my_tiles && !abort_flag; ++i) {
       const int ac = (int)(i & 1);
-      if (!mbar_wait(smem_u32(acc_full + ac), (uint32_t)((i >> 1) & 1), global_timer_ns())) {
+      const int64_t tile = blockIdx.x + i * gridDim.x;
+      const int64_t bz = tile / tiles_per_batch;
+      const int64_t n0 = (tile - bz * tiles_per_batch) * kTcN;
+      const float* Fz = F != nullptr ? F + bz * stride_f : nullptr;
+      const uint32_t taddr = tmem + (uint32_t)(ac * parts) * acc_cols + ((uint32_t)(quarter * 32) << 16);
+      const float* fst = f_stage + (int)(i & 1) * M * 32;
+      // accumulator lane 32 quarter + lane is column n0 + 32 quarter + lane of C; its columns are the rows of C,
+      // in 16-row steps over the four groups of epilogue warps
+      const int64_t col = n0 + quarter * 32 + lane;
+      float* Cz = C + bz * stride_c + col;
+      const bool add = accumulate || (Fz != nullptr && (col & 3) == 0);
+      float prev[16];
+      const auto load_c = [&](int m0) {
+#pragma unroll
+        for (int q = 0; q < 16; ++q) prev[q] = col < J && m0 + q < M ? Cz[(int64_t)(m0 + q) * ldc] : 0.f;
+      };
+      if (accumulate) load_c(m_first);
+      if (!mbar_wait(smem_u32(acc_full + ac), (uint32_t)((i >> 1) & 1))) {
         fail();
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int64_t tile = blockIdx.x + i * gridDim.x;
-      const int64_t bz = tile / tiles_per_batch;
-      const int64_t n0 = (tile - bz * tiles_per_batch) * kTcN;
-      float* Cz = C + bz * stride_c;
-      const float* Fz = F != nullptr ? F + bz * stride_f : nullptr;
-      const uint32_t taddr = tmem + (uint32_t)ac * acc_cols + ((uint32_t)(quarter * 32) << 16);
-      const float* fst = f_stage + (int)(i & 1) * M * 32;
-      if (f_tma && !mbar_wait(smem_u32(f_full + (int)(i & 1)), (uint32_t)((i >> 1) & 1), global_timer_ns())) {
+      if (f_tma && !mbar_wait(smem_u32(f_full + (int)(i & 1)), (uint32_t)((i >> 1) & 1))) {
         fail();
         break;
       }
-      {
-        // accumulator lane 32 quarter + lane is column n0 + 32 quarter + lane of C; its columns are the rows of C,
-        // split in 16-row steps between the two halves of the epilogue warps
-        const int64_t col = n0 + quarter * 32 + lane;
-        const bool add = accumulate || (Fz != nullptr && (col & 3) == 0);
-        for (int m0 = half * 16; m0 < n_t; m0 += 32) {
-          const int rows = min(16, M - m0);
-          float* out = Cz + (int64_t)m0 * ldc + col;
-          // the loads of C (accumulating) or of the means are issued before the tensor-memory load, so that the two
-          // latencies overlap
-          float prev[16];
+      for (int m0 = m_first; m0 < n_t; m0 += 16 * (kWsEpilogueWarps / 4)) {
+        const int rows = min(16, M - m0);
+        if (accumulate) {
+          if (m0 != m_first) load_c(m0);
+        } else {
 #pragma unroll
           for (int q = 0; q < 16; ++q) prev[q] = 0.f;
-          if (col < J) {
-            if (accumulate) {
+          if (add && col < J) {
+            const int fc = (quarter * 32 + lane) >> 2;  // the tile's column / 4
 #pragma unroll
-              for (int q = 0; q < 16; ++q)
-                if (q < rows) prev[q] = out[(int64_t)q * ldc];
-            } else if (add && f_tma) {
-              const int fc = (quarter * 32 + lane) >> 2;  // the tile's column / 4
-#pragma unroll
-              for (int q = 0; q < 16; ++q)
-                if (q < rows) prev[q] = fst[(m0 + q) * 32 + fc];
-            } else if (add) {
-#pragma unroll
-              for (int q = 0; q < 16; ++q)
-                if (q < rows) prev[q] = __ldg(Fz + (int64_t)(m0 + q) * ldf + (col >> 2));
-            }
+            for (int q = 0; q < 16; ++q)
+              if (q < rows)
+                prev[q] = f_tma ? fst[(m0 + q) * 32 + fc] : __ldg(Fz + (int64_t)(m0 + q) * ldf + (col >> 2));
           }
+        }
+        for (int part = 0; part < parts; ++part) {
           uint32_t r[16];
           asm volatile(
               "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
               "%14, %15}, [%16];"
               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
                 "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-              : "r"(taddr + (uint32_t)m0)
+              : "r"(taddr + (uint32_t)(part * acc_cols) + (uint32_t)m0)
               : "memory");
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          if (col < J) {
 #pragma unroll
-            for (int q = 0; q < 16; ++q)
-              if (q < rows) out[(int64_t)q * ldc] = add ? prev[q] + __uint_as_float(r[q]) : __uint_as_float(r[q]);
+          for (int q = 0; q < 16; ++q) {
+            const float x = __uint_as_float(r[q]);
+            prev[q] = part > 0 || add ? prev[q] + x : x;
           }
+        }
+        if (col < J) {
+#pragma unroll
+          for (int q = 0; q < 16; ++q)
+            if (q < rows) Cz[(int64_t)(m0 + q) * ldc] = prev[q];
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -521,23 +541,25 @@ __global__ void __launch_bounds__(kWsThreads, 1) gemm_ws_kernel(const float* __r
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * acc_cols) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * parts * acc_cols) : "memory");
 }
 
 // shared memory of the warp-specialised form: A hi/lo, kWsOps operand stages, the float32 stages (1 KB aligned),
 // the two stages of the means; ws_raw_stages: as many float32 stages as fit 227 KB with the rest, up to kWsRawMax
 constexpr size_t kWsSmemLimit = 227 * 1024;
-size_t ws_raw_stride(int K) { return (((size_t)K * kTcN * 4) + 1023) & ~(size_t)1023; }
-size_t ws_fixed_bytes(int K) {
-  const size_t KS = (size_t)(K + 15) / 16;
-  return KS * 2 * kTcM * 16 * 2 + kWsOps * KS * 2 * kTcN * 16 * 2 + kWsMeansBytes;
+size_t ws_raw_stride(int K) { return (((size_t)std::min(K, kWsPartK) * kTcN * 4) + 1023) & ~(size_t)1023; }
+size_t ws_fixed_bytes(int K, bool means) {
+  const size_t KS = (size_t)(K + 15) / 16, part_steps = (size_t)(std::min(K, kWsPartK) + 15) / 16;
+  return KS * 2 * kTcM * 16 * 2 + kWsOps * part_steps * 2 * kTcN * 16 * 2 + (means ? kWsMeansBytes : 0);
 }
-int ws_raw_stages(int K) {
-  const size_t fixed = ws_fixed_bytes(K), stride = ws_raw_stride(K);
+int ws_raw_stages(int K, bool means) {
+  const size_t fixed = ws_fixed_bytes(K, means), stride = ws_raw_stride(K);
   const size_t n = fixed < kWsSmemLimit ? (kWsSmemLimit - fixed) / stride : 0;
   return (int)std::min<size_t>(n, kWsRawMax);
 }
-size_t ws_smem_bytes(int K) { return ws_fixed_bytes(K) + (size_t)std::max(ws_raw_stages(K), 2) * ws_raw_stride(K); }
+size_t ws_smem_bytes(int K, bool means) {
+  return ws_fixed_bytes(K, means) + (size_t)std::max(ws_raw_stages(K, means), 2) * ws_raw_stride(K);
+}
 
 }  // namespace
 }  // namespace citrus
@@ -563,7 +585,7 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 }
 
 // B as a float32 tensor [batch][K][J] (J innermost, rows ldb floats apart, batches stride_b floats apart) with a
-// [1][K][128] box: one tensor copy per tile. The launcher has checked the 16-byte alignment of B, ldb and stride_b.
+// [1][min(K, 64)][128] box: one tensor copy per part of a tile. The launcher has checked the 16-byte alignment of B, ldb and stride_b.
 // the means F as [batch][M][J / 4] with a [1][M][32] box (the 128 columns of a tile / 4); false when F's alignment,
 // row or batch strides do not allow a tensor map (the epilogue then reads F from global memory)
 bool encode_f_map(CUtensorMap* map, const float* F, int64_t M, int64_t J, int64_t ldf, int64_t batch,
@@ -587,7 +609,7 @@ bool encode_b_map(CUtensorMap* map, const float* B, int64_t K, int64_t J, int64_
   if (enc == nullptr || J > 0x7fffffffLL || batch > 0x7fffffffLL) return false;
   const cuuint64_t dims[3] = {(cuuint64_t)J, (cuuint64_t)K, (cuuint64_t)batch};
   const cuuint64_t strides[2] = {(cuuint64_t)ldb * 4, (cuuint64_t)(batch > 1 ? stride_b : ldb * K) * 4};
-  const cuuint32_t box[3] = {(cuuint32_t)kTcN, (cuuint32_t)K, 1u};
+  const cuuint32_t box[3] = {(cuuint32_t)kTcN, (cuuint32_t)std::min<int64_t>(K, kWsPartK), 1u};
   const cuuint32_t elem[3] = {1u, 1u, 1u};
   return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(B), dims, strides, box, elem,
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -617,8 +639,8 @@ int launch_gemm_tc(const char* name, const float* A, int64_t lda, const float* B
   const size_t b_bytes = (size_t)KS * 2 * kTcN * 16 * 2;
   const size_t smem = std::max<size_t>((size_t)KS * 2 * kTcM * 16 * 2 + b_bytes, 50 * 1024);
   // the warp-specialised form when B's rows are runs of 16-byte units (bulk copies) and its stages fit one CTA
-  const size_t ws_smem = ws_smem_bytes((int)K);
-  const int raw_stages = ws_raw_stages((int)K);
+  const size_t ws_smem = ws_smem_bytes((int)K, F != nullptr);
+  const int raw_stages = ws_raw_stages((int)K, F != nullptr);
   if (J % 4 == 0 && ldb % 4 == 0 && stride_b % 4 == 0 && ((uintptr_t)B % 16) == 0 && raw_stages >= 2 &&
       ws_smem <= kWsSmemLimit && !ws_disabled()) {
     const void* wfn = (const void*)gemm_ws_kernel;
@@ -638,6 +660,13 @@ int launch_gemm_tc(const char* name, const float* A, int64_t lda, const float* B
         error_word, F, ldf, stride_f, raw_stages, b_map, use_map, f_map, use_f_map);
     note_launches();
     return launch_status(name);
+  }
+  if (K > kWsPartK) {  // in parts that accumulate, as the warp-specialised form adds them
+    const int status = launch_gemm_tc(name, A, lda, B, ldb, C, ldc, M, kWsPartK, J, batch, stride_b, stride_c, accumulate,
+                                      error_word, F, ldf, stride_f, stream);
+    if (status) return status;
+    return launch_gemm_tc(name, A + kWsPartK, lda, B + kWsPartK * ldb, ldb, C, ldc, M, K - kWsPartK, J, batch, stride_b,
+                          stride_c, 1, error_word, nullptr, 0, 0, stream);
   }
   const void* fn = (const void*)gemm_tc_kernel;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

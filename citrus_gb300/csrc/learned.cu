@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(kCvThreads) conv_tc_kernel(const ConvArgs a, i
       uint8_t* sb = sa_lo + a_bytes;
       // the stage's previous MMAs must be done before its operands are overwritten
       if (st == 0 ? pending0 : pending1) {
-        const bool ok = mbar_wait(smem_u32(&mbar[st]), st == 0 ? phase0 : phase1, global_timer_ns());
+        const bool ok = mbar_wait(smem_u32(&mbar[st]), st == 0 ? phase0 : phase1);
         if (st == 0) { phase0 ^= 1u; pending0 = false; } else { phase1 ^= 1u; pending1 = false; }
         if (!ok) abort_flag = 1;
       }
@@ -432,12 +432,12 @@ __global__ void __launch_bounds__(kCvThreads) conv_tc_kernel(const ConvArgs a, i
     }
     // every MMA of the tile done (both stages drained)
     if (pending0) {
-      if (!mbar_wait(smem_u32(&mbar[0]), phase0, global_timer_ns())) abort_flag = 1;
+      if (!mbar_wait(smem_u32(&mbar[0]), phase0)) abort_flag = 1;
       phase0 ^= 1u;
       pending0 = false;
     }
     if (pending1) {
-      if (!mbar_wait(smem_u32(&mbar[1]), phase1, global_timer_ns())) abort_flag = 1;
+      if (!mbar_wait(smem_u32(&mbar[1]), phase1)) abort_flag = 1;
       phase1 ^= 1u;
       pending1 = false;
     }
@@ -486,8 +486,8 @@ __global__ void __launch_bounds__(kCvThreads) conv_tc_kernel(const ConvArgs a, i
   }
   if (failed && tid == 0 && error_word != nullptr) atomicExch(error_word, 1u);
   // leave only after the tensor cores are done with this CTA's shared memory and tensor memory
-  if (pending0) mbar_wait(smem_u32(&mbar[0]), phase0, global_timer_ns());
-  if (pending1) mbar_wait(smem_u32(&mbar[1]), phase1, global_timer_ns());
+  if (pending0) mbar_wait(smem_u32(&mbar[0]), phase0);
+  if (pending1) mbar_wait(smem_u32(&mbar[1]), phase1);
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0)
