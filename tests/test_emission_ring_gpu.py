@@ -13,6 +13,7 @@ pytestmark = pytest.mark.gpu
 # points of a block 11 cm apart, which 401 nodes (of 0.005) spread over about 26 nodes
 @pytest.mark.parametrize("groups, q, traced, signal, K", [
     (1, 1, True, True, 255), (2, 2, False, True, 256), (4, 1, True, False, 257), (5, 2, True, True, 300),
+    (3, 1, True, False, 260), (6, 1, True, True, 260), (7, 2, True, True, 260), (12, 1, True, False, 260),
     (8, 1, True, True, 513), (16, 1, True, True, 260), (16, 2, False, False, 30)])
 @pytest.mark.parametrize("num_eta", [2, 101, 401, 2001])
 def test_ring_equals_group_lanes(cuda_device, monkeypatch, groups, q, traced, signal, K, num_eta):
