@@ -354,7 +354,7 @@ __device__ __forceinline__ void ray_walk(const Box& b, const Setup<float>& s, co
     const bool last = dt >= remaining;
     if (last) dt = fmaxf(remaining, 0.f);
     const float* vox = vol + ((int64_t)(iy * b.n[0] + ix) * b.n[2] + iz) * nC;
-    if (kC == 8 || kC == 4) {
+    if (kC > 0 && kC % 4 == 0) {
 #pragma unroll
       for (int c = 0; c < (kC > 0 ? kC : 1); c += 4) {
         const float4 w = __ldg(reinterpret_cast<const float4*>(vox + c));
@@ -998,6 +998,24 @@ int check_common(const float* vol, int64_t C, const double* box, const int64_t* 
   }                                                                                       \
   note_launches();
 
+// The oblique projection carries the groups of an image: a number of channels known at compile time keeps their sums in
+// registers instead of local memory (an image of 44 x 54 x 38 points, 5 groups and 61 x 83 pixels: 371 -> 227 us)
+#define CITRUS_OBLIQUE_DISPATCH(C, KERNEL, GRID, STREAM, ...)                            \
+  switch (C) {                                                                            \
+    case 1: KERNEL<1><<<GRID, kThreads, 0, STREAM>>>(__VA_ARGS__); break;                \
+    case 2: KERNEL<2><<<GRID, kThreads, 0, STREAM>>>(__VA_ARGS__); break;                \
+    case 3: KERNEL<3><<<GRID, kThreads, 0, STREAM>>>(__VA_ARGS__); break;                \
+    case 4: KERNEL<4><<<GRID, kThreads, 0, STREAM>>>(__VA_ARGS__); break;                \
+    case 5: KERNEL<5><<<GRID, kThreads, 0, STREAM>>>(__VA_ARGS__); break;                \
+    case 6: KERNEL<6><<<GRID, kThreads, 0, STREAM>>>(__VA_ARGS__); break;                \
+    case 7: KERNEL<7><<<GRID, kThreads, 0, STREAM>>>(__VA_ARGS__); break;                \
+    case 8: KERNEL<8><<<GRID, kThreads, 0, STREAM>>>(__VA_ARGS__); break;                \
+    case 12: KERNEL<12><<<GRID, kThreads, 0, STREAM>>>(__VA_ARGS__); break;              \
+    case 16: KERNEL<16><<<GRID, kThreads, 0, STREAM>>>(__VA_ARGS__); break;              \
+    default: KERNEL<0><<<GRID, kThreads, 0, STREAM>>>(__VA_ARGS__); break;               \
+  }                                                                                       \
+  note_launches();
+
 }  // namespace
 }  // namespace citrus
 
@@ -1209,7 +1227,9 @@ extern "C" int citrus_oblique_project_scratch(const float* field, int64_t channe
     note_launches();
   }
   dim3 grid((unsigned)cdiv(num_pixels, kThreads), (unsigned)num_directions);
-  CITRUS_CHANNEL_DISPATCH(C, oblique_kernel, grid, as_stream(stream), b, field, C, field_stride, omegas, pixels,
+  // float4 loads of multiples of four channels need every direction's field aligned (the field itself is checked above)
+  const int known = C % 4 == 0 && field_stride % 4 != 0 ? 0 : C;
+  CITRUS_OBLIQUE_DISPATCH(known, oblique_kernel, grid, as_stream(stream), b, field, C, field_stride, omegas, pixels,
                           num_pixels, center[0], center[1], center[2], half, out, os_k, os_c, os_r, os_col,
                           num_cols, dcs, dps)
   return launch_status("citrus_oblique_project");
