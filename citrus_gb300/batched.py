@@ -117,9 +117,11 @@ def _launch_views(solver: ScatterSolver, states: Sequence[CitrusState], fields: 
         fused = warm and N_sh <= 64 and all(f.means is not None for f in firsts)
         T_all = None
         if warm:  # the scattering moments of every view, formed before any chunk overwrites an accumulator
-            T_all = torch.zeros(B, N_sh, J, device=device)
+            T_all = torch.empty(B, N_sh, J, device=device)
             for j, p in enumerate(previous):
-                if p is not None:
+                if p is None:
+                    T_all[j].zero_()
+                else:
                     kernels.scattering_moments(fields.mu_s_l_coarse, p, "cell_major",
                                                out=T_all[j].view((N_sh,) + shape + (G, 4)))
         moments = torch.empty(B, N_sh, J, device=device) if store_out is None else store_out[b0:b0 + B]
