@@ -12,8 +12,8 @@ Tuned here:
 * ``small_k_gemm``: the small-K product's kernel — the float32 streaming forms against the shared-memory tiled
   kernel at each of its tile heights (``citrus_small_k_gemm_config``) and, in the bf16x3 precision, the tcgen05
   bf16 hi/lo product, timed into a scratch output;
-* ``sweep``: views per persistent sweep launch of the batched step and the form of the sweep threads
-  (``citrus_sweep_persistent_config``), timed on a store of ones of that many views (the sweep's memory traffic
+* ``sweep``: views per sweep launch of the batched step and the form of the sweep (``citrus_sweep_pencils``, above 128
+  groups ``citrus_sweep_persistent_config``), timed on a store of ones of that many views (the sweep's memory traffic
   does not depend on the values; non-zero moments keep the divisions on their usual path), the per-view time
   compared.
 """
