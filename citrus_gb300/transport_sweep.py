@@ -211,9 +211,12 @@ class SweepContext:
 
     def direction_indices(self, start: int, stop: int) -> Tensor:
         """Octant-major reordered indices of the per-octant chunk ``start <= d < stop``: ``o * D8 + d``."""
+        D8 = self.directions_per_octant
+        if start == 0 and stop == D8:  # all of them: one launch instead of four (about 8 us of host time each)
+            return torch.arange(8 * D8, dtype=torch.int64, device=self.device)
         d = torch.arange(start, stop, dtype=torch.int64, device=self.device)
         o = torch.arange(8, dtype=torch.int64, device=self.device)
-        return (o[:, None] * self.directions_per_octant + d[None, :]).reshape(-1)
+        return (o[:, None] * D8 + d[None, :]).reshape(-1)
 
 
 def make_sweep_context(grid: Grid, quadrature: Quadrature, L: int, device) -> SweepContext:
