@@ -289,7 +289,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) tiled_kernel(
 constexpr int kPencilSlots = 5;
 constexpr int kPencilAhead = kPencilSlots - 2;  // a slot is refilled a barrier after the neighbours read its outputs
 constexpr int kPencilThreads = 512;
-constexpr int kPencilFlag = 4;  // the first flag among the sync words: 0 the task counter, 2 the error word
+constexpr int kPencilFlag = 4;  // the first flag among the sync words: 0 the task counter, 1 progress, 2 the error word
+constexpr int kPencilBeat = 512 * kPencilSlots;  // steps between two signs of progress
 
 struct Pencils {
   uint32_t R, C, S, G, Dc, dpb, T;  // grid, groups, directions of an octant and of a task, tile edge
@@ -342,13 +343,20 @@ __device__ __forceinline__ bool next_pencil_task(const Pencils& p, unsigned* syn
   const uint32_t I = (D >= p.tiles_c ? D - p.tiles_c + 1 : 0) + place, J = D - I;
   const uint32_t flag = q * tiles + I * p.tiles_c + J;
   const unsigned* flags = sync + kPencilFlag;
-  const uint64_t t0 = global_timer_ns();
+  // the limit is on the time without progress of any block: upstream tasks may wait in turn, and a task of a long grid
+  // may take longer than any sensible limit
+  uint64_t t0 = global_timer_ns();
+  unsigned seen = ld_acquire_u32(&sync[1]);
   for (int a = 0; a < 2; ++a) {
     if ((a == 0 ? I : J) == 0) continue;
     const unsigned* f = flags + flag - (a == 0 ? p.tiles_c : 1);
     while (ld_acquire_u32(f) == 0u) {
       if (ld_acquire_u32(&sync[2]) != 0u) return false;
-      if (global_timer_ns() - t0 > timeout_ns) {
+      const unsigned now = ld_acquire_u32(&sync[1]);
+      if (now != seen) {
+        seen = now;
+        t0 = global_timer_ns();
+      } else if (global_timer_ns() - t0 > timeout_ns) {
         atomicExch(&sync[2], 1u);
         return false;
       }
@@ -410,6 +418,7 @@ __global__ void __launch_bounds__(kPencilThreads, 2) pencil_kernel(float4* __res
     float m_next = 0.f;
     // Step t runs in slot (t + kPencilAhead) % kPencilSlots; the inflow of a step is in the slot before it
     for (int t0 = -kPencilAhead; t0 < steps; t0 += kPencilSlots) {
+      if (tid == 0 && (uint32_t)(t0 + kPencilAhead) % kPencilBeat == kPencilBeat - kPencilSlots) atomicAdd(&sync[1], 1u);
 #pragma unroll
       for (int q5 = 0; q5 < kPencilSlots; ++q5) {
         constexpr int kA = kPencilAhead, kP = kPencilSlots;
@@ -458,7 +467,10 @@ __global__ void __launch_bounds__(kPencilThreads, 2) pencil_kernel(float4* __res
     }
     if (tid == 0) {  // the last step's barrier put the block's stores before this
       __threadfence();
-      if ((int)blockIdx.x != skip) st_release_u32(sync + kPencilFlag + s_task[3], 1u);
+      if ((int)blockIdx.x != skip) {
+        st_release_u32(sync + kPencilFlag + s_task[3], 1u);
+        atomicAdd(&sync[1], 1u);
+      }
     }
   }
 }

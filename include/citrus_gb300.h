@@ -96,8 +96,8 @@ int citrus_sweep_tiled(float* store, const float* mu_cells, const float* c, cons
  * dirs_per_block directions (1..dc) and views_per_thread views (1 or 2) once the tile's two upstream tiles are done.
  * tile^2 dirs_per_block num_groups is at most 512 threads. sync: sync_words device words, 4 and one per task (tiles x
  * 8 ceil(dc / dirs_per_block) x ceil(views / views_per_thread)), cleared by the call itself; sync[2] != 0 after the
- * launch: a wait ran past timeout_ns and the store is invalid. max_blocks caps the grid (0: as many as fit); skip_block
- * >= 0 is a test hook (that block never reports its tasks as done). */
+ * launch: a wait saw no progress of any block for timeout_ns and the store is invalid. max_blocks caps the grid (0: as
+ * many as fit); skip_block >= 0 is a test hook (that block never reports its tasks as done). */
 int citrus_sweep_pencils(float* store, const float* mu_cells, const float* c, int64_t rows, int64_t cols,
                          int64_t slices, int64_t num_groups, int64_t dc, int64_t views, int64_t tile,
                          int64_t dirs_per_block, int64_t views_per_thread, uint32_t* sync, int64_t sync_words,

@@ -72,3 +72,18 @@ def test_pencil_sweep_rejects_what_it_cannot_take(cuda_device):
             kernels.sweep_pencils(ctx.shape, store, mu, c, **kwargs)
     with pytest.raises(ValueError):
         kernels.sweep_pencils((4, 4, 5), store, mu, c)
+
+
+def test_waiting_tasks_outlast_the_limit_while_others_progress(cuda_device):
+    """The limit is on the time without progress: the last of the tiles waits for all those before it, here some 20 ms
+    with a limit of 5 ms, of which a tile takes a fraction."""
+    ctx = make_sweep_context(Grid((1, 64, 4096), 1.0), product_quadrature(2, 4), 1, cuda_device)
+    N, G = ctx.num_cells, 1
+    gen = torch.Generator().manual_seed(5)
+    store = torch.randn(8, 1, N, 4 * G, generator=gen).to(cuda_device)
+    mu = (torch.rand(N, G, generator=gen) + 0.1).to(cuda_device)
+    expected = store.clone()
+    kernels.sweep_planes(ctx.flat_index, expected, mu, ctx.c.contiguous())
+    sync = kernels.sweep_pencils(ctx.shape, store, mu, ctx.c.contiguous(), tile=2, timeout_ns=5_000_000)
+    assert int(sync[2]) == 0
+    assert torch.equal(store, expected)
