@@ -13,8 +13,9 @@
 // holds some, and the encoder reads it twice (maximum, then values). Blocks therefore take a run of cells times a tile
 // of groups, with the threads running over the groups first where those are the nearer neighbours in memory, and turn
 // the tile in shared memory for the side whose cells are contiguous. One block per (group, moment) walking its
-// cells at the stride of a whole cell used a line per 4 bytes: at 64^3 cells, 8 groups, 36 moments (1.2 GB) storing an
-// accumulator took 1.15 ms and bringing it back 2.98 ms; now the two with their host calls take 0.83 ms.
+// cells at the stride of a whole cell uses a line per 4 bytes: at 64^3 cells, 8 groups, 36 moments (1.2 GB) storing an
+// accumulator took 1.15 ms so and bringing it back 2.98 ms; by tiles the two with their host calls take 0.83 ms. A small
+// accumulator, or one whose cells are adjacent, is encoded that way all the same (encode_by_lines).
 #include <cuda_fp16.h>
 
 #include "common.cuh"
@@ -131,6 +132,99 @@ inline int state_tile_groups(int64_t groups, int64_t s_g, int64_t s_x) {
   return s_x <= s_g ? 1 : (int)(groups < kTileGroups ? groups : kTileGroups);
 }
 
+// The whole encoding of a (group, moment) in one block, which walks its cells twice with kLineLoads of them in flight per
+// thread; the second time they come from L2.
+constexpr int kLineLoads = 8;
+
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads) state_encode_lines_kernel(const float* __restrict__ acc, int N,
+                                                                      int64_t cells, int64_t s_g, int64_t s_n,
+                                                                      int64_t s_x, __half* __restrict__ data,
+                                                                      float* __restrict__ scale) {
+  __shared__ unsigned s_max[kThreads / 32];
+  const int gn = blockIdx.x;  // g * N + n
+  const int g = gn / N, n = gn - g * N;
+  const float* src = acc + g * s_g + n * s_n;
+  unsigned m = 0u;
+  for (int64_t x0 = threadIdx.x; x0 < cells; x0 += kLineLoads * kThreads) {
+    unsigned v[kLineLoads];
+#pragma unroll
+    for (int u = 0; u < kLineLoads; ++u) {
+      const int64_t x = x0 + u * kThreads;
+      v[u] = x < cells ? __float_as_uint(__ldg(src + x * s_x)) & 0x7fffffffu : 0u;
+    }
+#pragma unroll
+    for (int u = 0; u < kLineLoads; ++u) m = max(m, v[u]);
+  }
+  m = __reduce_max_sync(0xffffffffu, m);
+  if (threadIdx.x % 32 == 0) s_max[threadIdx.x / 32] = m;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < kThreads / 32; ++w) m = max(m, s_max[w]);
+  const float maximum = __uint_as_float(m);
+  const float sc = maximum > 0.f ? __fdiv_rn(maximum, kFloat16Target) : 1.f;
+  if (threadIdx.x == 0) scale[gn] = sc;
+  __half* dst = data + (int64_t)gn * cells;
+  for (int64_t x0 = threadIdx.x; x0 < cells; x0 += kLineLoads * kThreads) {
+    float v[kLineLoads];
+#pragma unroll
+    for (int u = 0; u < kLineLoads; ++u) {
+      const int64_t x = x0 + u * kThreads;
+      v[u] = x < cells ? __ldg(src + x * s_x) : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < kLineLoads; ++u) {
+      const int64_t x = x0 + u * kThreads;
+      if (x < cells) dst[x] = __float2half_rn(__fdiv_rn(v[u], sc));
+    }
+  }
+}
+
+int encode_lines(const float* acc, int64_t groups, int64_t moments, int64_t cells, int64_t s_g, int64_t s_n, int64_t s_x,
+                 uint16_t* data, float* scale, cudaStream_t s) {
+  const unsigned blocks = (unsigned)(groups * moments);
+  __half* out = reinterpret_cast<__half*>(data);
+  if (cells > 2048) {
+    state_encode_lines_kernel<1024><<<blocks, 1024, 0, s>>>(acc, (int)moments, cells, s_g, s_n, s_x, out, scale);
+  } else {
+    state_encode_lines_kernel<256><<<blocks, 256, 0, s>>>(acc, (int)moments, cells, s_g, s_n, s_x, out, scale);
+  }
+  note_launches();
+  return launch_status("citrus_state_encode");
+}
+
+int encode_tiles(const float* acc, int64_t groups, int64_t moments, int64_t cells, int64_t s_g, int64_t s_n, int64_t s_x,
+                 uint16_t* data, float* scale, cudaStream_t s) {
+  const int G = (int)groups, N = (int)moments, tile = state_tile_groups(groups, s_g, s_x);
+  const int64_t gtiles = cdiv(groups, tile), count = groups * moments;
+  const int64_t per_block = (int64_t)kStateThreads / tile * kMaxCells;
+  CITRUS_REQUIRE(moments * gtiles * cdiv(cells, kTileCells < per_block ? kTileCells : per_block) < (1ll << 31),
+                 "citrus_state_encode: the accumulator exceeds the launch grid");
+  cudaError_t e = cudaMemsetAsync(scale, 0, count * sizeof(float), s);
+  if (e != cudaSuccess) return set_error(CITRUS_ECUDA, "citrus_state_encode: %s", cudaGetErrorString(e));
+  state_max_kernel<<<(unsigned)(moments * gtiles * cdiv(cells, per_block)), kStateThreads, 0, s>>>(
+      acc, G, N, tile, per_block, cells, s_g, s_n, s_x, reinterpret_cast<unsigned*>(scale));
+  state_scale_kernel<<<(unsigned)cdiv(count, kStateThreads), kStateThreads, 0, s>>>(scale, count);
+  state_encode_kernel<<<(unsigned)(moments * gtiles * cdiv(cells, kTileCells)), kStateThreads, 0, s>>>(
+      acc, G, N, tile, cells, s_g, s_n, s_x, scale, reinterpret_cast<__half*>(data));
+  note_launches(3);
+  return launch_status("citrus_state_encode");
+}
+
+// Whether one launch (lines) encodes the accumulator, or the tiles' memset and three launches, which read whole lines and
+// spread a (group, moment) over many blocks but cost 10 us however small it is. us, lines / tiles, at 16^3, 32^3 and 64^3 cells:
+//   cells next to one another (or one group): 16 (group, moment)s 4 / 10, 9 / 14, 49 / 47; 4 of them 4 / 10, 9 / 11,
+//     49 / 19; 288 of them 6 / 19, 17 / 94, 171 / 690;
+//   8 groups next to one another, 16 moments: 7 / 12, 39 / 27, 278 / 193; 36 moments 13 / 14, 189 / 66, 2113 / 410.
+// From 20 blocks on adjacent cells are read as fast by lines, below that while a block's walk is short; adjacent groups
+// while the walk is short and the accumulator stays well inside L2 between the uses of a sector (two of them share
+// one, so that enough blocks of two groups lose nothing at any size).
+inline bool encode_by_lines(int64_t groups, int64_t moments, int64_t cells, int64_t s_g, int64_t s_x) {
+  const int64_t count = groups * moments;
+  if (state_tile_groups(groups, s_g, s_x) == 1) return count >= 20 || cells <= 49152;
+  return (groups == 2 && count >= 64) || (groups * cells <= 65536 && 16 * count * cells <= 25'000'000);
+}
+
 // full accumulator element (g, n, k, cell) at g * o_g + n * o_n + k * o_k + cell * o_x: k = 0 the decoded mean, else 0
 __global__ void __launch_bounds__(kStateThreads) state_decode_kernel(const __half* __restrict__ data,
                                                                      const float* __restrict__ scale, int N,
@@ -161,21 +255,8 @@ extern "C" int citrus_state_encode(const float* accumulator, int64_t groups, int
   CITRUS_REQUIRE(groups >= 1 && moments >= 1 && cells >= 1 && groups * moments <= (1 << 30),
                  "citrus_state_encode: bad sizes (groups %lld, moments %lld, cells %lld)", (long long)groups,
                  (long long)moments, (long long)cells);
-  const int G = (int)groups, N = (int)moments, tile = state_tile_groups(groups, s_g, s_x);
-  const int64_t gtiles = cdiv(groups, tile), count = groups * moments;
-  const int64_t per_block = (int64_t)kStateThreads / tile * kMaxCells;
-  CITRUS_REQUIRE(moments * gtiles * cdiv(cells, kTileCells < per_block ? kTileCells : per_block) < (1ll << 31),
-                 "citrus_state_encode: the accumulator exceeds the launch grid");
-  cudaStream_t s = as_stream(stream);
-  cudaError_t e = cudaMemsetAsync(scale, 0, count * sizeof(float), s);
-  if (e != cudaSuccess) return set_error(CITRUS_ECUDA, "citrus_state_encode: %s", cudaGetErrorString(e));
-  state_max_kernel<<<(unsigned)(moments * gtiles * cdiv(cells, per_block)), kStateThreads, 0, s>>>(
-      accumulator, G, N, tile, per_block, cells, s_g, s_n, s_x, reinterpret_cast<unsigned*>(scale));
-  state_scale_kernel<<<(unsigned)cdiv(count, kStateThreads), kStateThreads, 0, s>>>(scale, count);
-  state_encode_kernel<<<(unsigned)(moments * gtiles * cdiv(cells, kTileCells)), kStateThreads, 0, s>>>(
-      accumulator, G, N, tile, cells, s_g, s_n, s_x, scale, reinterpret_cast<__half*>(data));
-  note_launches(3);
-  return launch_status("citrus_state_encode");
+  const auto encode = encode_by_lines(groups, moments, cells, s_g, s_x) ? encode_lines : encode_tiles;
+  return encode(accumulator, groups, moments, cells, s_g, s_n, s_x, data, scale, as_stream(stream));
 }
 
 extern "C" int citrus_state_decode(const uint16_t* data, const float* scale, int64_t groups, int64_t moments,
@@ -185,8 +266,9 @@ extern "C" int citrus_state_decode(const uint16_t* data, const float* scale, int
   CITRUS_REQUIRE(groups >= 1 && moments >= 1 && cells >= 1 && groups * moments <= 65535,
                  "citrus_state_decode: bad sizes (groups %lld, moments %lld, cells %lld)", (long long)groups,
                  (long long)moments, (long long)cells);
-  if (o_k == 1 && o_g % 4 == 0 && o_n % 4 == 0 && o_x % 4 == 0 && ((uintptr_t)accumulator % 16) == 0) {
-    const int tile = state_tile_groups(groups, o_g, o_x);
+  const int tile = state_tile_groups(groups, o_g, o_x);
+  // by tiles of groups; a single group is read and written in order without one (64 moments of 32^3 cells 7 us, 20 in tiles)
+  if (tile > 1 && o_k == 1 && o_g % 4 == 0 && o_n % 4 == 0 && o_x % 4 == 0 && ((uintptr_t)accumulator % 16) == 0) {
     const int64_t blocks = moments * cdiv(groups, tile) * cdiv(cells, kTileCells);
     CITRUS_REQUIRE(blocks < (1ll << 31), "citrus_state_decode: the accumulator exceeds the launch grid");
     state_decode4_kernel<<<(unsigned)blocks, kStateThreads, 0, as_stream(stream)>>>(
