@@ -1,7 +1,8 @@
 // Spherical-harmonic moments of the scattering source, T[g, n, k, x] = sum_g' transfer[g', g, l(n), x] phi[g', n, k, x]
 // (citrus/scatter_solver/angular_quadrature.py:600-677 and kernels/scattering_kernels.py:159-252), summed over the
-// incoming groups in ascending order. One kernel over values of float4 (layouts with the 4 linear-discontinuous moments
-// contiguous, the sweep's cell-major storage) or float (any other strides: the image's cell means, moment-major).
+// incoming groups in ascending order. Two kernels, by blocks of points and one degree (moments_kernel) or by points
+// (moments_point_kernel), over values of float4 (layouts with the 4 linear-discontinuous moments contiguous, the sweep's
+// cell-major storage) or float (any other strides: the image's cell means, moment-major).
 #include "common.cuh"
 
 namespace citrus {
@@ -131,6 +132,72 @@ void launch_moments(const float* transfer, const float* phi, float* out, int GI,
                                                              k_count, ps_g, ps_n, ps_k, ps_x, os_g, os_n, os_k, os_x);
 }
 
+// A thread per (moment, point) with all of its incoming groups in registers, the moments fastest over the blocks, so that the
+// transfer rows of a degree, shared by its 2l + 1 moments, come from L2 after the first.
+constexpr int kPointThreads = 256;
+
+__device__ __forceinline__ int degree_of(int n) {
+  int l = (int)sqrtf((float)n);
+  while ((l + 1) * (l + 1) <= n) ++l;
+  while (l * l > n) --l;
+  return l;
+}
+
+template <int kGI, typename V>
+__global__ void __launch_bounds__(kPointThreads) moments_point_kernel(const float* __restrict__ transfer,
+                                                                      const float* __restrict__ phi,
+                                                                      float* __restrict__ out, int GI, int GO,
+                                                                      int num_legendre, int64_t X, int64_t ps_g,
+                                                                      int64_t ps_n, int64_t ps_k, int64_t ps_x,
+                                                                      int64_t os_g, int64_t os_n, int64_t os_k,
+                                                                      int64_t os_x) {
+  const int64_t x = (int64_t)blockIdx.y * kPointThreads + threadIdx.x;
+  const int n = blockIdx.x, k = blockIdx.z;
+  if (x >= X) return;
+  const float* src = phi + n * ps_n + k * ps_k + x * ps_x;
+  V ph[kGI];
+#pragma unroll
+  for (int gi = 0; gi < kGI; ++gi)
+    if (gi < GI) ph[gi] = *reinterpret_cast<const V*>(src + gi * ps_g);
+  const float* tr = transfer + (int64_t)degree_of(n) * X + x;
+  const int64_t pair = (int64_t)num_legendre * X;
+  float* dst = out + n * os_n + k * os_k + x * os_x;
+  for (int go = 0; go < GO; ++go) {
+    V acc;
+    set_zero(acc);
+#pragma unroll
+    for (int gi = 0; gi < kGI; ++gi)
+      if (gi < GI) add_product(acc, __ldg(tr + (int64_t)(gi * GO + go) * pair), ph[gi]);
+    *reinterpret_cast<V*>(dst + go * os_g) = acc;
+  }
+}
+
+template <int kGI, typename V>
+void launch_moments_point(const float* transfer, const float* phi, float* out, int GI, int GO, int num_legendre,
+                          int num_degrees, int64_t X, int k_count, int64_t ps_g, int64_t ps_n, int64_t ps_k, int64_t ps_x,
+                          int64_t os_g, int64_t os_n, int64_t os_k, int64_t os_x, cudaStream_t s) {
+  dim3 grid((unsigned)(num_degrees * num_degrees), (unsigned)cdiv(X, kPointThreads), (unsigned)k_count);
+  moments_point_kernel<kGI, V><<<grid, kPointThreads, 0, s>>>(transfer, phi, out, GI, GO, num_legendre, X, ps_g, ps_n,
+                                                              ps_k, ps_x, os_g, os_n, os_k, os_x);
+}
+
+// Whether the points' threads form the moments. The blocks above run a degree's moments one after the other with a warp
+// per four outgoing groups: with few groups that is one warp and little to load at a time, and in a small volume most
+// of the SMs wait. The points' threads run all moments at once, but read a point's groups from lines that have left the
+// caches between the groups once phi and T do not fit L2. us, points / blocks, cell-major:
+//   1 group, 16 moments: 32^3 cells 3.8 / 7.5, 64^3 24 / 44; 2 groups, 64 moments: 32^3 25 / 30, 64^3 186 / 208;
+//   3 groups, 36 moments: 20^3 7.0 / 15 (28 MB), 32^3 29 / 24 (113 MB); 4 groups: 16^3 6.9 / 17 (19 MB), 24^3 17 / 20 (64), 32^3
+//   54 / 33 (151); 5 groups: 24^3 19 / 26 (80), 32^3 63 / 52 (189); 8 groups: 16^3 14 / 21 (38), 24^3 60 / 33 (127).
+// With the points adjacent (moment-major) the blocks' tiles pay from 14 MB on, except over so few moments that the
+// transfers are most of what is read (4 moments of 5 groups, 64^3: 123 / 157). bytes: the lines of phi and T that are touched.
+inline bool moments_by_points(int GI, int degrees, int64_t bytes, bool points_adjacent) {
+  if (GI <= 2) return true;
+  if (GI > 8 || (GI > 6 && degrees < 4)) return false;
+  if (degrees == 1) return true;
+  if (points_adjacent) return bytes <= 14'000'000 || (degrees == 2 && GI != 4);
+  return bytes <= (GI == 4 ? 60'000'000 : GI == 5 ? 170'000'000 : GI <= 6 ? 100'000'000 : 40'000'000);
+}
+
 }  // namespace
 }  // namespace citrus
 
@@ -159,6 +226,29 @@ extern "C" int citrus_scattering_moments(const float* transfer, const float* phi
   CITRUS_REQUIRE(num_points <= 65535ll * 256, "citrus_scattering_moments: %lld points exceed the grid",
                  (long long)num_points);
   const int GI = (int)g_in, GO = (int)g_out, NL = (int)num_legendre;
+  const bool points_adjacent = !vec && ps_x == 1;
+  const int64_t bytes = 4 * (g_in + g_out) * num_moments * num_points * (points_adjacent ? k_count : 4);
+#define CITRUS_MOMENTS_POINT(KGI)                                                                                     \
+  if (vec)                                                                                                           \
+    launch_moments_point<KGI, float4>(transfer, phi, out, GI, GO, NL, L + 1, num_points, 1, ps_g, ps_n, 0, ps_x, os_g, \
+                                      os_n, 0, os_x, s);                                                             \
+  else                                                                                                               \
+    launch_moments_point<KGI, float>(transfer, phi, out, GI, GO, NL, L + 1, num_points, (int)k_count, ps_g, ps_n,    \
+                                     ps_k, ps_x, os_g, os_n, os_k, os_x, s);
+  if (moments_by_points(GI, L + 1, bytes, points_adjacent)) {
+    if (GI == 1) {
+      CITRUS_MOMENTS_POINT(1)
+    } else if (GI == 2) {
+      CITRUS_MOMENTS_POINT(2)
+    } else if (GI <= 4) {
+      CITRUS_MOMENTS_POINT(4)
+    } else {
+      CITRUS_MOMENTS_POINT(8)
+    }
+    note_launches();
+    return launch_status("citrus_scattering_moments");
+  }
+#undef CITRUS_MOMENTS_POINT
   // the incoming groups a thread's transfers are unrolled for: four outgoing groups each up to 16, two above, which
   // keeps the 64 transfers in registers
 #define CITRUS_MOMENTS_LAUNCH(KGI, KGT)                                                                              \
