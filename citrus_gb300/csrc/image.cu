@@ -210,63 +210,75 @@ __global__ void weighted_group_sum_kernel(const float* __restrict__ img, const f
   out[((int64_t)k * R + r) * C + c] = acc;
 }
 
-// Sums over directions: a thread takes one pixel of one block of kSumBlock directions, and the first of a pixel's
-// threads adds the blocks' sums to the accumulator in order. The rounding is that of one call per block, so a sum over
-// all 512 directions of an image is as accurate as eight over 64, and a small panel (64 x 64 pixels are 16 blocks of
-// 256 threads) has a thread per block of directions instead of one walk down all of them: a full image of 5 groups 332 -> 59 us.
-constexpr int kSumBlock = 64, kSumPixels = 64, kSumSlices = 8;
+// Sums over directions. Up to kSumBlock of them a thread takes one pixel and walks them. Above, a thread takes one pixel
+// of one block of kSumBlock directions, and the first of a pixel's threads adds the blocks' sums to the accumulator in order:
+// the rounding is that of one call per block, so a sum over all 512 directions of an image is as accurate as eight over
+// 64, and a small panel (64 x 64 pixels are 16 blocks of 256 threads) has a thread per block of directions instead of one walk
+// down all of them: a full image of 5 groups 332 -> 59 us. With one block of directions the shared sums and barriers
+// only cost: 64 directions of 384 x 512 pixels 7.9 us, 4.7 without.
+constexpr int kSumBlock = 64, kSumPixels = 64, kSumSlices = 8, kSumThreads = 256;
 
-template <typename Term>
-__device__ __forceinline__ void sum_blocks(int K, bool inside, float* __restrict__ acc, int accumulate, Term term) {
-  __shared__ float s_part[kSumSlices][kSumPixels];
-  const int slices = blockDim.y;
-  float total = inside && accumulate && threadIdx.y == 0 ? *acc : 0.f;
-  bool have = accumulate != 0;
-  for (int k0 = 0; k0 < K; k0 += slices * kSumBlock) {
-    const int first = k0 + threadIdx.y * kSumBlock, last = min(first + kSumBlock, K);
+template <bool kBlocks, typename Term>
+__device__ __forceinline__ void sum_directions(int K, bool inside, float* __restrict__ acc, int accumulate, Term term) {
+  if constexpr (!kBlocks) {
+    if (!inside) return;
     float s = 0.f;
-    if (inside) {
+    for (int k = 0; k < K; ++k) term(k, s);
+    *acc = accumulate ? *acc + s : s;
+  } else {
+    __shared__ float s_part[kSumSlices][kSumPixels];
+    const int slices = blockDim.y;
+    float total = inside && accumulate && threadIdx.y == 0 ? *acc : 0.f;
+    bool have = accumulate != 0;
+    for (int k0 = 0; k0 < K; k0 += slices * kSumBlock) {
+      const int first = k0 + threadIdx.y * kSumBlock, last = min(first + kSumBlock, K);
+      float s = 0.f;
+      if (inside) {
 #pragma unroll 8
-      for (int k = first; k < last; ++k) term(k, s);
-    }
-    s_part[threadIdx.y][threadIdx.x] = s;
-    __syncthreads();
-    if (threadIdx.y == 0)
-      for (int j = 0; j < slices && k0 + j * kSumBlock < K; ++j) {
-        total = have ? total + s_part[j][threadIdx.x] : s_part[j][threadIdx.x];
-        have = true;
+        for (int k = first; k < last; ++k) term(k, s);
       }
-    __syncthreads();
+      s_part[threadIdx.y][threadIdx.x] = s;
+      __syncthreads();
+      if (threadIdx.y == 0)
+        for (int j = 0; j < slices && k0 + j * kSumBlock < K; ++j) {
+          total = have ? total + s_part[j][threadIdx.x] : s_part[j][threadIdx.x];
+          have = true;
+        }
+      __syncthreads();
+    }
+    if (inside && threadIdx.y == 0) *acc = total;
   }
-  if (inside && threadIdx.y == 0) *acc = total;
 }
 
+// the block of a sum over K directions, and its pixels
 inline dim3 sum_threads(int64_t K) {
-  const int64_t blocks = cdiv(K, kSumBlock);
-  return dim3(kSumPixels, (unsigned)(blocks < 1 ? 1 : blocks < kSumSlices ? blocks : kSumSlices));
+  if (K <= kSumBlock) return dim3(kSumThreads);
+  return dim3(kSumPixels, (unsigned)(cdiv(K, kSumBlock) < kSumSlices ? cdiv(K, kSumBlock) : kSumSlices));
 }
 
 // acc[p] (+)= sum_k img[k, p]
+template <bool kBlocks>
 __global__ void sum_directions_kernel(const float* __restrict__ img, int K, int64_t P, int64_t stride_k,
                                       float* __restrict__ acc, int accumulate) {
-  const int64_t p = (int64_t)blockIdx.x * kSumPixels + threadIdx.x;
-  sum_blocks(K, p < P, acc + p, accumulate, [&](int k, float& s) { s += img[k * stride_k + p]; });
+  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  sum_directions<kBlocks>(K, p < P, acc + p, accumulate, [&](int k, float& s) { s += img[k * stride_k + p]; });
 }
 
 // acc[g, r, c] (+)= sum_k W[k, g, r | 0, c | 0] img[k, g, r, c], images through strides (the accumulation of the full
 // images, DirectionSetContext.accumulate, scatter_image.py:340-371)
+template <bool kBlocks>
 __global__ void weighted_direction_sum_kernel(const float* __restrict__ img, int K, int G, int R, int C, int64_t is_k,
                                               int64_t is_g, int64_t is_r, int64_t is_c, const float* __restrict__ W,
                                               int w_rows, int w_cols, float* __restrict__ acc, int accumulate) {
-  const int64_t t = (int64_t)blockIdx.x * kSumPixels + threadIdx.x;
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int g = (int)(t / ((int64_t)R * C));
   const int64_t rc = t - (int64_t)g * R * C;
   const int r = (int)(rc / C), c = (int)(rc - (int64_t)r * C);
   const int64_t w_k = (int64_t)G * w_rows * w_cols;
   const float* w = W + ((int64_t)g * w_rows + (w_rows > 1 ? r : 0)) * w_cols + (w_cols > 1 ? c : 0);
   const float* src = img + g * is_g + r * is_r + c * is_c;
-  sum_blocks(K, t < (int64_t)G * R * C, acc + t, accumulate,
-             [&](int k, float& s) { s = fmaf(w[k * w_k], src[k * is_k], s); });
+  sum_directions<kBlocks>(K, t < (int64_t)G * R * C, acc + t, accumulate,
+                          [&](int k, float& s) { s = fmaf(w[k * w_k], src[k * is_k], s); });
 }
 
 }  // namespace
@@ -284,7 +296,9 @@ extern "C" int citrus_weighted_direction_sum(const float* image, int64_t num_dir
                  "citrus_weighted_direction_sum: weights must be [K, G, rows | 1, cols | 1]");
   const int64_t total = groups * rows * cols;
   if (total == 0) return CITRUS_OK;
-  weighted_direction_sum_kernel<<<(unsigned)cdiv(total, kSumPixels), sum_threads(num_directions), 0, as_stream(stream)>>>(
+  const dim3 threads = sum_threads(num_directions);
+  auto kernel = num_directions > kSumBlock ? weighted_direction_sum_kernel<true> : weighted_direction_sum_kernel<false>;
+  kernel<<<(unsigned)cdiv(total, threads.x), threads, 0, as_stream(stream)>>>(
       image, (int)num_directions, (int)groups, (int)rows, (int)cols, is_k, is_g, is_r, is_c, weights,
       (int)weight_rows, (int)weight_cols, accumulator, accumulate);
   note_launches();
@@ -356,8 +370,10 @@ extern "C" int citrus_sum_directions(const float* image, int64_t num_directions,
                                      float* accumulator, int32_t accumulate, void* stream) {
   CITRUS_REQUIRE(image && accumulator && num_directions >= 0 && pixels >= 0, "citrus_sum_directions: bad arguments");
   if (pixels == 0) return CITRUS_OK;
-  sum_directions_kernel<<<(unsigned)cdiv(pixels, kSumPixels), sum_threads(num_directions), 0, as_stream(stream)>>>(image, (int)num_directions, pixels,
-                                                                                   stride_k, accumulator, accumulate);
+  const dim3 threads = sum_threads(num_directions);
+  auto kernel = num_directions > kSumBlock ? sum_directions_kernel<true> : sum_directions_kernel<false>;
+  kernel<<<(unsigned)cdiv(pixels, threads.x), threads, 0, as_stream(stream)>>>(image, (int)num_directions, pixels, stride_k,
+                                                                               accumulator, accumulate);
   note_launches();
   return launch_status("citrus_sum_directions");
 }
