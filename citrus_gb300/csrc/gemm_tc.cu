@@ -206,8 +206,9 @@ __global__ void __launch_bounds__(kTcThreads) gemm_tc_kernel(const float* __rest
 //   * MMA issuer (one thread of warp 20): 3 x (K / 16) tcgen05.mma per tile into one of two float32 accumulators in
 //     tensor memory, committed to the operand stage (freed once read) and to the accumulator (full);
 //   * epilogue (warps 0 to 15): warp w reads accumulator lanes 32 (w % 4) .. + 31 (columns of C) and every fourth
-//     16 of its rows, and writes (or adds to) C, so that the stores of one tile overlap the loads, splits and MMAs
-//     of the next; the rows of C that it adds to are loaded before it waits for the accumulator; the means come from
+//     16 of its rows (with fewer than 64 rows the warps past them leave: waiting with the others they take issue slots
+//     of the converters, 3 M columns of 4 x 16 149 us, 127 without them), and writes (or adds to) C, so that the stores
+//     of one tile overlap the loads, splits and MMAs of the next; the rows of C that it adds to are loaded before it waits for the accumulator; the means come from
 //     their own two-stage ring (one tensor copy of [M][32] per tile).
 //
 // An inner dimension above 64 goes through the rings in two parts of at most 64 rows, each with an accumulator of its
@@ -310,6 +311,8 @@ __global__ void __launch_bounds__(kWsThreads, 1) gemm_ws_kernel(const float* __r
         *reinterpret_cast<uint4*>(a_hi + off) = hi;
         *reinterpret_cast<uint4*>(a_lo + off) = lo;
       }
+  const int n_t = ((M + 15) / 16) * 16;
+  const int epilogue_warps = min(n_t / 4, kWsEpilogueWarps);  // four for each 16 rows of C; the others go to the end
   if (tid == 0) {
     abort_flag = 0;
     for (int i = 0; i < raw_stages; ++i) {
@@ -322,16 +325,15 @@ __global__ void __launch_bounds__(kWsThreads, 1) gemm_ws_kernel(const float* __r
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(acc_full + i), 1);
-      mbar_init(smem_u32(acc_empty + i), 32 * kWsEpilogueWarps);
+      mbar_init(smem_u32(acc_empty + i), 32 * epilogue_warps);
     }
     mbar_init(smem_u32(mma_done), 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(f_full + i), 1);
-      mbar_init(smem_u32(f_empty + i), 32 * kWsEpilogueWarps);
+      mbar_init(smem_u32(f_empty + i), 32 * epilogue_warps);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  const int n_t = ((M + 15) / 16) * 16;
   const uint32_t acc_cols = n_t <= 64 ? 64u : 128u;  // one accumulator; two per part are allocated
   const uint32_t idesc = idesc_bf16(n_t);
   if (warp == 0) {
@@ -465,7 +467,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) gemm_ws_kernel(const float* __r
       tc_commit(smem_u32(mma_done));  // tracks every MMA issued above
       if (!mbar_wait(smem_u32(mma_done), 0u)) fail();
     }
-  } else {  // epilogue warps
+  } else if (warp < epilogue_warps) {
     const int quarter = warp % 4, m_first = warp / 4 * 16;
     for (int64_t i = 0; i < my_tiles && !abort_flag; ++i) {
       const int ac = (int)(i & 1);
@@ -504,10 +506,15 @@ __global__ void __launch_bounds__(kWsThreads, 1) gemm_ws_kernel(const float* __r
           for (int q = 0; q < 16; ++q) prev[q] = 0.f;
           if (add && col < J) {
             const int fc = (quarter * 32 + lane) >> 2;  // the tile's column / 4
+            if (f_tma) {  // two bodies: a pointer to either is a generic one, whose loads are no shared-memory loads
 #pragma unroll
-            for (int q = 0; q < 16; ++q)
-              if (q < rows)
-                prev[q] = f_tma ? fst[(m0 + q) * 32 + fc] : __ldg(Fz + (int64_t)(m0 + q) * ldf + (col >> 2));
+              for (int q = 0; q < 16; ++q)
+                if (q < rows) prev[q] = fst[(m0 + q) * 32 + fc];
+            } else {
+#pragma unroll
+              for (int q = 0; q < 16; ++q)
+                if (q < rows) prev[q] = __ldg(Fz + (int64_t)(m0 + q) * ldf + (col >> 2));
+            }
           }
         }
         for (int part = 0; part < parts; ++part) {
