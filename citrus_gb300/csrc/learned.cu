@@ -245,6 +245,98 @@ __global__ void __launch_bounds__(kThreads * kSplit) conv_kernel(const ConvArgs 
   }
 }
 
+// The convolution by bricks, for few output channels: a CTA takes a 4 x 8 x 8 brick of voxels x 16 output channels, a thread
+// one voxel; per chunk of kCiT input channels the haloed input brick and the chunk's weights (tap-major, the 16 output
+// channels contiguous for float4 broadcasts) are staged in shared memory. The sums run in the tiles' order, bit for bit.
+constexpr int kCiT = 4;  // input channels per staging step
+
+template <int kK>
+__global__ void __launch_bounds__(kConvThreads) conv_brick_kernel(const ConvArgs a) {
+  constexpr int kH = kK / 2;
+  constexpr int SZ = kTZ + 2 * kH, SY = kTY + 2 * kH, SX = kTX + 2 * kH, S3 = SZ * SY * SX;
+  constexpr int K3 = kK * kK * kK;
+  __shared__ float s_in[kCiT * S3];
+  __shared__ __align__(16) float s_w[kCiT * K3 * kCoT];
+
+  const int tid = threadIdx.x;
+  const int ntx = (a.W + kTX - 1) / kTX, nty = (a.H + kTY - 1) / kTY;
+  const int tile = blockIdx.x;
+  const int x0 = (tile % ntx) * kTX, y0 = ((tile / ntx) % nty) * kTY, z0 = (tile / (ntx * nty)) * kTZ;
+  const int co0 = blockIdx.y * kCoT, b = blockIdx.z;
+  const int lx = tid % kTX, ly = (tid / kTX) % kTY, lz = tid / (kTX * kTY);
+  const int O = a.oa + a.ob, Ci = a.ca + a.cb;
+  const int64_t V = (int64_t)a.D * a.H * a.W;
+  const int Dc = a.D >> 1, Hc = a.H >> 1, Wc = a.W >> 1;
+
+  float acc[kCoT];
+#pragma unroll
+  for (int j = 0; j < kCoT; ++j) acc[j] = (a.bias != nullptr && co0 + j < O) ? a.bias[co0 + j] : 0.f;
+
+  for (int ci0 = 0; ci0 < Ci; ci0 += kCiT) {
+    __syncthreads();
+    for (int e = tid; e < kCiT * S3; e += kConvThreads) {
+      const int c = e / S3, r = e % S3;
+      const int gz = z0 + r / (SY * SX) - kH, gy = y0 + (r / SX) % SY - kH, gx = x0 + r % SX - kH;
+      const int ci = ci0 + c;
+      float v = 0.f;
+      if (ci < Ci && gz >= 0 && gz < a.D && gy >= 0 && gy < a.H && gx >= 0 && gx < a.W) {
+        if (ci < a.ca) {
+          v = __ldg(a.in_a + ((int64_t)b * a.ca + ci) * V + ((int64_t)gz * a.H + gy) * a.W + gx);
+        } else if (a.b_up) {
+          v = __ldg(a.in_b + (((int64_t)b * a.cb + (ci - a.ca)) * Dc + (gz >> 1)) * Hc * Wc + (int64_t)(gy >> 1) * Wc +
+                    (gx >> 1));
+        } else {
+          v = __ldg(a.in_b + ((int64_t)b * a.cb + (ci - a.ca)) * V + ((int64_t)gz * a.H + gy) * a.W + gx);
+        }
+      }
+      s_in[e] = v;
+    }
+    for (int e = tid; e < kCiT * K3 * kCoT; e += kConvThreads) {
+      const int j = e % kCoT, t = (e / kCoT) % K3, c = e / (kCoT * K3);
+      const int o = co0 + j, i = ci0 + c;
+      s_w[e] = (o < O && i < Ci) ? __uint_as_float((uint32_t)a.w[a.w_base + o * a.w_o + i * a.w_i + t * a.w_t] << 16) : 0.f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < kCiT; ++c) {
+#pragma unroll
+      for (int tz = 0; tz < kK; ++tz)
+#pragma unroll
+        for (int ty = 0; ty < kK; ++ty)
+#pragma unroll
+          for (int tx = 0; tx < kK; ++tx) {
+            const float v = s_in[c * S3 + ((lz + tz) * SY + (ly + ty)) * SX + lx + tx];
+            const float4* w4 = reinterpret_cast<const float4*>(s_w + (c * K3 + (tz * kK + ty) * kK + tx) * kCoT);
+#pragma unroll
+            for (int q = 0; q < kCoT / 4; ++q) {
+              const float4 wq = w4[q];
+              acc[4 * q + 0] = fmaf(wq.x, v, acc[4 * q + 0]);
+              acc[4 * q + 1] = fmaf(wq.y, v, acc[4 * q + 1]);
+              acc[4 * q + 2] = fmaf(wq.z, v, acc[4 * q + 2]);
+              acc[4 * q + 3] = fmaf(wq.w, v, acc[4 * q + 3]);
+            }
+          }
+    }
+  }
+
+  const int x = x0 + lx, y = y0 + ly, z = z0 + lz;
+  if (x >= a.W || y >= a.H || z >= a.D) return;
+  const int64_t vox = ((int64_t)z * a.H + y) * a.W + x;
+#pragma unroll
+  for (int j = 0; j < kCoT; ++j) {
+    const int o = co0 + j;
+    if (o >= O) break;
+    float r = a.relu ? fmaxf(acc[j], 0.f) : acc[j];
+    if (o < a.oa) {
+      const int64_t idx = ((int64_t)b * a.oa + o) * V + vox;
+      if (a.mask_a != nullptr && !(a.mask_a[idx] > 0.f)) r = 0.f;
+      a.out_a[idx] = r;
+    } else {
+      a.out_b[((int64_t)b * a.ob + (o - a.oa)) * V + vox] = r;
+    }
+  }
+}
+
 // The same convolution as an implicit GEMM on the tcgen05 tensor cores: D[voxel, o] = sum_k A[voxel, k] B[o, k] with
 // k = tap C_in + input channel (tap-major, so that a run of k shares one spatial offset and its bounds test). A CTA
 // takes a tile of 128 consecutive voxels (the MMA's M) x n_tile output channels (its N, a multiple of 16 up to 256)
@@ -869,7 +961,6 @@ int launch_conv_tile(const ConvArgs& a, cudaStream_t s) {
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return set_error(CITRUS_ECUDA, "conv3d: %s", cudaGetErrorString(e));
   const int64_t tiles = cdiv(M, TM);
-  CITRUS_REQUIRE((int64_t)(a.ca + a.cb) * (a.oa + a.ob) * kK * kK * kK < (1ll << 31), "conv3d: too many weights");
   CITRUS_REQUIRE(tiles < (1ll << 31), "conv3d: too many voxel tiles");
   dim3 grid((unsigned)tiles, (unsigned)cdiv(a.oa + a.ob, TN));
   conv_kernel<kK, kTM, kThreads, kCI, kSplit><<<grid, kThreads * kSplit, smem, s>>>(a, M);
@@ -877,10 +968,30 @@ int launch_conv_tile(const ConvArgs& a, cudaStream_t s) {
   return CITRUS_OK;
 }
 
+// Whether bricks take the convolution. The tiles hold 32 output channels and pay for all of them, and 16 input channels of a
+// 1^3 kernel; the bricks hold 16 and 4, but keep an SM busy only from some 1.5 of them on. us, bricks / tiles:
+//   3^3, 16 -> 16 channels: 32^3 (128 bricks) 52 / 47, 48 x 48 x 32 (288) 57 / 61, 64^3 151 / 192, 96^3 472 / 614; 3 -> 16 channels: 32^3
+//   11 / 12, 96^3 119 / 205; 32 -> 16: 96^3 938 / 1151; 32 -> 24: 64^3 571 / 358;
+//   1^3, 96^3: 1 -> 1 19 / 56, 8 -> 8 42 / 74, 4 -> 32 67 / 73, 16 -> 16 95 / 81, 32 -> 1 156 / 94; 8 -> 8 at 16^3 4.9 / 4.0.
+// The weights of a tile are indexed in 32 bits; more of them go by bricks too.
+inline bool conv_by_bricks(const ConvArgs& a, int kernel_size) {
+  const int64_t O = a.oa + a.ob, Ci = a.ca + a.cb;
+  if (Ci * O * kernel_size * kernel_size * kernel_size >= (1ll << 31)) return true;
+  const int64_t bricks = a.B * cdiv(a.W, kTX) * cdiv(a.H, kTY) * cdiv(a.D, kTZ);
+  if (kernel_size == 1) return Ci <= 4 || (O <= 16 && Ci <= 8 && bricks >= 228);
+  return O <= 16 && Ci > 1 && bricks >= (Ci <= 4 ? 128 : 228);
+}
+
 template <int kK>
 int launch_conv_simt_k(const ConvArgs& a, cudaStream_t s) {
   constexpr int kCI = kK == 3 ? 1 : 16;  // input channels of a chunk, a tap each for 1^3 kernels
   const int64_t M = (int64_t)a.B * a.D * a.H * a.W, O = a.oa + a.ob;
+  const int64_t bricks = cdiv(a.W, kTX) * cdiv(a.H, kTY) * cdiv(a.D, kTZ);
+  if (conv_by_bricks(a, kK)) {
+    conv_brick_kernel<kK><<<dim3((unsigned)bricks, (unsigned)cdiv(O, kCoT), (unsigned)a.B), kConvThreads, 0, s>>>(a);
+    note_launches();
+    return CITRUS_OK;
+  }
   auto tiles = [&](int tm) { return cdiv(M, tm) * cdiv(O, 32); };
   // a chunk of several channels takes them from one input
   if (a.cb > 0 && a.ca % kCI != 0) return launch_conv_tile<kK, 4, 128, 1, 1>(a, s);
