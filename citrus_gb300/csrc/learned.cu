@@ -8,8 +8,9 @@
 //     2x upsampling fused into the input staging (B is read at half resolution), and an optional ReLU. The same kernel
 //     runs the input gradient of a convolution (the transposed convolution: flipped taps, swapped channel roles,
 //     outputs split back into the A and B parts and the A part masked by its ReLU activation).
-//   * wgrad3_kernel (3^3), wgrad_kernel (1^3): weight gradients as fixed-order reductions over (batch, voxel bricks), split over CTAs into
-//     partial sums that wgrad_reduce_kernel adds in split order (deterministic).
+//   * wgrad3_kernel (3^3), wgrad_kernel (1^3, and 3^3 in small volumes or of few channels): weight gradients as
+//     fixed-order reductions over (batch, voxel bricks), split over CTAs into partial sums that wgrad_reduce_kernel adds
+//     in split order (deterministic).
 //   * pooling (2x average), the upsampling's backward pass, MSE and Adam.
 #include <cuda_bf16.h>
 
@@ -1095,22 +1096,41 @@ extern "C" int citrus_conv3d_backward_input(const float* grad_out, int64_t chann
                                              stream);
 }
 
+namespace citrus {
+namespace {
+// Whether a thread per tap (wgrad_kernel) forms the 3^3 weight gradients. Its blocks hold 8 input channels, not 16, and finish a
+// brick in two thirds of the time, so it is the faster one with at most 8 channels, and while all (block, brick)s are
+// resident at once, two an SM. us, per tap / wgrad3: 8 -> 16 channels 64^3 118 / 168; 16 -> 32 channels 16^3 (64) 23 / 34; 24 -> 32
+// channels 24 x 24 x 16 (216) 34 / 36; 40 -> 64 channels 16^3 (320) 45 / 46; 32 -> 32 channels 32^3 (1024) 101 / 85.
+inline bool wgrad_by_taps(int64_t channels_out, int64_t channels_in, int64_t bricks) {
+  return channels_in <= 8 || cdiv(channels_out, kCoT) * cdiv(channels_in, 8) * bricks <= 2 * (int64_t)num_sms();
+}
+}  // namespace
+}  // namespace citrus
+
 extern "C" int64_t citrus_conv3d_weight_grad_splits(int64_t channels_out, int64_t channels_a, int64_t channels_b,
                                                     int64_t batch, int64_t depth, int64_t height, int64_t width,
                                                     int32_t kernel_size) {
   if (kernel_size != 1 && kernel_size != 3) return 1;
-  const int64_t ciw = 16;
-  const int64_t blocks = cdiv(channels_out, kCoT) * cdiv(channels_a + channels_b, ciw);
+  const int64_t ci = channels_a + channels_b;
   const int64_t bricks = batch * cdiv(width, kTX) * cdiv(height, kTY) * cdiv(depth, kTZ);
+  const bool taps = kernel_size == 3 && wgrad_by_taps(channels_out, ci, bricks);
+  const int64_t blocks = cdiv(channels_out, kCoT) * cdiv(ci, taps ? 8 : 16);
   int64_t splits = cdiv(4 * (int64_t)num_sms(), blocks);
-  if (kernel_size == 3) {
-    // three blocks an SM at a time: the fewest bricks in a row over the waves, and the fewest partial sums for that (32 and
-    // 96 channels at 24 x 24 x 16 cells: 612 blocks of three bricks were three waves, 272 us; 432 of four are one, 228)
-    const int64_t places = 3 * (int64_t)num_sms();
-    int64_t best = INT64_MAX;
-    for (int64_t n = 1; n <= bricks && n <= 4096; ++n) {
-      const int64_t turns = cdiv(blocks * n, places) * cdiv(bricks, n);
-      if (turns < best) best = turns, splits = n;
+  if (kernel_size == 3 && !taps) {
+    // wgrad3, three blocks an SM at a time: bricks one after the other take about 45 us each, and the partial sums are written
+    // and read once (4 bytes each way at 6.8 TB/s). Whole numbers of waves are tried, with the fewest
+    // splits for their bricks in a row, up to 64 MB of partial sums. Without their cost 64 -> 64 channels at 4 x 48 x 48 x 32
+    // cells took 1152 splits of 510 MB for 41 bricks in a row, where 28 splits of 12 MB have 42.
+    const int64_t places = 3 * (int64_t)num_sms(), weights = channels_out * ci * 27;
+    const int64_t most = std::max<int64_t>(1, std::min(bricks, (int64_t)64'000'000 / (4 * weights)));
+    double best = 1e300;
+    for (int64_t waves = 1; waves <= 16; ++waves) {
+      const int64_t n = std::min(std::max<int64_t>(1, places * waves / blocks), most);
+      const int64_t row = cdiv(bricks, n), fewest = cdiv(bricks, row);
+      const double us = 45.0 * (double)(cdiv(blocks * fewest, places) * row) + 8.0 * (double)(fewest * weights) / 6.8e6;
+      if (us < best) best = us, splits = fewest;
+      if (n == most) break;
     }
   }
   if (splits > bricks) splits = bricks;
@@ -1142,19 +1162,25 @@ extern "C" int citrus_conv3d_backward_weight(const float* grad_out, int64_t chan
   if (partial == nullptr || partial_capacity < 2 * nW) splits = 1;
   else if (splits * nW > partial_capacity) splits = partial_capacity / nW;
   float* dst = splits == 1 ? grad_weight : partial;
-  const int ciw = 16;
-  dim3 grid((unsigned)cdiv(channels_out, kCoT), (unsigned)cdiv(channels_a + channels_b, ciw), (unsigned)splits);
-  if (kernel_size == 3) {
+  const bool taps = kernel_size == 3 && wgrad_by_taps(channels_out, channels_a + channels_b,
+                                                      batch * cdiv(width, kTX) * cdiv(height, kTY) * cdiv(depth, kTZ));
+  dim3 grid((unsigned)cdiv(channels_out, kCoT), (unsigned)cdiv(channels_a + channels_b, taps ? 8 : 16), (unsigned)splits);
+  if (taps) {
+    wgrad_kernel<3, 8><<<grid, kConvThreads, 0, s>>>(grad_out, (int)channels_out, in_a, (int)channels_a, in_b,
+                                                     (int)channels_b, b_upsampled ? 1 : 0, dst, (int)splits,
+                                                     (int)batch, (int)depth, (int)height, (int)width);
+  } else if (kernel_size == 3) {
     const cudaError_t e =
         cudaFuncSetAttribute(wgrad3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWgSmem);
     if (e != cudaSuccess) return set_error(CITRUS_ECUDA, "citrus_conv3d_backward_weight: %s", cudaGetErrorString(e));
     wgrad3_kernel<<<grid, kWgThreads, kWgSmem, s>>>(grad_out, (int)channels_out, in_a, (int)channels_a, in_b,
                                                     (int)channels_b, b_upsampled ? 1 : 0, dst, (int)splits, (int)batch,
                                                     (int)depth, (int)height, (int)width);
-  } else
+  } else {
     wgrad_kernel<1, 16><<<grid, kConvThreads, 0, s>>>(grad_out, (int)channels_out, in_a, (int)channels_a, in_b,
                                                       (int)channels_b, b_upsampled ? 1 : 0, dst, (int)splits,
                                                       (int)batch, (int)depth, (int)height, (int)width);
+  }
   note_launches();
   if (splits > 1) {
     wgrad_reduce_kernel<<<(unsigned)cdiv(nW, kLearnThreads), kLearnThreads, 0, s>>>(partial, (int)splits, nW,
