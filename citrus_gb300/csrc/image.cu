@@ -153,8 +153,11 @@ __global__ void __launch_bounds__(32 * kBlurLines) box_blur_warp_kernel(const fl
 // a sector of its own: 64 wavefronts per 32 pixels, twice the arithmetic. A block takes kTileLines adjacent lines through
 // shared memory instead, read and written by rows of kTileLines floats (two whole sectors), two lines per warp: the rows
 // of 512 images of 192 x 256 pixels 241 -> 175 us (the arithmetic remains), of 5 groups of 61 x 83 pixels 164 -> 150 us.
-// Up to kTileMaxN pixels a line two blocks fit an SM; longer lines keep the form above.
+// Up to kTileMaxN pixels a line two blocks fit an SM; longer lines keep the form above. So do images of few pixels, whose
+// tiles leave SMs idle (two lines per warp, one after the other; us, lines / tiles): 16 directions of 17 x 19 pixels 2.7 /
+// 3.9, 4 of 192 x 256 5.0 / 6.9, 16 of 128 x 128 5.1 / 5.6, 32 of them 8.0 / 6.6, 16 of 192 x 256 10.4 / 8.3.
 constexpr int kTileLines = 16, kTileMaxN = 440;
+constexpr int64_t kTilePixels = 1 << 19;  // of all directions
 
 __host__ __device__ constexpr int blur_tile_stride(int N) { return (4 * N + 2) | 1; }  // odd: no bank conflicts across lines
 
@@ -316,7 +319,8 @@ extern "C" int citrus_box_blur(const float* in, float* out, int64_t num_directio
   CITRUS_REQUIRE(in != out, "citrus_box_blur: in and out must not alias");
   if (num_directions == 0 || lines == 0) return CITRUS_OK;
   WidthArgs wa{widths, height_sums, cell_width, axis, (float)(pitch > 0 ? 1.0 / pitch : 0.0), (float)center_height};
-  if (length <= kTileMaxN && is_l == 1 && os_l == 1 && is_p != 1 && cdiv(lines, kTileLines) <= 0x7fffffff) {
+  if (length <= kTileMaxN && num_directions * lines * length >= kTilePixels && is_l == 1 && os_l == 1 && is_p != 1 &&
+      cdiv(lines, kTileLines) <= 0x7fffffff) {
     const size_t smem = (size_t)kTileLines * blur_tile_stride((int)length) * sizeof(float);
     cudaError_t e = cudaFuncSetAttribute(box_blur_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)(kTileLines * blur_tile_stride(kTileMaxN) * sizeof(float)));
