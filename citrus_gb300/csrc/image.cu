@@ -213,26 +213,31 @@ __global__ void weighted_group_sum_kernel(const float* __restrict__ img, const f
   out[((int64_t)k * R + r) * C + c] = acc;
 }
 
-// Sums over directions. Up to kSumBlock of them a thread takes one pixel and walks them. Above, a thread takes one pixel
-// of one block of kSumBlock directions, and the first of a pixel's threads adds the blocks' sums to the accumulator in order:
-// the rounding is that of one call per block, so a sum over all 512 directions of an image is as accurate as eight over
-// 64, and a small panel (64 x 64 pixels are 16 blocks of 256 threads) has a thread per block of directions instead of one walk
-// down all of them: a full image of 5 groups 332 -> 59 us. With one block of directions the shared sums and barriers
-// only cost: 64 directions of 384 x 512 pixels 7.9 us, 4.7 without.
+// Sums over directions in blocks of kSumBlock, each added to the accumulator in order: the rounding is that of one call per
+// block, so a sum over all 512 directions of an image is as accurate as eight over 64. A thread takes a pixel and walks all
+// its directions; where there are several blocks and too few pixels to fill the SMs, a thread takes a pixel of one block
+// and the first of the pixel's threads adds the sums up (kBlocks): a full image of 5 groups, 64 x 64 pixels 332 -> 59 us.
 constexpr int kSumBlock = 64, kSumPixels = 64, kSumSlices = 8, kSumThreads = 256;
 
-template <bool kBlocks, typename Term>
-__device__ __forceinline__ void sum_directions(int K, bool inside, float* __restrict__ acc, int accumulate, Term term) {
+// sum over k of term(k, s) into acc; walk(first, last) gives a block's sum to a thread that takes the pixel alone
+template <bool kBlocks, typename Term, typename Walk>
+__device__ __forceinline__ void sum_directions(int K, bool inside, float* __restrict__ acc, int accumulate, Term term,
+                                               Walk walk) {
+  float total = inside && accumulate && threadIdx.y == 0 ? *acc : 0.f;
+  bool have = accumulate != 0;
   if constexpr (!kBlocks) {
     if (!inside) return;
-    float s = 0.f;
-    for (int k = 0; k < K; ++k) term(k, s);
-    *acc = accumulate ? *acc + s : s;
+    int k0 = 0;
+    do {
+      const float s = walk(k0, min(k0 + kSumBlock, K));
+      total = have ? total + s : s;
+      have = true;
+      k0 += kSumBlock;
+    } while (k0 < K);
+    *acc = total;
   } else {
     __shared__ float s_part[kSumSlices][kSumPixels];
     const int slices = blockDim.y;
-    float total = inside && accumulate && threadIdx.y == 0 ? *acc : 0.f;
-    bool have = accumulate != 0;
     for (int k0 = 0; k0 < K; k0 += slices * kSumBlock) {
       const int first = k0 + threadIdx.y * kSumBlock, last = min(first + kSumBlock, K);
       float s = 0.f;
@@ -253,9 +258,13 @@ __device__ __forceinline__ void sum_directions(int K, bool inside, float* __rest
   }
 }
 
-// the block of a sum over K directions, and its pixels
-inline dim3 sum_threads(int64_t K) {
-  if (K <= kSumBlock) return dim3(kSumThreads);
+// The block of a sum over K directions of the given pixels; two dimensions: by blocks of directions. us, a thread per pixel / by
+// blocks: 65 directions of 192 x 256 pixels 3.4 / 4.5, 256 of them 7.3 / 8.2, 512 of 384 x 512 64 / 69, of 64 x 64 13 / 4.7; weighted, 65
+// directions of 192 x 256 pixels 10.9 / 8.4, of 384 x 512 9.9 / 20, 96 of them 14 / 26, 128 of them 51 / 35.
+inline dim3 sum_threads(int64_t K, int64_t pixels, bool weighted) {
+  const int64_t alone = weighted ? (pixels >= 131072 ? 96 : kSumBlock)
+                                 : (pixels >= 131072 ? K : pixels >= 32768 ? 256 : 96);
+  if (K <= alone) return dim3(kSumThreads);
   return dim3(kSumPixels, (unsigned)(cdiv(K, kSumBlock) < kSumSlices ? cdiv(K, kSumBlock) : kSumSlices));
 }
 
@@ -264,7 +273,13 @@ template <bool kBlocks>
 __global__ void sum_directions_kernel(const float* __restrict__ img, int K, int64_t P, int64_t stride_k,
                                       float* __restrict__ acc, int accumulate) {
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  sum_directions<kBlocks>(K, p < P, acc + p, accumulate, [&](int k, float& s) { s += img[k * stride_k + p]; });
+  sum_directions<kBlocks>(
+      K, p < P, acc + p, accumulate, [&](int k, float& s) { s += img[k * stride_k + p]; },
+      [&](int first, int last) {
+        float s = 0.f;
+        for (int k = first; k < last; ++k) s += img[k * stride_k + p];
+        return s;
+      });
 }
 
 // acc[g, r, c] (+)= sum_k W[k, g, r | 0, c | 0] img[k, g, r, c], images through strides (the accumulation of the full
@@ -280,8 +295,15 @@ __global__ void weighted_direction_sum_kernel(const float* __restrict__ img, int
   const int64_t w_k = (int64_t)G * w_rows * w_cols;
   const float* w = W + ((int64_t)g * w_rows + (w_rows > 1 ? r : 0)) * w_cols + (w_cols > 1 ? c : 0);
   const float* src = img + g * is_g + r * is_r + c * is_c;
-  sum_directions<kBlocks>(K, t < (int64_t)G * R * C, acc + t, accumulate,
-                          [&](int k, float& s) { s = fmaf(w[k * w_k], src[k * is_k], s); });
+  sum_directions<kBlocks>(
+      K, t < (int64_t)G * R * C, acc + t, accumulate, [&](int k, float& s) { s = fmaf(w[k * w_k], src[k * is_k], s); },
+      [&](int first, int last) {
+        const float *wk = w + first * w_k, *x = src + first * is_k;
+        float s = 0.f;
+#pragma unroll 4
+        for (int k = first; k < last; ++k, wk += w_k, x += is_k) s = fmaf(*wk, *x, s);
+        return s;
+      });
 }
 
 }  // namespace
@@ -299,8 +321,8 @@ extern "C" int citrus_weighted_direction_sum(const float* image, int64_t num_dir
                  "citrus_weighted_direction_sum: weights must be [K, G, rows | 1, cols | 1]");
   const int64_t total = groups * rows * cols;
   if (total == 0) return CITRUS_OK;
-  const dim3 threads = sum_threads(num_directions);
-  auto kernel = num_directions > kSumBlock ? weighted_direction_sum_kernel<true> : weighted_direction_sum_kernel<false>;
+  const dim3 threads = sum_threads(num_directions, total, true);
+  auto kernel = threads.y > 1 ? weighted_direction_sum_kernel<true> : weighted_direction_sum_kernel<false>;
   kernel<<<(unsigned)cdiv(total, threads.x), threads, 0, as_stream(stream)>>>(
       image, (int)num_directions, (int)groups, (int)rows, (int)cols, is_k, is_g, is_r, is_c, weights,
       (int)weight_rows, (int)weight_cols, accumulator, accumulate);
@@ -374,8 +396,8 @@ extern "C" int citrus_sum_directions(const float* image, int64_t num_directions,
                                      float* accumulator, int32_t accumulate, void* stream) {
   CITRUS_REQUIRE(image && accumulator && num_directions >= 0 && pixels >= 0, "citrus_sum_directions: bad arguments");
   if (pixels == 0) return CITRUS_OK;
-  const dim3 threads = sum_threads(num_directions);
-  auto kernel = num_directions > kSumBlock ? sum_directions_kernel<true> : sum_directions_kernel<false>;
+  const dim3 threads = sum_threads(num_directions, pixels, false);
+  auto kernel = threads.y > 1 ? sum_directions_kernel<true> : sum_directions_kernel<false>;
   kernel<<<(unsigned)cdiv(pixels, threads.x), threads, 0, as_stream(stream)>>>(image, (int)num_directions, pixels, stride_k,
                                                                                accumulator, accumulate);
   note_launches();
