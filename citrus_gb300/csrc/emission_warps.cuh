@@ -169,6 +169,7 @@ __global__ void __launch_bounds__(32 * kEmitWarps, emission_blocks(kGP, kMM)) em
   __shared__ __align__(16) float s_tmu[kMM][kGP];
   __shared__ int s_first[kEmitBins + 1];              // directions before each bin
   __shared__ short s_order[kEmitDirs], s_bin[kEmitDirs];
+  __shared__ int s_longest;                           // bits of the largest squared length of a direction
   const int G = kExact > 0 ? kExact : tb.G, TM = kExact ? kMM : traced_materials, M = kExact ? kMM : tb.M;
   const bool traced = kExact || tau_mu != nullptr;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -180,6 +181,7 @@ __global__ void __launch_bounds__(32 * kEmitWarps, emission_blocks(kGP, kMM)) em
     s_tmu[m][q] = (traced && m < TM && q < G) ? tau_mu[m * G + q] : 0.f;
   }
   for (int i = tid; i <= kEmitBins; i += nthreads) s_first[i] = 0;
+  if (tid == 0) s_longest = __float_as_int(1.f);
 
   const int64_t v = (int64_t)blockIdx.x * 32 + lane;
   const bool valid = v < in.V;
@@ -227,6 +229,8 @@ __global__ void __launch_bounds__(32 * kEmitWarps, emission_blocks(kGP, kMM)) em
   while (((tb.N - 1) >> shift) >= kEmitBins) ++shift;
   __syncthreads();  // s_om, s_tmu and the zeroed bins are complete
   for (int i = tid; i < nd; i += nthreads) {
+    const float length2 = s_om[i][0] * s_om[i][0] + s_om[i][1] * s_om[i][1] + s_om[i][2] * s_om[i][2];
+    if (!(length2 <= 1.005f)) atomicMax(&s_longest, __float_as_int(length2));
     int node;
     float w;
     table_position(tb, c[0] * s_om[i][0] + c[1] * s_om[i][1] + c[2] * s_om[i][2], node, w);
@@ -234,8 +238,9 @@ __global__ void __launch_bounds__(32 * kEmitWarps, emission_blocks(kGP, kMM)) em
     atomicAdd(&s_first[(node >> shift) + 1], 1);
   }
   __syncthreads();
-  // the directions' lengths and the cosines are rounded: one node and 1.01 cover more than that
-  const float nodes_away = 1.01f * sqrtf(margin) * (float)(tb.N - 1) / (tb.eta_hi - tb.eta_lo) + 1.f;
+  // the directions' lengths (up to 1.0025 taken as 1) and the cosines are rounded: one node and 1.01 cover more than that
+  const float nodes_away =
+      1.01f * sqrtf(margin * __int_as_float(s_longest)) * (float)(tb.N - 1) / (tb.eta_hi - tb.eta_lo) + 1.f;
   const int reach = nodes_away < 4096.f ? (int)nodes_away + 1 : 4096;
   // nodes [first of a bin - reach, last of the bin + reach + 1] have to fit the ring, or the window of rows in its place
   constexpr int kFloats = emission_floats(kGP, kMM);

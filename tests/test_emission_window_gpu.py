@@ -15,7 +15,7 @@ from citrus_gb300.workloads import bremsstrahlung_spectrum
 pytestmark = pytest.mark.gpu
 
 
-def _emission(device, groups, materials, distance, K, length=1.0, q=1, signal=True, traced=True):
+def _emission(device, groups, materials, distance, K, length, q=1, signal=True, traced=True):
     """A column of 3 x 2 cells, 32 along the axis (25.6 cm): every block's points span all of it."""
     rng = np.random.default_rng(groups + materials)
     dev = lambda x: torch.as_tensor(np.asarray(x), dtype=torch.float32, device=device)  # noqa: E731
@@ -49,11 +49,13 @@ def _emission(device, groups, materials, distance, K, length=1.0, q=1, signal=Tr
     (8, 1, {"traced": False}), (8, 2, {"q": 2, "signal": False}), (8, 3, {}), (8, 7, {}), (12, 2, {}), (16, 2, {}),
     (16, 3, {"signal": False})])
 @pytest.mark.parametrize("distance", [100.0, 60.0, 45.0, 15.0])
-def test_wide_fans_equal_group_lanes(cuda_device, monkeypatch, groups, materials, options, distance):
+@pytest.mark.parametrize("length", [1.0, 2.5])
+def test_wide_fans_equal_group_lanes(cuda_device, monkeypatch, groups, materials, options, distance, length):
+    """Directions of another length than 1 reach more nodes (their cosines are held at the ends of the table)."""
     monkeypatch.delenv("CITRUS_EMISSION_KERNEL", raising=False)
-    new = _emission(cuda_device, groups, materials, distance, 300, **options)
+    new = _emission(cuda_device, groups, materials, distance, 300, length, **options)
     monkeypatch.setenv("CITRUS_EMISSION_KERNEL", "groups")
-    old = _emission(cuda_device, groups, materials, distance, 300, **options)
+    old = _emission(cuda_device, groups, materials, distance, 300, length, **options)
     for a, b in zip(new, old):
         assert torch.equal(a, b)
     assert np.isfinite(float(new[0].sum()))
