@@ -24,7 +24,7 @@ from torch import Tensor
 
 from . import kernels
 from .citrus_step import CitrusState, project_scatter
-from .scatter_solver import MaterialFields, ScatterSolver
+from .scatter_solver import MaterialFields, ScatterSolver, free_memory
 
 
 def _check_states(states: Sequence[CitrusState], angles: Sequence[float]) -> None:
@@ -58,22 +58,21 @@ def sweep_launch_config(solver: ScatterSolver, fields: MaterialFields, views: in
     mu_cells = fields.mu_t_coarse.reshape(G, ctx.num_cells).t().contiguous()
     tuned_views, form = sweep_config(ctx, mu_cells, G, views, dc=dc)
     chosen = min(int(batch), max(1, views)) if batch > 0 else tuned_views
-    return min(chosen, views_that_fit(ctx, G, dc, solver.device)), form, dc
+    image = solver.image_direction_chunk(fields) * solver.image_bytes_per_direction(fields)
+    return min(chosen, views_that_fit(ctx, G, dc, solver.device, image_bytes=image)), form, dc
 
 
-def views_that_fit(ctx, num_groups: int, dc: int, device, share: float = 0.6) -> int:
-    """Views per sweep launch whose working set fits ``share`` of the free device memory: per view its scattering
-    moments and new accumulator (N_sh x N x 4G floats each), the chunk's store (8 x dc x N x 4G) and first-collision
+def views_that_fit(ctx, num_groups: int, dc: int, device, share: float = 0.6, image_bytes: int = 0) -> int:
+    """Views per sweep launch whose working set fits ``share`` of the free device memory that the buffers of the images
+    (``image_bytes``, one view at a time) leave: per view its scattering moments and new accumulator (N_sh x N x 4G floats each), the chunk's store (8 x dc x N x 4G) and first-collision
     means (8 x dc x N x G)."""
     N, J = ctx.num_cells, ctx.num_cells * 4 * num_groups
     per_view = 4 * (2 * ctx.num_moments * J + 8 * dc * J + 8 * dc * N * num_groups)
     if torch.cuda.is_current_stream_capturing():
         return 1 << 30
-    free, _ = torch.cuda.mem_get_info(device)
     # memory the caching allocator holds but no tensor uses counts as free: the count then does not depend on what
     # the previous step left cached, and the views per launch (and the products' tuned shapes) stay the same
-    free += torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)
-    return max(1, int(share * free) // per_view)
+    return max(1, int(share * (free_memory(device) - image_bytes)) // per_view)
 
 
 def resolve_batch(solver: ScatterSolver, fields: MaterialFields, views: int, batch: int) -> int:

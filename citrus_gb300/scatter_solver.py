@@ -37,12 +37,19 @@ from .uncollided import (FirstCollisionSamplingCorrection, first_collision_means
 
 SWEEP_CHUNK_BUDGET_BYTES = 8 * 2 ** 30
 IMAGE_CHUNK_BUDGET_BYTES = 8 * 2 ** 30
+IMAGE_CHUNK_MEMORY_SHARE = 0.25   # of the memory free at a solver's first image, beside other users of the device
 # Directions per image chunk at most. A chunk is 17 launches and about 0.5 ms of host work, and its buffers are past L2
 # from a few directions on, so the budget is the limit that matters: with chunks of 64 the image of a 32^3 grid with
 # one group waited for the host (whole view step 5.9 ms; one chunk of 512 directions: 3.0 ms). The emission takes up to
 # 256 directions per block and forms a point's sums at the table nodes once for them, so 64^3 x 8 groups gets two equal
 # chunks of 256 (4 GiB would make four of 128).
 IMAGE_CHUNK_MAX_DIRECTIONS = 512
+
+
+def free_memory(device) -> int:
+    """Device memory in bytes that a new tensor could take: free, or held by the caching allocator and in no tensor."""
+    free, _ = torch.cuda.mem_get_info(device)
+    return free + torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)
 
 
 @dataclass(frozen=True)
@@ -160,6 +167,7 @@ class ScatterSolver:
         self._cone_quadratures: dict = {}
         self.direction_context_cache_size = int(direction_context_cache_size)
         self._direction_contexts: OrderedDict = OrderedDict()
+        self._image_budget: Optional[int] = None
 
     # ---- grids and caches --------------------------------------------------------------------------------------
     @property
@@ -197,13 +205,26 @@ class ScatterSolver:
             self._cone_quadratures[key] = q
         return q
 
+    def image_budget(self) -> int:
+        """Bytes of an image chunk's buffers: ``IMAGE_CHUNK_BUDGET_BYTES``, or a share of the device memory that was
+        free when the solver first asked where that is less. Fixed then, so that the chunks (and what is captured with
+        them) stay the same whatever else the device holds later."""
+        if self._image_budget is not None:
+            return self._image_budget
+        if torch.cuda.is_current_stream_capturing():   # not asked under capture, nor decided by one
+            return IMAGE_CHUNK_BUDGET_BYTES
+        self._image_budget = min(IMAGE_CHUNK_BUDGET_BYTES, int(IMAGE_CHUNK_MEMORY_SHARE * free_memory(self.device)))
+        return self._image_budget
+
+    def image_bytes_per_direction(self, fields: MaterialFields) -> int:
+        """The emission at the points, optical depths and multiple-collision source of the cells, three panel images."""
+        Rd, Cd = self.geometry.image_shape
+        return 4 * self.num_groups * (fields.grid_quadrature.num_voxels + 2 * fields.grid_coarse.num_voxels
+                                      + 3 * Rd * Cd)
+
     def image_direction_chunk(self, fields: MaterialFields) -> int:
         """Directions per image chunk: as many as fit the budget, in equal chunks of ``direction_chunk`` to 512."""
-        G = self.num_groups
-        Rd, Cd = self.geometry.image_shape
-        # the emission at the points, optical depths and multiple-collision source of the cells, three panel images
-        per_direction = 4 * G * (fields.grid_quadrature.num_voxels + 2 * fields.grid_coarse.num_voxels + 3 * Rd * Cd)
-        most = min(IMAGE_CHUNK_MAX_DIRECTIONS, IMAGE_CHUNK_BUDGET_BYTES // max(1, per_direction))
+        most = min(IMAGE_CHUNK_MAX_DIRECTIONS, self.image_budget() // max(1, self.image_bytes_per_direction(fields)))
         directions = self.config.cone_num_polar * self.config.cone_num_azimuthal
         chunks = -(-directions // max(1, int(most)))
         return int(max(self.config.direction_chunk, -(-directions // chunks)))
