@@ -510,7 +510,11 @@ def _device_primary(library: MultigroupLibrary, path: Tensor, materials, geometr
     starts = np.cumsum([0, columns.size, u.size, v.size, theta.size]) * 8 + tables.data_ptr()
     extras = source.device_tables(geometry, angle, device)
     thickness = extras["thickness"]
-    filter_mu = None if thickness is None else _lib.upload(source.filter_attenuation(library), device, torch.float32)
+    filter_mu = None
+    if thickness is not None:
+        filter_mu = _lib.upload(source.filter_attenuation(library), device, torch.float32)
+        if filter_mu.numel() != w.numel():
+            raise ValueError(f"filter_attenuation has {filter_mu.numel()} energies, the library {w.numel()}")
     path = path.to(torch.float32).contiguous()
     fluence, planar, per_group = (torch.empty(G, Rd, Cd, device=device) for _ in range(3))
     signal = torch.empty(Rd, Cd, device=device)
