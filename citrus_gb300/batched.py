@@ -166,7 +166,7 @@ def _finish(states: Sequence[CitrusState], angles: Sequence[float], cones: list,
             norms: Tensor, sync_words: Tensor) -> list:
     """One read-back for every view's change norm and the sweeps' barrier words; the new states."""
     if sync_words.numel() and bool(sync_words[:, 2].ne(0).any()):
-        raise kernels._lib.CitrusKernelError("batched sweep: a grid-barrier wait of the persistent sweep ran out")
+        raise kernels._lib.CitrusKernelError("batched sweep: a bounded wait of the sweep kernel ran out")
     values = norms.tolist()
     new_states = []
     for v, (norm, diff) in enumerate(values):

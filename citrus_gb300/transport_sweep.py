@@ -342,7 +342,7 @@ def sweep(ctx: SweepContext, mu_t: Tensor, source_function, direction_chunk: Opt
             psi_out[index] = store.view(8 * chunk, N, Q).permute(0, 2, 1).reshape(8 * chunk, G, 4, N)
     if check and syncs:
         if bool(torch.stack([s[2] for s in syncs]).ne(0).any()):
-            raise kernels._lib.CitrusKernelError("sweep: a grid-barrier wait of the persistent sweep ran out")
+            raise kernels._lib.CitrusKernelError("sweep: a bounded wait of the sweep kernel ran out")
     phi = moments.view(ctx.num_moments, N, G, 4).permute(2, 0, 3, 1).reshape(G, ctx.num_moments, 4, *ctx.shape)
     if psi_out is not None:
         return phi, psi_out.view(ctx.num_directions, G, 4, *ctx.shape)
