@@ -473,16 +473,21 @@ __global__ void __launch_bounds__(kEmitPoints * kGP) fc_correction_kernel(
 // row is gathered from global memory. 120 directions over the sphere take 401 nodes, 24 of them 80, and the points of
 // a block spread a node over up to 28 more: 120 nodes of two materials and 8 groups are 64 KB. (32 directions in 48
 // KB, 88 nodes, never fitted: 1.77 ms at 64^3 points, 8 groups and 120 directions, now 0.75.)
+// kWindow: up to 8 groups the window is taken from 4 on, where kFcWindowNodes nodes of all materials fit it. With fewer groups
+// filling it costs more than it saves, and a batch that does not fit after all gathers its rows without the L1 that the
+// window holds; so a block whose batch does not fit goes on in batches of one direction per warp.
 constexpr int kFcWarps = 8;
-__host__ __device__ constexpr int fc_batch(int gp) { return gp > 8 ? 16 : 24; }
+constexpr int kFcWindowNodes = 140;
+__host__ __device__ constexpr int fc_batch(int gp, bool window) { return window ? (gp > 8 ? 16 : 24) : 32; }
 __host__ __device__ constexpr int fc_window_bytes(int gp) { return gp > 8 ? 176 * 1024 : 64 * 1024; }
+__host__ __device__ constexpr int fc_sums_bytes(int gp) { return kFcWarps * 3 * gp * 32 * 4; }
 
-template <int kGP, int kMM, bool kVec, bool kExact>  // kExact: kGP groups and kMM materials
+template <int kGP, int kMM, bool kVec, bool kExact, bool kWindow>  // kExact: kGP groups and kMM materials
 __global__ void __launch_bounds__(32 * kFcWarps, kGP > 8 ? 1 : 3) fc_correction_warps_kernel(
     FCInputs in, Table tb, PointGrid pg, const float* __restrict__ omegas, const float* __restrict__ weights, int K,
     const float* __restrict__ moments /*[M, 2, G, G]*/, float* __restrict__ sums /*[5, G, V] or null*/,
     float* __restrict__ scale, float* __restrict__ beta, float* __restrict__ cache /*[K, G, V] or null*/) {
-  constexpr int nthreads = 32 * kFcWarps, kFcDirBatch = fc_batch(kGP);
+  constexpr int nthreads = 32 * kFcWarps, kFcDirBatch = fc_batch(kGP, kWindow);
   extern __shared__ float4 s_dyn4[];
   float* s_tab = reinterpret_cast<float*>(s_dyn4);
   __shared__ float s_key[kMaxSorted];
@@ -494,7 +499,7 @@ __global__ void __launch_bounds__(32 * kFcWarps, kGP > 8 ? 1 : 3) fc_correction_
   __shared__ int s_window[2];
   __shared__ float s_u0[3];
   // after the direction loop the window's shared memory holds the warps' partial sums [kFcWarps][3][kGP][32]
-  static_assert(kFcWarps * 3 * kGP * 32 * 4 <= fc_window_bytes(kGP), "partial sums exceed the window");
+  static_assert(fc_sums_bytes(kGP) <= fc_window_bytes(kGP), "partial sums exceed the window");
   const int G = kExact ? kGP : tb.G, M = kExact ? kMM : tb.M;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t v = (int64_t)blockIdx.x * 32 + lane;
@@ -543,8 +548,11 @@ __global__ void __launch_bounds__(32 * kFcWarps, kGP > 8 ? 1 : 3) fc_correction_
 #pragma unroll
   for (int q = 0; q < kGP; ++q) I0[q] = I1[q] = I2[q] = 0.f;
   const int NS = window_node_stride(M, G);
-  for (int b0 = 0; b0 < K; b0 += kFcDirBatch) {
-    const int nb = min(kFcDirBatch, K - b0);
+  const int W = window_nodes(M, G, fc_window_bytes(kGP));
+  int held = 0, held_end = 0;  // the nodes in the window
+  int most = kFcDirBatch, nb;
+  for (int b0 = 0; b0 < K; b0 += nb) {
+    nb = min(most, K - b0);
     if (tid < nb) {
       const int d = sorted ? s_order[b0 + tid] : b0 + tid;
       s_d[tid] = d;
@@ -554,9 +562,35 @@ __global__ void __launch_bounds__(32 * kFcWarps, kGP > 8 ? 1 : 3) fc_correction_
       s_w[tid] = __ldg(weights + d);
     }
     __syncthreads();
-    stage_window<kExact ? kGP : 0>(tb, valid, ux, uy, uz, s_om, nb, warp, kFcWarps, warp, kFcWarps, tid, nthreads,
-                                   s_range, s_window, s_tab, fc_window_bytes(kGP));
-    const int win_lo = s_window[0];
+    // the window's slots are a ring over the nodes, node n in slot n % W: the batches' nodes move up the table, and only
+    // those that no batch before has brought are copied
+    bool windowed = false;
+    int first_node = 0, first_slot = 0;
+    if constexpr (kWindow) {
+      window_range(tb, valid, ux, uy, uz, s_om, nb, warp, kFcWarps, warp, kFcWarps, tid, s_range, s_window);
+      first_node = s_window[0];
+      const int end = first_node + s_window[1];  // all of it uniform over the block
+      windowed = s_window[1] <= W;
+      if (!windowed && nb > kFcWarps) {
+        most = kFcWarps;
+        nb = 0;
+        continue;
+      }
+      if (windowed) {
+        int from = held_end;
+        if (first_node < held || first_node > held_end || max(end, held_end) - first_node > W) from = held = first_node;
+        held_end = from == first_node ? end : max(end, held_end);
+        held = max(held, held_end - W);
+        first_slot = first_node % W;
+        const int slot = from % W, n = held_end - from, straight = min(n, W - slot);
+        if (n > 0) {
+          copy_window<kExact ? kGP : 0>(tb, from, straight, warp, kFcWarps, tid, nthreads, s_tab + slot * NS);
+          if (n > straight)
+            copy_window<kExact ? kGP : 0>(tb, from + straight, n - straight, warp, kFcWarps, tid, nthreads, s_tab);
+          __syncthreads();
+        }
+      }
+    }
     // one body per place of the rows: a pointer to either is a generic one, whose loads are no shared-memory loads
     auto batch = [&](auto windowed) {
       constexpr bool kWin = decltype(windowed)::value;
@@ -565,6 +599,9 @@ __global__ void __launch_bounds__(32 * kFcWarps, kGP > 8 ? 1 : 3) fc_correction_
         int i0;
         float w;
         table_position(tb, cosine, i0, w);
+        int slot0 = i0 - first_node + first_slot;
+        if (slot0 >= W) slot0 -= W;
+        const int slot1 = slot0 + 1 == W ? 0 : slot0 + 1;
         float S[kGP];
 #pragma unroll
         for (int q = 0; q < kGP; ++q) S[q] = 0.f;
@@ -572,8 +609,8 @@ __global__ void __launch_bounds__(32 * kFcWarps, kGP > 8 ? 1 : 3) fc_correction_
         for (int m = 0; m < kMM; ++m) {
           const float r = rho[m];
           if (m >= M || r == 0.f) continue;
-          const float* row0 = kWin ? s_tab + (i0 - win_lo) * NS + m * G * G : tb.t + ((int64_t)m * tb.N + i0) * G * G;
-          const float* row1 = row0 + (kWin ? NS : G * G);
+          const float* row0 = kWin ? s_tab + slot0 * NS + m * G * G : tb.t + ((int64_t)m * tb.N + i0) * G * G;
+          const float* row1 = kWin ? s_tab + slot1 * NS + m * G * G : row0 + G * G;
 #pragma unroll
           for (int g = 0; g < kGP; ++g) {
             if (g >= G) break;
@@ -596,7 +633,7 @@ __global__ void __launch_bounds__(32 * kFcWarps, kGP > 8 ? 1 : 3) fc_correction_
       }
     };
     if (valid) {
-      if (win_lo >= 0) batch(std::true_type{});
+      if (kWindow && windowed) batch(std::bool_constant<kWindow>{});
       else batch(std::false_type{});
     }
     __syncthreads();  // the batch's directions and window are replaced next
@@ -967,16 +1004,15 @@ int launch_fc_correction_m(dim3 grid, int G, cudaStream_t s, const FCInputs& in,
   return CITRUS_OK;
 }
 
-template <int kGP, int kMM, bool kVec, bool kExact>
-int launch_fc_correction_warps_e(dim3 grid, cudaStream_t s, const FCInputs& in, const Table& tb, const PointGrid& pg,
-                               const float* omegas, const float* weights, int K, const float* moments, float* sums,
-                               float* scale, float* beta, float* cache) {
-  constexpr int bytes = fc_window_bytes(kGP);
-  cudaError_t e = cudaFuncSetAttribute(fc_correction_warps_kernel<kGP, kMM, kVec, kExact>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+template <int kGP, int kMM, bool kVec, bool kExact, bool kWindow>
+int launch_fc_correction_warps_w(dim3 grid, cudaStream_t s, const FCInputs& in, const Table& tb, const PointGrid& pg,
+                                 const float* omegas, const float* weights, int K, const float* moments, float* sums,
+                                 float* scale, float* beta, float* cache) {
+  constexpr int bytes = kWindow ? fc_window_bytes(kGP) : fc_sums_bytes(kGP);
+  auto kernel = fc_correction_warps_kernel<kGP, kMM, kVec, kExact, kWindow>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e != cudaSuccess) return set_error(CITRUS_ECUDA, "first-collision window: %s", cudaGetErrorString(e));
-  fc_correction_warps_kernel<kGP, kMM, kVec, kExact><<<grid, 32 * kFcWarps, bytes, s>>>(in, tb, pg, omegas, weights, K,
-                                                                                moments, sums, scale, beta, cache);
+  kernel<<<grid, 32 * kFcWarps, bytes, s>>>(in, tb, pg, omegas, weights, K, moments, sums, scale, beta, cache);
   note_launches();
   return CITRUS_OK;
 }
@@ -985,13 +1021,20 @@ template <int kGP, int kMM, bool kVec>
 int launch_fc_correction_warps(dim3 grid, cudaStream_t s, const FCInputs& in, const Table& tb, const PointGrid& pg,
                                const float* omegas, const float* weights, int K, const float* moments, float* sums,
                                float* scale, float* beta, float* cache) {
-  if constexpr (kMM == 2 && (kVec || kGP < 4)) {
-    if (tb.G == kGP && tb.M == kMM)
-      return launch_fc_correction_warps_e<kGP, kMM, kVec, true>(grid, s, in, tb, pg, omegas, weights, K, moments, sums,
-                                                                scale, beta, cache);
+#define CITRUS_FCW(EXACT, WINDOW)                                                                                        \
+  launch_fc_correction_warps_w<kGP, kMM, kVec, EXACT, WINDOW>(grid, s, in, tb, pg, omegas, weights, K, moments, sums, \
+                                                              scale, beta, cache)
+  constexpr bool kExact = kMM == 2 && (kVec || kGP < 4);
+  const bool exact = kExact && tb.G == kGP && tb.M == kMM;
+  if constexpr (kGP > 8) {
+    return exact ? CITRUS_FCW(kExact, true) : CITRUS_FCW(false, true);
+  } else {
+    constexpr bool kWindow = kGP >= 4;
+    if (kWindow && tb.G >= 4 && (exact || window_nodes(tb.M, tb.G, fc_window_bytes(kGP)) >= kFcWindowNodes))
+      return exact ? CITRUS_FCW(kExact, kWindow) : CITRUS_FCW(false, kWindow);
+    return exact ? CITRUS_FCW(kExact, false) : CITRUS_FCW(false, false);
   }
-  return launch_fc_correction_warps_e<kGP, kMM, kVec, false>(grid, s, in, tb, pg, omegas, weights, K, moments, sums,
-                                                             scale, beta, cache);
+#undef CITRUS_FCW
 }
 
 // CITRUS_FC_KERNEL=groups selects the group-lane correction kernel (fc_correction_kernel); read at every call

@@ -98,12 +98,12 @@ __device__ __forceinline__ float row_dot(const float* __restrict__ row, const fl
 
 // The window of table nodes a block needs: its points' cosines with its directions span a few dozen of the eta nodes,
 // so the rows of those nodes ([node][m][g][g']) are staged in shared memory once and every interpolation of the block
-// reads them there. The lanes' nodes are neighbours: a node's stride is 16 bytes (4 where rows are read as floats) past a
-// multiple of all banks, so that eight neighbouring nodes are read without conflicts (16 bytes per (node, m) let four).
+// reads them there. The lanes' nodes are neighbours: a node's stride is an odd number of 16-byte reads (of floats where rows
+// are read as floats), so that neighbouring nodes are read without bank conflicts (16 bytes per (node, m) let four of them).
 constexpr int kWindowBytes = 32 * 1024;
 
 __host__ __device__ inline int window_node_stride(int M, int G) {
-  return (M * G * G + 31) / 32 * 32 + (G % 4 == 0 ? 4 : 1);
+  return G % 4 == 0 ? (M * G * G / 4 | 1) * 4 : M * G * G | 1;
 }
 __host__ __device__ inline int window_nodes(int M, int G, int bytes = kWindowBytes) {
   const int n = bytes / (4 * window_node_stride(M, G));
@@ -190,7 +190,6 @@ __device__ __forceinline__ void window_range(const Table& tb, bool valid, float 
 
 // Stages the table window of a block for the directions s_om[0..n) if its nodes fit, else s_window[0] = -1 (rows read from
 // global memory); arguments and barrier as window_range.
-template <int kG = 0>
 __device__ __forceinline__ void stage_window(const Table& tb, bool valid, float ux, float uy, float uz,
                                              const float (*s_om)[3], int n, int first_dir, int dir_step, int warp,
                                              int nwarps, int tid, int nthreads, int (*s_range)[32], int* s_window,
@@ -198,7 +197,7 @@ __device__ __forceinline__ void stage_window(const Table& tb, bool valid, float 
   window_range(tb, valid, ux, uy, uz, s_om, n, first_dir, dir_step, warp, nwarps, tid, s_range, s_window);
   const int lo = s_window[0], count = s_window[1];
   const bool fits = count >= 2 && count <= window_nodes(tb.M, tb.G, window_bytes);
-  if (fits) copy_window<kG>(tb, lo, count, warp, nwarps, tid, nthreads, s_tab);
+  if (fits) copy_window<0>(tb, lo, count, warp, nwarps, tid, nthreads, s_tab);
   __syncthreads();  // s_window is read, the copies are complete
   if (!fits) {
     if (tid == 0) s_window[0] = -1;
