@@ -473,11 +473,18 @@ __global__ void __launch_bounds__(kEmitPoints * kGP) fc_correction_kernel(
 // row is gathered from global memory. 120 directions over the sphere take 401 nodes, 24 of them 80, and the points of
 // a block spread a node over up to 28 more: 120 nodes of two materials and 8 groups are 64 KB. (32 directions in 48
 // KB, 88 nodes, never fitted: 1.77 ms at 64^3 points, 8 groups and 120 directions, now 0.75.)
-// kWindow: up to 8 groups the window is taken from 4 on, where kFcWindowNodes nodes of all materials fit it. With fewer groups
-// filling it costs more than it saves, and a batch that does not fit after all gathers its rows without the L1 that the
-// window holds; so a block whose batch does not fit goes on in batches of one direction per warp.
+// kWindow: up to 8 groups the window is taken from 4 on, where kFcWindowNodes nodes of all materials fit it (8 directions of
+// 120 take 27 of 401 nodes, and 32 points along a column 25.6 long spread them over up to 104 from a source at 60). With fewer
+// groups filling it costs more than it saves, and a batch that does not fit after all gathers its rows without the L1 that the
+// window holds; so a block whose batch does not fit goes on in batches of one direction per warp (and gathers those
+// that don't fit either; going back to whole batches for them took registers, 246 -> 262 us below). us at 32^3 points, 120
+// directions, the source at 100 / 60, without the window or with one of 24 directions or none -> now: two materials, 8
+// groups 546 / 786 -> 246 / 722, 7 groups 525 / 1201 -> 179 / 469, 5 groups 208 / 443 -> 126 / 179, one group 82 / 43 -> 23 / 23;
+// three materials and 7 groups, no window, 1322 / 2008 -> 805 / 904.
 constexpr int kFcWarps = 8;
-constexpr int kFcWindowNodes = 140;
+// Where the table has more than kFcNodesPerDirection nodes for each direction, the nodes of 8 directions are too many to copy for
+// them, and the whole batch gathers: 11 groups, 32 directions 135 us, in batches of 8 219; 5 groups, 80 directions 278 / 309.
+constexpr int kFcWindowNodes = 140, kFcNodesPerDirection = 4;
 __host__ __device__ constexpr int fc_batch(int gp, bool window) { return window ? (gp > 8 ? 16 : 24) : 32; }
 __host__ __device__ constexpr int fc_window_bytes(int gp) { return gp > 8 ? 176 * 1024 : 64 * 1024; }
 __host__ __device__ constexpr int fc_sums_bytes(int gp) { return kFcWarps * 3 * gp * 32 * 4; }
@@ -571,7 +578,7 @@ __global__ void __launch_bounds__(32 * kFcWarps, kGP > 8 ? 1 : 3) fc_correction_
       first_node = s_window[0];
       const int end = first_node + s_window[1];  // all of it uniform over the block
       windowed = s_window[1] <= W;
-      if (!windowed && nb > kFcWarps) {
+      if (!windowed && nb > kFcWarps && tb.N <= kFcNodesPerDirection * K) {
         most = kFcWarps;
         nb = 0;
         continue;
@@ -1024,6 +1031,8 @@ int launch_fc_correction_warps(dim3 grid, cudaStream_t s, const FCInputs& in, co
 #define CITRUS_FCW(EXACT, WINDOW)                                                                                        \
   launch_fc_correction_warps_w<kGP, kMM, kVec, EXACT, WINDOW>(grid, s, in, tb, pg, omegas, weights, K, moments, sums, \
                                                               scale, beta, cache)
+  // two materials and the padded number of groups known to the compiler: us at 32^3 points and 120 directions, known / not: one
+  // group 23 / 29, two 43 / 41, 8 groups 246 / 717 (not known, their window of 124 nodes is not taken), 16 groups 1438 / 1497
   constexpr bool kExact = kMM == 2 && (kVec || kGP < 4);
   const bool exact = kExact && tb.G == kGP && tb.M == kMM;
   if constexpr (kGP > 8) {
