@@ -190,8 +190,10 @@ void launch_moments_point(const float* transfer, const float* phi, float* out, i
 //   54 / 33 (151); 5 groups: 24^3 19 / 26 (80), 32^3 63 / 52 (189); 8 groups: 16^3 14 / 21 (38), 24^3 60 / 33 (127).
 // With the points adjacent (moment-major) the blocks' tiles pay from 14 MB on, except over so few moments that the
 // transfers are most of what is read (4 moments of 5 groups, 64^3: 123 / 157). bytes: the lines of phi and T that are touched.
-inline bool moments_by_points(int GI, int degrees, int64_t bytes, bool points_adjacent) {
-  if (GI <= 2) return true;
+// From points adjacent to cells adjacent the blocks' tiles pay for two groups too (64^3, 36 moments, 604 MB: 499 / 409).
+inline bool moments_by_points(int GI, int degrees, int64_t bytes, bool points_adjacent, bool out_adjacent) {
+  if (GI == 1) return true;
+  if (GI == 2) return !points_adjacent || out_adjacent || bytes <= 300'000'000;
   if (GI > 8 || (GI > 6 && degrees < 4)) return false;
   if (degrees == 1) return true;
   if (points_adjacent) return bytes <= 14'000'000 || (degrees == 2 && GI != 4);
@@ -235,7 +237,7 @@ extern "C" int citrus_scattering_moments(const float* transfer, const float* phi
   else                                                                                                               \
     launch_moments_point<KGI, float>(transfer, phi, out, GI, GO, NL, L + 1, num_points, (int)k_count, ps_g, ps_n,    \
                                      ps_k, ps_x, os_g, os_n, os_k, os_x, s);
-  if (moments_by_points(GI, L + 1, bytes, points_adjacent)) {
+  if (moments_by_points(GI, L + 1, bytes, points_adjacent, os_x == 1)) {
     if (GI == 1) {
       CITRUS_MOMENTS_POINT(1)
     } else if (GI == 2) {
