@@ -488,6 +488,9 @@ int launch_emission_warps_q(const EmissionCall& c) {
 template <int kGP, int kMM, bool kVec>
 int launch_emission_warps_v(const EmissionCall& c) {
   const bool q1 = c.pg.f == 1;
+  // Numbers of groups and materials known to the compiler, where the optical depths come by material: us at 32^3 points and
+  // 512 directions, known / not: 1 group 151 / 163, 2 155 / 208, 5 282 / 402, 8 326 / 482, 12 688 / 886, 16 782 / 1021. Each number
+  // costs two kernels a material count and their compile time, so 9 to 11, 13 to 15 and three materials have none.
   if (c.tau_mu != nullptr && c.tb.M == kMM && c.TM == kMM) {
 #define CITRUS_EWE(EXACT)                                                                                     \
   if constexpr (kMM <= 2 && kVec == (EXACT % 4 == 0) && kGP >= EXACT && kGP < 2 * EXACT) {                    \

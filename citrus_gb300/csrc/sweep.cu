@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) tiled_kernel(
 // earliest unfinished task never waits, so every wait ends, however many blocks are resident.
 // Against the plane wavefront it reads a cell's source once and its own outputs not at all (three neighbours per cell
 // came from L2), loads no entry tables, and needs no grid barrier: 64^3 cells, 8 groups, 120 directions 3.81 -> 2.31 ms,
-// in pairs of views 2.92 -> 1.77 ms per view; 32^3, one group 0.57 -> 0.21 ms. Its issue slots are 70 % busy (about 200
+// in pairs of views 2.92 -> 1.77 ms per view; 32^3, one group 0.57 -> 0.21 ms. Its issue slots are 70 % busy (about 250
 // instructions per cell, half of them the coefficients that two views share); HBM's floor at 64^3 is 1.19 ms.
 constexpr int kPencilSlots = 5;
 constexpr int kPencilAhead = kPencilSlots - 2;  // a slot is refilled a barrier after the neighbours read its outputs
@@ -791,6 +791,8 @@ extern "C" int citrus_sweep_pencils(float* store, const float* mu_cells, const f
   (views_per_thread == 2                                                                                          \
        ? launch_pencils<KG, 2>(store, mu_cells, c, p, views, sy, sync_words, max_blocks, t, skip, s)              \
        : launch_pencils<KG, 1>(store, mu_cells, c, p, views, sy, sync_words, max_blocks, t, skip, s))
+  // the number of groups known to the compiler for the two commonest: us at 64^3 cells and 120 directions, with it / without,
+  // one group 630 / 635, 8 groups 2242 / 2263 (32^3: 366 / 374); 16 groups have nothing more to gain
   switch (num_groups) {
     case 1: return CITRUS_PENCILS(1);
     case 8: return CITRUS_PENCILS(8);
