@@ -1039,7 +1039,10 @@ int launch_fc_correction_warps(dim3 grid, cudaStream_t s, const FCInputs& in, co
     return exact ? CITRUS_FCW(kExact, true) : CITRUS_FCW(false, true);
   } else {
     constexpr bool kWindow = kGP >= 4;
-    if (kWindow && tb.G >= 4 && (exact || window_nodes(tb.M, tb.G, fc_window_bytes(kGP)) >= kFcWindowNodes))
+    // up to 33 directions on 401 nodes fit no window but that of the last batch, which costs the others the L1: 5 groups, 32
+    // directions 50 us with it, 39 without; 48 directions pay
+    if (kWindow && tb.G >= 4 && (exact || (window_nodes(tb.M, tb.G, fc_window_bytes(kGP)) >= kFcWindowNodes &&
+                                           tb.N <= 3 * kFcNodesPerDirection * (int64_t)K)))
       return exact ? CITRUS_FCW(kExact, kWindow) : CITRUS_FCW(false, kWindow);
     return exact ? CITRUS_FCW(kExact, false) : CITRUS_FCW(false, false);
   }

@@ -20,6 +20,17 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("distance", [100.0, 60.0, 30.0, 12.0])
 @pytest.mark.parametrize("num_eta", [2, 401, 1201])
 def test_windows_of_wide_fans(cuda_device, monkeypatch, groups, materials, distance, num_eta):
+    _compare(cuda_device, monkeypatch, groups, materials, distance, num_eta, 117)     # a last batch that is not full
+
+
+# up to 33 directions of 401 nodes take no window below 9 groups; whole batches gather up to 100
+@pytest.mark.parametrize("groups, materials", [(4, 3), (5, 2), (6, 3), (7, 2), (8, 1), (8, 2), (11, 2)])
+@pytest.mark.parametrize("directions", [1, 7, 33, 34, 100, 101])
+def test_few_directions(cuda_device, monkeypatch, groups, materials, directions):
+    _compare(cuda_device, monkeypatch, groups, materials, 60.0, 401, directions)
+
+
+def _compare(cuda_device, monkeypatch, groups, materials, distance, num_eta, directions):
     rng = np.random.default_rng(groups)
     library = spectral_library(np.linspace(120.0, 30.0, groups + 1), bremsstrahlung_spectrum(seed=0),
                                ([WATER, BONE] * 4)[:materials], 1, num_eta=num_eta, fine_per_group=2)
@@ -28,7 +39,7 @@ def test_windows_of_wide_fans(cuda_device, monkeypatch, groups, materials, dista
     rho = dev(rng.random((materials, *grid.shape)) * (rng.random((materials, *grid.shape)) < 0.7))
     phi = dev(rng.random((groups, *grid.shape)) + 0.1)
     q = product_quadrature(6, 20)
-    omega, weight = dev(q.omega[:117]), dev(q.weight[:117])     # a last batch that is not full
+    omega, weight = dev(q.omega[:directions]), dev(q.weight[:directions])
     geo = ConeGeometry(distance, distance + 50.0, 64, 64, 0.4, 0.4)
 
     def run():
@@ -40,7 +51,7 @@ def test_windows_of_wide_fans(cuda_device, monkeypatch, groups, materials, dista
     monkeypatch.setenv("CITRUS_FC_KERNEL", "groups")
     old = run()
     assert torch.equal(new.cache, old.cache)
-    # 117 positive terms in another order, each rounded at a partial sum of at most the whole
+    # up to 117 positive terms in another order, each rounded at a partial sum of at most the whole
     magnitude = (weight.double()[:, None, None] * old.cache.double()).sum(0).view(groups, *grid.shape)
     for i in range(3):
         error = (new.sums[i].double() - old.sums[i].double()).abs()
